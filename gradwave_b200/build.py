@@ -14,6 +14,7 @@ import os
 import shutil
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
@@ -51,14 +52,18 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         return LIB
     nvcc = _nvcc()
     BUILD.mkdir(exist_ok=True)
-    objs = []
-    for src in sources():
+
+    def compile_one(src: Path) -> str:
         obj = BUILD / (src.stem + ".o")
         cmd = [nvcc, *ARCH, *NVCC_FLAGS, "-I", str(INCLUDE), "-c", str(src), "-o", str(obj)]
         if verbose:
             print(" ".join(cmd), flush=True)
         subprocess.run(cmd, check=True)
-        objs.append(str(obj))
+        return str(obj)
+
+    # the FFT sources hold one instantiation per axis length: compiled side by side
+    with ThreadPoolExecutor(max(1, min(8, os.cpu_count() or 1))) as pool:
+        objs = list(pool.map(compile_one, sources()))
     cuda_lib = Path(nvcc).resolve().parents[1] / "lib64"
     link = [nvcc, *ARCH, "-shared", "-o", str(LIB), *objs, "-L", str(cuda_lib), "-lcublas",
             "-Xlinker", "-rpath," + str(cuda_lib)]

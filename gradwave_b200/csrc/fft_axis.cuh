@@ -1,0 +1,551 @@
+// One-axis FFT kernels of the local term, for every box axis length 2^a 3^b
+// 5^c 7^d <= 128 (the 52 lengths of GWB_FFT_LENGTHS, one instantiation each).
+//
+// A length N is split as N = R1 R2 (both <= 16; 125 = 5 x 25; lengths up to 16
+// are not split). With n = a + R2 b and k = k1 + R1 k2,
+//
+//   X[k1 + R1 k2] = sum_a w_R2^(a k2) [ w_N^(a k1) sum_b w_R1^(b k1) x[a + R2 b] ]
+//
+// so a thread that holds the R1 points x[a + R2 b] transforms them in registers
+// (rdft.cuh), multiplies by the twiddles w_N^(a k1) and hands them through
+// shared memory to the thread that holds the R2 points of one k1 (Cooley &
+// Tukey, Math. Comp. 19 (1965) 297). Two register passes and one exchange per
+// axis: a pass per radix in shared memory, as these kernels had it before, cost
+// three to four exchanges with two block barriers each, and a block that holds a
+// whole plane leaves room for one to three blocks per SM.
+//
+// Kernels (k = k-point, b = band of the chunk):
+//   k_rows_inverse   sphere -> W2: axis 2 of the occupied rows (j0, i1); the
+//                    coefficients go from c straight to registers (map)
+//   k_cols_inverse   W2 -> W: axis 1 of the occupied planes j0, all n2 columns
+//   k_pencil_vloc    W -> W: axis 0, times v(r)/N, axis 0 back
+//   k_cols_forward   W -> W2: axis 1, the occupied rows only
+//   k_rows_forward   W2 -> out: axis 2, gathered to the sphere, + t c
+//   k_pencil_density W -> rho: axis 0 and sum of w |psi|^2 over a band group
+// Rows and columns are separate launches so that each kernel needs only its own
+// axis length and a few tens of KB of shared memory; the price is W2 (the rows
+// of the sphere's disc, 0.4 of W) written and read once more each way. Measured
+// against the passes in shared memory (whole applies, us): 42^3 float32 240 rows
+// 1086 -> 212, 36x36x108 float64 244 rows 2760 -> 763, 84^3 float64 258 rows
+// 13836 -> 5513, 108^3 float32 166 rows 14936 -> 3096, 96^3 float64 240 rows
+// 12031 -> 7830. Bound by the float64 pipe and by latency (1.6 to 4 TB/s of
+// scratch traffic), not by HBM.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include "common.cuh"
+#include "rdft.cuh"
+
+namespace gwb {
+
+#define GWB_FFT_LENGTHS(X)                                                                                     \
+  X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(12) X(14) X(15) X(16) X(18) X(20) X(21) X(24) X(25) X(27)    \
+  X(28) X(30) X(32) X(35) X(36) X(40) X(42) X(45) X(48) X(49) X(50) X(54) X(56) X(60) X(63) X(64) X(70) X(72)  \
+  X(75) X(80) X(81) X(84) X(90) X(96) X(98) X(100) X(105) X(108) X(112) X(120) X(125) X(126) X(128)
+
+// What one chunk of bands of the local term (or the density) works on.
+template <typename T> struct FftRun {
+  int n0, n1, n2;        // box
+  int M0, L0, M2;        // occupied extents of axes 0 and 2 (M = n: all of the axis)
+  int nk, nrow;          // k-points, row slots per k of W2
+  int nbc, b0;           // bands of this chunk, first band
+  int npw_max;
+  const int* map;        // (nk, nrow, n2) sphere index of each row point, -1: none
+  const int* rowof;      // (nk, L0, n1) row slot of (j0, i1), -1: none
+  const int* npw;        // (nk)
+  const cplx<T>* tw0;    // exp(-2 pi i t / n) per axis
+  const cplx<T>* tw1;
+  const cplx<T>* tw2;
+  cplx<T>* W2;           // (nk, nbc, nrow, n2)
+  cplx<T>* W;            // (nk, nbc, L0, n1, n2)
+  const T* v;            // (n0, n1, n2) v(r) / N
+  const T* t;            // (nk, npw_max)
+  const void* c;         // rows (nk, ., npw_max), complex128 when io64 else complex64
+  void* out;
+  int64_t ck, ok;        // k strides of c and out
+  int io64;
+  // density
+  const double* w;       // (nk, .) band weights, k stride wk
+  int64_t wk;
+  double* rho;           // (nk, ngrp, n0, n1, n2)
+  int ngrp, first;       // band groups; first: start from zero
+};
+
+// R1 of N = R1 R2, R1 <= R2 (R2 = 1: not split)
+constexpr int fft_r1(int n) {
+  if (n <= 16) return n;
+  int best = 0;
+  for (int r = 2; r * r <= n; ++r)
+    if (n % r == 0 && (n / r <= 16 || n == 125)) best = r;
+  return best;
+}
+
+template <typename T, int N> struct AxisCfg {
+  static constexpr int R1 = fft_r1(N), R2 = N / R1;
+  static_assert(R1 * R2 == N && R1 > 0, "axis length without a split");
+  // strided pencils per block (consecutive lanes take consecutive pencils, so a
+  // warp's loads are whole 128-byte lines); two passes: R2 threads per pencil
+  static constexpr int PB = R2 == 1 ? 128 : (R2 >= 8 ? 16 : 32);
+  static constexpr int NT = PB * R2;
+  // contiguous rows per block; padded so that a column of the exchange (one
+  // element per row of R2) hits different banks
+  static constexpr int P2 = R2 | 1;
+  static constexpr int RB = R2 == 1 ? 64 : (192 / R2 > 0 ? 192 / R2 : 1);
+  static constexpr int NTR = RB * R2;
+  // blocks per SM the registers are limited for (at most 113 registers in
+  // float64, 64 in float32; the 25-point pass of 125 needs more)
+  static constexpr int minb(int nt, int threads = sizeof(T) == 8 ? 576 : 1024) {
+    return R2 > 16 || threads < nt ? 1 : threads / nt;
+  }
+  static constexpr size_t smem_strided = R2 == 1 ? 0 : (size_t)N * PB * sizeof(cplx<T>);
+  static constexpr size_t smem_rows = R2 == 1 ? 0 : (size_t)RB * R1 * P2 * sizeof(cplx<T>);
+};
+
+namespace fft_detail {
+
+using rdft_detail::StaticFor;
+
+template <int SIGN, typename T> __device__ __forceinline__ cplx<T> tw_at(const cplx<T>* __restrict__ tw, int i) {
+  const cplx<T> w = tw[i];
+  return SIGN > 0 ? conj(w) : w;
+}
+
+// First pass: R1 points x[a + R2 b] -> exchange slots [k1][a], twiddled.
+template <typename T, int R1, int SIGN, class PUT>
+__device__ __forceinline__ void pass1(cplx<T> (&x)[R1], int a, const cplx<T>* __restrict__ tw, PUT&& put) {
+  rdft<R1, SIGN>(x);
+  StaticFor<0, R1>::run([&](auto kc) {
+    constexpr int k1 = decltype(kc)::value;
+    put(k1, k1 == 0 ? x[0] : x[k1] * tw_at<SIGN>(tw, a * k1));
+  });
+}
+
+template <typename T> __device__ __forceinline__ cplx<T> load_io(const void* p, int io64, size_t i) {
+  return io64 ? ld<T>((const cplx<double>*)p, i) : ld<T>((const cplx<float>*)p, i);
+}
+
+// memory row r of axis 0 -> offset of its occupied plane in W, or -1
+__device__ __forceinline__ int plane_of(int r, int M0, int L0, int n0, int plane) {
+  if (r <= M0) return r * plane;
+  return r >= n0 - (L0 - M0 - 1) ? (r - (n0 - L0)) * plane : -1;
+}
+
+}  // namespace fft_detail
+
+template <typename T, int N>
+__global__ void __launch_bounds__(AxisCfg<T, N>::NTR, AxisCfg<T, N>::minb(AxisCfg<T, N>::NTR))
+    k_rows_inverse(const FftRun<T> f) {
+  using C = AxisCfg<T, N>;
+  using namespace fft_detail;
+  constexpr int R1 = C::R1, R2 = C::R2, P2 = C::P2, RB = C::RB;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  cplx<T>* ex = reinterpret_cast<cplx<T>*>(smem_raw);
+  const int bl = blockIdx.y, k = blockIdx.z, tid = threadIdx.x;
+  const int row0 = blockIdx.x * RB;
+  const size_t crow = (size_t)k * f.ck + (size_t)(f.b0 + bl) * f.npw_max;
+  {
+    const int a = tid % R2, r = tid / R2, row = row0 + r;
+    if (row < f.nrow) {
+      const int* mp = f.map + ((size_t)k * f.nrow + row) * N;
+      int idx[R1];
+      StaticFor<0, R1>::run([&](auto bc) {
+        constexpr int b = decltype(bc)::value;
+        const int i2 = a + R2 * b;
+        idx[b] = (i2 <= f.M2 || i2 >= N - f.M2) ? mp[i2] : -1;
+      });
+      cplx<T> x[R1];
+      StaticFor<0, R1>::run([&](auto bc) {
+        constexpr int b = decltype(bc)::value;
+        x[b] = idx[b] >= 0 ? load_io<T>(f.c, f.io64, crow + idx[b]) : mk<T>(0, 0);
+      });
+      if constexpr (R2 == 1) {
+        rdft<R1, +1>(x);
+        cplx<T>* dst = f.W2 + (((size_t)k * f.nbc + bl) * f.nrow + row) * N;
+        StaticFor<0, R1>::run([&](auto bc) { dst[decltype(bc)::value] = x[decltype(bc)::value]; });
+      } else {
+        cplx<T>* e = ex + r * (R1 * P2) + a;
+        pass1<T, R1, +1>(x, a, f.tw2, [&](int k1, cplx<T> v) { e[k1 * P2] = v; });
+      }
+    }
+  }
+  if constexpr (R2 > 1) {
+    __syncthreads();
+    const int k1 = tid % R1, r = tid / R1, row = row0 + r;
+    if (r < RB && row < f.nrow) {
+      const cplx<T>* e = ex + r * (R1 * P2) + k1 * P2;
+      cplx<T> y[R2];
+      StaticFor<0, R2>::run([&](auto ac) { y[decltype(ac)::value] = e[decltype(ac)::value]; });
+      rdft<R2, +1>(y);
+      cplx<T>* dst = f.W2 + (((size_t)k * f.nbc + bl) * f.nrow + row) * N + k1;
+      StaticFor<0, R2>::run([&](auto kc) { dst[R1 * decltype(kc)::value] = y[decltype(kc)::value]; });
+    }
+  }
+}
+
+template <typename T, int N>
+__global__ void __launch_bounds__(AxisCfg<T, N>::NTR, AxisCfg<T, N>::minb(AxisCfg<T, N>::NTR))
+    k_rows_forward(const FftRun<T> f) {
+  using C = AxisCfg<T, N>;
+  using namespace fft_detail;
+  constexpr int R1 = C::R1, R2 = C::R2, P2 = C::P2, RB = C::RB;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  cplx<T>* ex = reinterpret_cast<cplx<T>*>(smem_raw);
+  const int bl = blockIdx.y, k = blockIdx.z, tid = threadIdx.x;
+  const int row0 = blockIdx.x * RB;
+  const size_t crow = (size_t)k * f.ck + (size_t)(f.b0 + bl) * f.npw_max;
+  const size_t orow = (size_t)k * f.ok + (size_t)(f.b0 + bl) * f.npw_max;
+  const T* tk = f.t + (size_t)k * f.npw_max;
+  auto store = [&](int g, cplx<T> val) {
+    const cplx<T> cv = load_io<T>(f.c, f.io64, crow + g);
+    const cplx<T> o = val + scale(cv, tk[g]);
+    if (f.io64) st((cplx<double>*)f.out, orow + g, o);
+    else st((cplx<float>*)f.out, orow + g, o);
+  };
+  {
+    const int a = tid % R2, r = tid / R2, row = row0 + r;
+    if (row < f.nrow) {
+      const cplx<T>* src = f.W2 + (((size_t)k * f.nbc + bl) * f.nrow + row) * N + a;
+      cplx<T> x[R1];
+      StaticFor<0, R1>::run([&](auto bc) { x[decltype(bc)::value] = src[R2 * decltype(bc)::value]; });
+      if constexpr (R2 == 1) {
+        rdft<R1, -1>(x);
+        const int* mp = f.map + ((size_t)k * f.nrow + row) * N;
+        StaticFor<0, R1>::run([&](auto bc) {
+          const int g = mp[decltype(bc)::value];
+          if (g >= 0) store(g, x[decltype(bc)::value]);
+        });
+      } else {
+        cplx<T>* e = ex + r * (R1 * P2) + a;
+        pass1<T, R1, -1>(x, a, f.tw2, [&](int k1, cplx<T> v) { e[k1 * P2] = v; });
+      }
+    }
+  }
+  if constexpr (R2 > 1) {
+    __syncthreads();
+    const int k1 = tid % R1, r = tid / R1, row = row0 + r;
+    if (r < RB && row < f.nrow) {
+      const int* mp = f.map + ((size_t)k * f.nrow + row) * N + k1;
+      const cplx<T>* e = ex + r * (R1 * P2) + k1 * P2;
+      cplx<T> y[R2];
+      StaticFor<0, R2>::run([&](auto ac) { y[decltype(ac)::value] = e[decltype(ac)::value]; });
+      rdft<R2, -1>(y);
+      StaticFor<0, R2>::run([&](auto kc) {
+        constexpr int o = R1 * decltype(kc)::value;
+        const int i2 = k1 + o;
+        const int g = (i2 <= f.M2 || i2 >= N - f.M2) ? mp[o] : -1;
+        if (g >= 0) store(g, y[decltype(kc)::value]);
+      });
+    }
+  }
+  if (blockIdx.x == 0) {
+    for (int g = f.npw[k] + tid; g < f.npw_max; g += blockDim.x) {
+      if (f.io64) st((cplx<double>*)f.out, orow + g, mk<T>(0, 0));
+      else st((cplx<float>*)f.out, orow + g, mk<T>(0, 0));
+    }
+  }
+}
+
+// Axis 1 of the columns (j0, i2) of one (band, k); columns are numbered
+// q = j0 n2 + i2, so that neighbouring lanes take neighbouring i2.
+template <typename T, int N>
+__global__ void __launch_bounds__(AxisCfg<T, N>::NT, AxisCfg<T, N>::minb(AxisCfg<T, N>::NT))
+    k_cols_inverse(const FftRun<T> f) {
+  using C = AxisCfg<T, N>;
+  using namespace fft_detail;
+  constexpr int R1 = C::R1, R2 = C::R2, PB = C::PB;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  cplx<T>* ex = reinterpret_cast<cplx<T>*>(smem_raw);
+  const int bl = blockIdx.y, k = blockIdx.z, n2 = f.n2;
+  const int c = threadIdx.x % PB, s = threadIdx.x / PB;
+  const int q = blockIdx.x * PB + c;
+  const bool live = q < f.L0 * n2;
+  const int j0 = live ? q / n2 : 0, i2 = q - j0 * n2;
+  const size_t kb = (size_t)k * f.nbc + bl;
+  if (live) {
+    const int* ro = f.rowof + ((size_t)k * f.L0 + j0) * N + s;
+    const cplx<T>* src = f.W2 + kb * f.nrow * n2 + i2;
+    int idx[R1];
+    StaticFor<0, R1>::run([&](auto bc) { idx[decltype(bc)::value] = ro[R2 * decltype(bc)::value]; });
+    cplx<T> x[R1];
+    StaticFor<0, R1>::run([&](auto bc) {
+      constexpr int b = decltype(bc)::value;
+      x[b] = idx[b] >= 0 ? src[idx[b] * n2] : mk<T>(0, 0);
+    });
+    if constexpr (R2 == 1) {
+      rdft<R1, +1>(x);
+      cplx<T>* dst = f.W + (kb * f.L0 + j0) * (size_t)(N * n2) + i2;
+      StaticFor<0, R1>::run([&](auto bc) { dst[decltype(bc)::value * n2] = x[decltype(bc)::value]; });
+    } else {
+      cplx<T>* e = ex + s * PB + c;
+      pass1<T, R1, +1>(x, s, f.tw1, [&](int k1, cplx<T> v) { e[k1 * (R2 * PB)] = v; });
+    }
+  }
+  if constexpr (R2 > 1) {
+    __syncthreads();
+    if (s < R1 && live) {
+      const cplx<T>* e = ex + s * (R2 * PB) + c;
+      cplx<T> y[R2];
+      StaticFor<0, R2>::run([&](auto ac) { y[decltype(ac)::value] = e[decltype(ac)::value * PB]; });
+      rdft<R2, +1>(y);
+      cplx<T>* dst = f.W + (kb * f.L0 + j0) * (size_t)(N * n2) + (size_t)s * n2 + i2;
+      StaticFor<0, R2>::run([&](auto kc) { dst[R1 * decltype(kc)::value * n2] = y[decltype(kc)::value]; });
+    }
+  }
+}
+
+template <typename T, int N>
+__global__ void __launch_bounds__(AxisCfg<T, N>::NT, AxisCfg<T, N>::minb(AxisCfg<T, N>::NT))
+    k_cols_forward(const FftRun<T> f) {
+  using C = AxisCfg<T, N>;
+  using namespace fft_detail;
+  constexpr int R1 = C::R1, R2 = C::R2, PB = C::PB;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  cplx<T>* ex = reinterpret_cast<cplx<T>*>(smem_raw);
+  const int bl = blockIdx.y, k = blockIdx.z, n2 = f.n2;
+  const int c = threadIdx.x % PB, s = threadIdx.x / PB;
+  const int q = blockIdx.x * PB + c;
+  const bool live = q < f.L0 * n2;
+  const int j0 = live ? q / n2 : 0, i2 = q - j0 * n2;
+  const size_t kb = (size_t)k * f.nbc + bl;
+  cplx<T>* dst = f.W2 + kb * f.nrow * n2 + i2;
+  const int* ro = f.rowof + ((size_t)k * f.L0 + j0) * N;
+  if (live) {
+    const cplx<T>* src = f.W + (kb * f.L0 + j0) * (size_t)(N * n2) + (size_t)s * n2 + i2;
+    cplx<T> x[R1];
+    StaticFor<0, R1>::run([&](auto bc) { x[decltype(bc)::value] = src[R2 * decltype(bc)::value * n2]; });
+    if constexpr (R2 == 1) {
+      rdft<R1, -1>(x);
+      StaticFor<0, R1>::run([&](auto bc) {
+        const int row = ro[decltype(bc)::value];
+        if (row >= 0) dst[row * n2] = x[decltype(bc)::value];
+      });
+    } else {
+      cplx<T>* e = ex + s * PB + c;
+      pass1<T, R1, -1>(x, s, f.tw1, [&](int k1, cplx<T> v) { e[k1 * (R2 * PB)] = v; });
+    }
+  }
+  if constexpr (R2 > 1) {
+    __syncthreads();
+    if (s < R1 && live) {
+      const cplx<T>* e = ex + s * (R2 * PB) + c;
+      cplx<T> y[R2];
+      StaticFor<0, R2>::run([&](auto ac) { y[decltype(ac)::value] = e[decltype(ac)::value * PB]; });
+      rdft<R2, -1>(y);
+      StaticFor<0, R2>::run([&](auto kc) {
+        constexpr int k2 = decltype(kc)::value;
+        const int row = ro[s + R1 * k2];
+        if (row >= 0) dst[row * n2] = y[k2];
+      });
+    }
+  }
+}
+
+// Axis 0 of the pencils p = i1 n2 + i2 of a group of bands: inverse, times
+// v(r)/N, forward. After the inverse a thread holds the R2 points
+// i0 = k1 + R1 k2 of its pencil; the forward transform starts on exactly these
+// (DFT over k2 first, twiddle w_N^(k1 m2), exchange, DFT over k1), so the pair
+// costs two exchanges. v is read from L1 after the first band of the group
+// (kept in registers it made the float64 kernels spill).
+template <typename T, int N>
+__global__ void __launch_bounds__(AxisCfg<T, N>::NT, AxisCfg<T, N>::minb(AxisCfg<T, N>::NT))
+    k_pencil_vloc(const FftRun<T> f, int bands_per_block) {
+  using C = AxisCfg<T, N>;
+  using namespace fft_detail;
+  constexpr int R1 = C::R1, R2 = C::R2, PB = C::PB;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  cplx<T>* ex1 = reinterpret_cast<cplx<T>*>(smem_raw);
+  cplx<T>* ex2 = ex1 + N * PB;
+  const int k = blockIdx.z;
+  const int plane = f.n1 * f.n2;  // box indices fit 32 bits (axes <= 128)
+  const int c = threadIdx.x % PB, s = threadIdx.x / PB;
+  const int p = blockIdx.x * PB + c;
+  const bool live = p < plane;
+  const int M0 = f.M0, L0 = f.L0;
+  const int bl0 = blockIdx.y * bands_per_block, bl1 = min(f.nbc, bl0 + bands_per_block);
+  for (int bl = bl0; bl < bl1; ++bl) {
+    // opaque per band: hoisted out of the loop, the twiddles and the 2 R1 + R2
+    // addresses take more registers than there are
+    const T* vp = f.v + p + s * plane;
+    const cplx<T>* tw = f.tw0;
+    int s_ = s;
+    asm volatile("" : "+l"(vp), "+l"(tw), "+r"(s_));
+    cplx<T>* base = f.W + ((size_t)k * f.nbc + bl) * (size_t)(L0 * plane) + p;
+    if (live) {
+      cplx<T> x[R1];
+      StaticFor<0, R1>::run([&](auto bc) {
+        constexpr int b = decltype(bc)::value;
+        const int o = plane_of(s_ + R2 * b, M0, L0, N, plane);
+        x[b] = o >= 0 ? base[o] : mk<T>(0, 0);
+      });
+      if constexpr (R2 == 1) {
+        rdft<R1, +1>(x);
+        StaticFor<0, R1>::run([&](auto bc) {
+          x[decltype(bc)::value] = scale(x[decltype(bc)::value], vp[decltype(bc)::value * plane]);
+        });
+        rdft<R1, -1>(x);
+        StaticFor<0, R1>::run([&](auto bc) {
+          constexpr int b = decltype(bc)::value;
+          const int o = plane_of(b, M0, L0, N, plane);
+          if (o >= 0) base[o] = x[b];
+        });
+      } else {
+        cplx<T>* e = ex1 + s * PB + c;
+        pass1<T, R1, +1>(x, s_, tw, [&](int k1, cplx<T> v) { e[k1 * (R2 * PB)] = v; });
+      }
+    }
+    if constexpr (R2 > 1) {
+      __syncthreads();  // also: every thread has read ex2 of the band before
+      if (s < R1 && live) {
+        const cplx<T>* e = ex1 + s * (R2 * PB) + c;
+        cplx<T> y[R2];
+        StaticFor<0, R2>::run([&](auto ac) { y[decltype(ac)::value] = e[decltype(ac)::value * PB]; });
+        rdft<R2, +1>(y);
+        StaticFor<0, R2>::run([&](auto kc) {
+          y[decltype(kc)::value] = scale(y[decltype(kc)::value], vp[R1 * decltype(kc)::value * plane]);
+        });
+        rdft<R2, -1>(y);
+        cplx<T>* o = ex2 + s * (R2 * PB) + c;
+        StaticFor<0, R2>::run([&](auto mc) {
+          constexpr int m2 = decltype(mc)::value;
+          o[m2 * PB] = m2 == 0 ? y[0] : y[m2] * tw_at<-1>(tw, s_ * m2);
+        });
+      }
+      __syncthreads();  // also: every thread has read ex1 before the next band fills it
+      if (live) {
+        const cplx<T>* e = ex2 + s * PB + c;
+        cplx<T> x[R1];
+        StaticFor<0, R1>::run([&](auto kc) { x[decltype(kc)::value] = e[decltype(kc)::value * (R2 * PB)]; });
+        rdft<R1, -1>(x);
+        StaticFor<0, R1>::run([&](auto bc) {
+          constexpr int b = decltype(bc)::value;
+          const int o = plane_of(s_ + R2 * b, M0, L0, N, plane);
+          if (o >= 0) base[o] = x[b];
+        });
+      }
+    }
+  }
+}
+
+// Density (gradwave core/batch.py:562-587, density_b): axis 0 of each pencil
+// and rho[k][group][r] += w[k][b] |psi_b(r)|^2 over the chunk's bands of the
+// group, in registers: one thread owns each output element, so the sums run in
+// a fixed order without atomics.
+template <typename T, int N>
+__global__ void __launch_bounds__(AxisCfg<T, N>::NT, AxisCfg<T, N>::minb(AxisCfg<T, N>::NT, 448))
+    k_pencil_density(const FftRun<T> f) {
+  using C = AxisCfg<T, N>;
+  using namespace fft_detail;
+  constexpr int R1 = C::R1, R2 = C::R2, PB = C::PB;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  cplx<T>* ex1 = reinterpret_cast<cplx<T>*>(smem_raw);
+  const int k = blockIdx.z, grp = blockIdx.y;
+  const int plane = f.n1 * f.n2;  // box indices fit 32 bits (axes <= 128)
+  const int c = threadIdx.x % PB, s = threadIdx.x / PB;
+  const int p = blockIdx.x * PB + c;
+  const bool live = p < plane;
+  const int M0 = f.M0, L0 = f.L0;
+  constexpr int RV = R2 == 1 ? R1 : R2, SV = R2 == 1 ? 1 : R1;
+  const bool own = live && s < SV;
+  double* rk = f.rho + ((size_t)k * f.ngrp + grp) * N * plane + p + (R2 == 1 ? 0 : s * plane);
+  double acc[RV];
+  StaticFor<0, RV>::run([&](auto kc) {
+    acc[decltype(kc)::value] = own && !f.first ? rk[SV * decltype(kc)::value * plane] : 0.0;
+  });
+  int buf = 0;
+  // band b belongs to group b % ngrp whatever the chunks are
+  for (int bl = (grp + f.ngrp - f.b0 % f.ngrp) % f.ngrp; bl < f.nbc; bl += f.ngrp) {
+    const double wb = f.w[(size_t)k * f.wk + f.b0 + bl];
+    if (wb == 0.0) continue;  // the same for every thread of the block
+    const cplx<T>* base = f.W + ((size_t)k * f.nbc + bl) * (size_t)(L0 * plane) + p;
+    auto add = [&](double& a, cplx<T> z) { a += wb * ((double)z.x * (double)z.x + (double)z.y * (double)z.y); };
+    cplx<T>* exb = ex1 + buf * (N * PB);
+    const cplx<T>* tw = f.tw0;  // opaque per band, as in k_pencil_vloc
+    int s_ = s;
+    asm volatile("" : "+l"(tw), "+r"(s_));
+    if (live) {
+      cplx<T> x[R1];
+      StaticFor<0, R1>::run([&](auto bc) {
+        constexpr int b = decltype(bc)::value;
+        const int o = plane_of(s_ + R2 * b, M0, L0, N, plane);
+        x[b] = o >= 0 ? base[o] : mk<T>(0, 0);
+      });
+      if constexpr (R2 == 1) {
+        rdft<R1, +1>(x);
+        StaticFor<0, R1>::run([&](auto bc) { add(acc[decltype(bc)::value], x[decltype(bc)::value]); });
+      } else {
+        cplx<T>* e = exb + s * PB + c;
+        pass1<T, R1, +1>(x, s_, tw, [&](int k1, cplx<T> v) { e[k1 * (R2 * PB)] = v; });
+      }
+    }
+    if constexpr (R2 > 1) {
+      __syncthreads();  // the other buffer is free: its readers have arrived here too
+      if (own) {
+        const cplx<T>* e = exb + s * (R2 * PB) + c;
+        cplx<T> y[R2];
+        StaticFor<0, R2>::run([&](auto ac) { y[decltype(ac)::value] = e[decltype(ac)::value * PB]; });
+        rdft<R2, +1>(y);
+        StaticFor<0, R2>::run([&](auto kc) { add(acc[decltype(kc)::value], y[decltype(kc)::value]); });
+      }
+      buf ^= 1;
+    }
+  }
+  if (own)
+    StaticFor<0, RV>::run([&](auto kc) { rk[SV * decltype(kc)::value * plane] = acc[decltype(kc)::value]; });
+}
+
+// Launchers: cudaErrorInvalidValue when the axis length is not one of GWB_FFT_LENGTHS.
+template <typename T> cudaError_t fft_rows_inverse(const FftRun<T>& f, cudaStream_t st);
+template <typename T> cudaError_t fft_rows_forward(const FftRun<T>& f, cudaStream_t st);
+template <typename T> cudaError_t fft_cols_inverse(const FftRun<T>& f, cudaStream_t st);
+template <typename T> cudaError_t fft_cols_forward(const FftRun<T>& f, cudaStream_t st);
+template <typename T> cudaError_t fft_pencil_vloc(const FftRun<T>& f, cudaStream_t st);
+cudaError_t fft_pencil_density(const FftRun<double>& f, cudaStream_t st);
+
+namespace fft_detail {
+
+template <typename T, int N, class K> cudaError_t launch_rows(K* kern, const FftRun<T>& f, cudaStream_t st) {
+  using C = AxisCfg<T, N>;
+  dim3 g((f.nrow + C::RB - 1) / C::RB, f.nbc, f.nk);
+  kern<<<g, C::NTR, C::smem_rows, st>>>(f);
+  return cudaGetLastError();
+}
+
+template <typename T, int N, class K> cudaError_t launch_cols(K* kern, const FftRun<T>& f, cudaStream_t st) {
+  using C = AxisCfg<T, N>;
+  dim3 g((f.L0 * f.n2 + C::PB - 1) / C::PB, f.nbc, f.nk);
+  kern<<<g, C::NT, C::smem_strided, st>>>(f);
+  return cudaGetLastError();
+}
+
+template <typename T, int N> cudaError_t launch_vloc(const FftRun<T>& f, cudaStream_t st) {
+  using C = AxisCfg<T, N>;
+  const int blocks = (f.n1 * f.n2 + C::PB - 1) / C::PB;
+  // bands per block: v is then read once for several bands, as long as four
+  // blocks per SM remain
+  int groups = (f.nbc + 3) / 4;
+  while (groups < f.nbc && (int64_t)blocks * f.nk * groups < 4 * 148) ++groups;
+  const int bpb = (f.nbc + groups - 1) / groups;
+  dim3 g(blocks, (f.nbc + bpb - 1) / bpb, f.nk);
+  if (2 * C::smem_strided > 48 * 1024) {
+    const cudaError_t e = allow_smem(k_pencil_vloc<T, N>);
+    if (e != cudaSuccess) return e;
+  }
+  k_pencil_vloc<T, N><<<g, C::NT, 2 * C::smem_strided, st>>>(f, bpb);
+  return cudaGetLastError();
+}
+
+template <typename T, int N> cudaError_t launch_density(const FftRun<T>& f, cudaStream_t st) {
+  using C = AxisCfg<T, N>;
+  dim3 g((f.n1 * f.n2 + C::PB - 1) / C::PB, f.ngrp, f.nk);
+  if (2 * C::smem_strided > 48 * 1024) {
+    const cudaError_t e = allow_smem(k_pencil_density<T, N>);
+    if (e != cudaSuccess) return e;
+  }
+  k_pencil_density<T, N><<<g, C::NT, 2 * C::smem_strided, st>>>(f);
+  return cudaGetLastError();
+}
+
+}  // namespace fft_detail
+
+}  // namespace gwb

@@ -3,23 +3,12 @@
 //
 // Local term (replaces gradwave core/batch.py:405-428). The sphere of each k
 // occupies Miller indices |m_a| <= M_a of a box n0 x n1 x n2, so only
-// L_a = 2 M_a + 1 planes/rows/columns per axis ever hold data:
-//
-//   K1 plane_inverse  one CTA per (axis-0 plane j0 < L0, band, k):
-//                     scatter the sphere points of the plane into a shared-
-//                     memory n1 x n2 plane, inverse FFT along axis 2 on the L1
-//                     occupied rows, inverse FFT along axis 1 on all columns,
-//                     store the plane to the scratch W (L0 planes per band).
-//   K2 pencil_vloc    one CTA per (axis-1 row i1, band, k): load the L0 planes'
-//                     row i1 as n2 pencils along axis 0, inverse FFT, multiply
-//                     by v(r)/N, forward FFT, store back the L0 occupied planes
-//                     (the V(r) psi(r) product never leaves shared memory).
-//   K3 plane_forward  one CTA per (j0, band, k): forward FFT along axis 1 and
-//                     along axis 2 on the occupied rows, gather the sphere,
-//                     add the kinetic term t c, write out (padding zeroed).
-//
-// The bands are processed in chunks whose scratch W fits in L2, so W is
-// written and re-read from L2 rather than HBM.
+// L_a = 2 M_a + 1 planes/rows/columns per axis ever hold data, and of the rows
+// (j0, i1) only those of a disc. Five launches per chunk of bands
+// (fft_axis.cuh): axis 2 of the disc's rows, axis 1 of the occupied planes,
+// axis 0 with the product with v(r)/N and back, axis 1, axis 2 with the
+// kinetic term. The bands are processed in chunks that bound the scratch (W and
+// W2).
 //
 // Nonlocal term (replaces gradwave core/batch.py:499-500 and becp_b :590-595):
 //   K4 becp_partial   becp partial sums conj(p) . c over a slice of G
@@ -35,8 +24,7 @@
 #include <vector>
 
 #include "common.cuh"
-#include "fft.cuh"
-#include "rdft.cuh"
+#include "fft_axis.cuh"
 
 namespace gwb {
 
@@ -49,7 +37,7 @@ struct FftGeom {
   int n[3];
   int M[3];  // max |Miller index| per axis over all k (compact row map)
   int L[3];  // occupied extent per axis (2M+1, capped at n)
-  AxisPlan plan[3];
+  int nrow;  // row slots (j0, i1) per k, the most of any k
 };
 
 }  // namespace gwb
@@ -61,9 +49,10 @@ struct gwb_ham {
   std::vector<int64_t> npw_host;
   // device tables
   int* d_npw = nullptr;
-  int* d_plane_ptr = nullptr;  // (nk*L0 + 1)
-  int* d_plane_g = nullptr;    // sphere index of each plane entry
-  int* d_plane_pos = nullptr;  // i1*n2 + i2 of each plane entry
+  int* d_map = nullptr;    // (nk, nrow, n2) sphere index of each row point, -1: none
+  int* d_rowof = nullptr;  // (nk, L0, n1) row slot of (j0, i1), -1: none
+  int* d_dup = nullptr;    // (ndup, 3) k, slot, other slot of the same box cell
+  int ndup = 0;
   double* d_t64 = nullptr;
   float* d_t32 = nullptr;
   double* d_v64 = nullptr;  // v(r)/N
@@ -77,7 +66,7 @@ struct gwb_ham {
   gwb::cplx<double>* d_tw64[3] = {nullptr, nullptr, nullptr};
   gwb::cplx<float>* d_tw32[3] = {nullptr, nullptr, nullptr};
   // scratch
-  void* d_W = nullptr;
+  void* d_W = nullptr;  // planes of a band chunk, then its rows
   size_t W_bytes = 0;
   void* d_part = nullptr;  // becp partials
   size_t part_bytes = 0;
@@ -104,393 +93,53 @@ struct gwb_ham {
   // tuning (gwb_ham_set_tuning; 0 = the built-in rule)
   size_t w_budget = 0;   // bytes of FFT scratch W per band chunk
   int nl_target = 0;     // CTAs the G-sliced becp contraction aims for
-  int fft_nt[2] = {0, 0};  // threads of the shared-memory FFT blocks (float32, float64); 0: the built-in rule
 };
 
 namespace gwb {
 
-static bool plan_axis(int n, AxisPlan* pl) {
+static bool axis_ok(int n) {
   if (n < 2 || n > 128) return false;
-  pl->n = n;
-  pl->nst = 0;
-  pl->code = 0;
-  int m = n;
-  const int order[7] = {8, 4, 6, 3, 2, 5, 7};
-  while (m > 1) {
-    bool found = false;
-    for (int R : order) {
-      if (m % R == 0) {
-        if (pl->nst >= 8) return false;
-        pl->code |= (unsigned)R << (4 * pl->nst);
-        pl->nst++;
-        m /= R;
-        found = true;
-        break;
-      }
-    }
-    if (!found) return false;
-  }
-  return true;
+  for (int p : {2, 3, 5, 7})
+    while (n % p == 0) n /= p;
+  return n == 1;
 }
+
+// Scratch of one band chunk. Measured on the FFT launches of a float64 96^3
+// apply of 240 rows: 8.9 ms at 48 MB (L2 sized), 8.4 at 96, 7.9 at 400, 7.7 at
+// 1200 (launch ramps and last waves weigh more than L2 misses).
+constexpr long kWBudgetMB = 512, kWBudgetLowMB = 48;
 
 static size_t w_budget_bytes() {
   const char* s = std::getenv("GWB_W_BUDGET_MB");
-  long mb = s ? std::atol(s) : 48;
+  long mb = s ? std::atol(s) : kWBudgetMB;
   if (mb < 1) mb = 1;
   return (size_t)mb << 20;
 }
 
-// ---------------------------------------------------------------------------
-// K1: sphere scatter + inverse FFT along axes 2 and 1, one plane per CTA.
-// Blocks per SM the shared-memory FFT kernels are compiled for: three 256-thread
-// blocks (the 72^3 and 96^3 planes of float32 fit three per SM), one block of
-// 512 or 1024 threads (float64 planes fill the shared memory with one).
-template <typename T, int NT, bool CT> constexpr int fft_minb() {
-  return !CT ? 1 : (NT == 256 ? 3 : (NT == 512 && sizeof(T) == 4 ? 2 : 1));
-}
-
-template <typename T, typename SIO, unsigned C1, unsigned C2, int NT = 256>
-__global__ void __launch_bounds__(NT, (fft_minb<T, NT, (C1 && C2)>())) k_plane_inverse(FftGeom g, const int* __restrict__ plane_ptr,
-                                                       const int* __restrict__ plane_g,
-                                                       const int* __restrict__ plane_pos,
-                                                       const SIO* __restrict__ c, cplx<T>* __restrict__ W,
-                                                       const cplx<T>* __restrict__ tw1,
-                                                       const cplx<T>* __restrict__ tw2, int64_t ck, int b0,
-                                                       int nbc, int npw_max) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int n1 = g.n[1], n2 = g.n[2], L0 = g.L[0];
-  const int j0 = blockIdx.x, bl = blockIdx.y, k = blockIdx.z;
-  cplx<T>* S = reinterpret_cast<cplx<T>*>(smem_raw);
-  cplx<T>* t1 = S + n1 * n2;
-  cplx<T>* t2 = t1 + n1;
-  for (int i = threadIdx.x; i < n1; i += blockDim.x) t1[i] = tw1[i];
-  for (int i = threadIdx.x; i < n2; i += blockDim.x) t2[i] = tw2[i];
-  for (int i = threadIdx.x; i < n1 * n2; i += blockDim.x) S[i] = mk<T>(0, 0);
-  __syncthreads();
-  const size_t crow = (size_t)k * ck + (size_t)(b0 + bl) * npw_max;
-  const int e0 = plane_ptr[k * L0 + j0], e1 = plane_ptr[k * L0 + j0 + 1];
-  for (int e = e0 + threadIdx.x; e < e1; e += blockDim.x) S[plane_pos[e]] = ld<T>(c, crow + plane_g[e]);
-  __syncthreads();
-  fft_any<T, false, +1, C2>(S, g.L[1], g.plan[2], n2, 1, g.M[1], n1, t2);
-  fft_any<T, true, +1, C1>(S, n2, g.plan[1], 1, n2, n2, n2, t1);
-  cplx<T>* dst = W + (((size_t)k * nbc + bl) * L0 + j0) * (size_t)(n1 * n2);
-  for (int i = threadIdx.x; i < n1 * n2; i += blockDim.x) dst[i] = S[i];
-}
-
-// K2: pencils along axis 0 for one (i1, band, k): inverse FFT, x v(r)/N, forward FFT.
-template <typename T, unsigned C0, int NT = 256>
-__global__ void __launch_bounds__(NT, (fft_minb<T, NT, (C0 != 0)>())) k_pencil_vloc(FftGeom g, cplx<T>* __restrict__ W,
-                                                     const T* __restrict__ v,
-                                                     const cplx<T>* __restrict__ tw0, int nbc) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int n0 = g.n[0], n1 = g.n[1], n2 = g.n[2], L0 = g.L[0];
-  const int i1 = blockIdx.x, bl = blockIdx.y, k = blockIdx.z;
-  cplx<T>* S = reinterpret_cast<cplx<T>*>(smem_raw);  // [i0][i2]
-  cplx<T>* t0 = S + n0 * n2;
-  for (int i = threadIdx.x; i < n0; i += blockDim.x) t0[i] = tw0[i];
-  cplx<T>* base = W + ((size_t)k * nbc + bl) * L0 * (size_t)(n1 * n2) + (size_t)i1 * n2;
-  for (int i = threadIdx.x; i < n0 * n2; i += blockDim.x) {
-    const int r = i / n2, i2 = i - r * n2;
-    // memory row r holds compact plane j0 (or stays zero)
-    int j0;
-    if (r <= g.M[0]) j0 = r;
-    else if (r >= n0 - (L0 - g.M[0] - 1)) j0 = r - (n0 - L0);
-    else j0 = -1;
-    S[i] = j0 >= 0 ? base[(size_t)j0 * n1 * n2 + i2] : mk<T>(0, 0);
-  }
-  __syncthreads();
-  fft_any<T, true, +1, C0>(S, n2, g.plan[0], 1, n2, n2, n2, t0);
-  for (int i = threadIdx.x; i < n0 * n2; i += blockDim.x) {
-    const int i0 = i / n2, i2 = i - i0 * n2;
-    S[i] = scale(S[i], v[((size_t)i0 * n1 + i1) * n2 + i2]);
-  }
-  __syncthreads();
-  fft_any<T, true, -1, C0>(S, n2, g.plan[0], 1, n2, n2, n2, t0);
-  for (int i = threadIdx.x; i < L0 * n2; i += blockDim.x) {
-    const int j0 = i / n2, i2 = i - j0 * n2;
-    const int r = rowmap(j0, g.M[0], L0, n0);
-    base[(size_t)j0 * n1 * n2 + i2] = S[r * n2 + i2];
-  }
-}
-
-// K2 with the whole axis-0 transform in registers (cubic box, N0 <= 48): one
-// thread per pencil (i1, i2) of one (band, k); the occupied planes are loaded
-// (coalesced over i2), inverse DFT, x v(r)/N, forward DFT, occupied planes
-// stored back. No shared memory, no barriers; the plane stride is a constant,
-// so every load and store is one base register plus an immediate offset.
-template <typename T, int N0>
-__global__ void __launch_bounds__(128) k_pencil_vloc_reg(FftGeom g, cplx<T>* __restrict__ W, const T* __restrict__ v,
-                                                         int nbc) {
-  constexpr int PLANE = N0 * N0;
-  const int L0 = g.L[0], M0 = g.M[0];
-  const int bl = blockIdx.y, k = blockIdx.z;
-  const int pidx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (pidx >= PLANE) return;
-  cplx<T>* base = W + ((size_t)k * nbc + bl) * L0 * (size_t)PLANE + pidx;
-  // occupied rows: 0..M0 hold planes 0..M0; rows N0-(L0-M0-1)..N0-1 hold the
-  // wrapped planes M0+1..L0-1, i.e. plane r - (N0 - L0)
-  const int hi0 = N0 - (L0 - M0 - 1);
-  cplx<T>* wrap = base - (ptrdiff_t)(N0 - L0) * PLANE;
-  cplx<T> x[N0];
-  rdft_detail::StaticFor<0, N0>::run([&](auto rc) {
-    constexpr int r = decltype(rc)::value;
-    x[r] = r <= M0 ? base[r * PLANE] : (r >= hi0 ? wrap[r * PLANE] : mk<T>(0, 0));
-  });
-  rdft<N0, +1>(x);
-  const T* vp = v + pidx;
-  rdft_detail::StaticFor<0, N0>::run([&](auto rc) {
-    constexpr int r = decltype(rc)::value;
-    x[r] = scale(x[r], vp[r * PLANE]);
-  });
-  rdft<N0, -1>(x);
-  rdft_detail::StaticFor<0, N0>::run([&](auto rc) {
-    constexpr int r = decltype(rc)::value;
-    if (r <= M0) base[r * PLANE] = x[r];
-    else if (r >= hi0) wrap[r * PLANE] = x[r];
-  });
-}
-
-// Density (gradwave core/batch.py:562-587, density_b): after K1 has put a
-// chunk of bands into W (inverse FFT along axes 2 and 1 over the occupied
-// planes), the axis-0 inverse FFT of each pencil and rho_k[k][r] +=
-// w[k][b] |psi_b(r)|^2, float64. One CTA (general box) or one thread (cubic
-// box, whole pencil in registers) owns each output element of one k and loops
-// over the chunk's bands, so the sums need no atomics and run in a fixed order.
-template <typename T, unsigned C0>
-__global__ void __launch_bounds__(256) k_pencil_density(FftGeom g, const cplx<T>* __restrict__ W,
-                                                        const cplx<T>* __restrict__ tw0,
-                                                        const double* __restrict__ w, int64_t wk, int b0, int nbc,
-                                                        double* __restrict__ rho_k, int first) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int n0 = g.n[0], n1 = g.n[1], n2 = g.n[2], L0 = g.L[0];
-  const int i1 = blockIdx.x, k = blockIdx.z;
-  const size_t N = (size_t)n0 * n1 * n2;
-  cplx<T>* S = reinterpret_cast<cplx<T>*>(smem_raw);  // [i0][i2]
-  cplx<T>* t0 = S + n0 * n2;
-  for (int i = threadIdx.x; i < n0; i += blockDim.x) t0[i] = tw0[i];
-  double* rk = rho_k + (size_t)k * N + (size_t)i1 * n2;
-  if (first)
-    for (int i = threadIdx.x; i < n0 * n2; i += blockDim.x) {
-      const int i0 = i / n2, i2 = i - i0 * n2;
-      rk[(size_t)i0 * n1 * n2 + i2] = 0.0;
-    }
-  for (int bl = 0; bl < nbc; ++bl) {
-    const double wb = w[(size_t)k * wk + b0 + bl];
-    if (wb == 0.0) continue;  // the same for every thread of the CTA
-    const cplx<T>* base = W + ((size_t)k * nbc + bl) * L0 * (size_t)(n1 * n2) + (size_t)i1 * n2;
-    __syncthreads();  // S of the previous band fully read
-    for (int i = threadIdx.x; i < n0 * n2; i += blockDim.x) {
-      const int r = i / n2, i2 = i - r * n2;
-      int j0;
-      if (r <= g.M[0]) j0 = r;
-      else if (r >= n0 - (L0 - g.M[0] - 1)) j0 = r - (n0 - L0);
-      else j0 = -1;
-      S[i] = j0 >= 0 ? base[(size_t)j0 * n1 * n2 + i2] : mk<T>(0, 0);
-    }
-    __syncthreads();
-    fft_any<T, true, +1, C0>(S, n2, g.plan[0], 1, n2, n2, n2, t0);
-    __syncthreads();
-    for (int i = threadIdx.x; i < n0 * n2; i += blockDim.x) {
-      const int i0 = i / n2, i2 = i - i0 * n2;
-      const cplx<T> v = S[i];
-      rk[(size_t)i0 * n1 * n2 + i2] += wb * ((double)v.x * (double)v.x + (double)v.y * (double)v.y);
-    }
-  }
-}
-
-template <typename T, int N0>
-__global__ void __launch_bounds__(128) k_pencil_density_reg(FftGeom g, const cplx<T>* __restrict__ W,
-                                                            const double* __restrict__ w, int64_t wk, int b0,
-                                                            int nbc, double* __restrict__ rho_k, int first) {
-  constexpr int PLANE = N0 * N0;
-  const int L0 = g.L[0], M0 = g.M[0];
-  const int k = blockIdx.z;
-  const int pidx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (pidx >= PLANE) return;
-  double* rk = rho_k + (size_t)k * N0 * PLANE + pidx;
-  if (first)
-    rdft_detail::StaticFor<0, N0>::run([&](auto rc) { rk[decltype(rc)::value * PLANE] = 0.0; });
-  const int hi0 = N0 - (L0 - M0 - 1);
-  for (int bl = 0; bl < nbc; ++bl) {
-    const double wb = w[(size_t)k * wk + b0 + bl];
-    if (wb == 0.0) continue;
-    const cplx<T>* base = W + ((size_t)k * nbc + bl) * L0 * (size_t)PLANE + pidx;
-    const cplx<T>* wrap = base - (ptrdiff_t)(N0 - L0) * PLANE;
-    cplx<T> x[N0];
-    rdft_detail::StaticFor<0, N0>::run([&](auto rc) {
-      constexpr int r = decltype(rc)::value;
-      x[r] = r <= M0 ? base[r * PLANE] : (r >= hi0 ? wrap[r * PLANE] : mk<T>(0, 0));
-    });
-    rdft<N0, +1>(x);
-    rdft_detail::StaticFor<0, N0>::run([&](auto rc) {
-      constexpr int r = decltype(rc)::value;
-      rk[r * PLANE] += wb * ((double)x[r].x * (double)x[r].x + (double)x[r].y * (double)x[r].y);
-    });
-  }
-}
-
-// rho[r] = scale sum_k rho_k[k][r], k in order.
-__global__ void k_density_sum(int nk, int64_t N, const double* __restrict__ rho_k, double scale,
+// rho[r] = scale sum_s rho_s[s][r] over the nsum accumulators (k, band group), in order.
+__global__ void k_density_sum(int nsum, int64_t N, const double* __restrict__ rho_s, double scale,
                               double* __restrict__ rho) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
     double a = 0.0;
-    for (int k = 0; k < nk; ++k) a += rho_k[(int64_t)k * N + i];
+    for (int k = 0; k < nsum; ++k) a += rho_s[(int64_t)k * N + i];
     rho[i] = scale * a;
   }
 }
 
-// K1 and K3 with whole transforms in registers (cubic box, N <= 48): a CTA
-// takes PLR planes of one (band, k), N threads per plane, the planes in shared
-// memory with rows padded to N + 1. K1: sphere scatter, one thread per
-// occupied row runs the axis-2 inverse DFT, then one thread per column the
-// axis-1 inverse DFT and writes the column (coalesced over i2) to W. K3: one
-// thread per column loads it from W and runs the axis-1 forward DFT, one
-// thread per occupied row the axis-2 forward DFT, then the sphere gather + t c.
-// Two barriers after the staging, instead of two per radix pass.
-constexpr int PLR = 4;  // planes per CTA
-
-template <int N>
-__device__ __forceinline__ int occ_row(int rr, int M, int L) {  // memory row of occupied row rr
-  return rr <= M ? rr : rr + N - L;
-}
-
-template <typename T, typename SIO, int N>
-__global__ void __launch_bounds__(PLR * N) k_plane_inverse_reg(FftGeom g, const int* __restrict__ plane_ptr,
-                                                              const int* __restrict__ plane_g,
-                                                              const int* __restrict__ plane_pos,
-                                                              const SIO* __restrict__ c, cplx<T>* __restrict__ W,
-                                                              int64_t ck, int b0, int nbc, int npw_max) {
-  constexpr int LDS = N + 1, PS = N * LDS;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  cplx<T>* S = reinterpret_cast<cplx<T>*>(smem_raw);  // [PLR][N][LDS]
-  const int L0 = g.L[0], L1 = g.L[1], M1 = g.M[1];
-  const int jb = blockIdx.x * PLR, bl = blockIdx.y, k = blockIdx.z;
-  const int np = min(PLR, L0 - jb);
-  for (int i = threadIdx.x; i < PLR * PS; i += blockDim.x) S[i] = mk<T>(0, 0);
-  __syncthreads();
-  const size_t crow = (size_t)k * ck + (size_t)(b0 + bl) * npw_max;
-  const int* pp = plane_ptr + k * L0 + jb;
-  const int e0 = pp[0], e1 = pp[np];
-  for (int e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
-    int q = 0;
-#pragma unroll
-    for (int qq = 1; qq < PLR; ++qq) q += (qq < np && e >= pp[qq]) ? 1 : 0;
-    const int pos = plane_pos[e], i1 = pos / N, i2 = pos - i1 * N;
-    S[q * PS + i1 * LDS + i2] = ld<T>(c, crow + plane_g[e]);
-  }
-  __syncthreads();
-  const int p = threadIdx.x / N, lane = threadIdx.x - p * N;
-  if (p < np && lane < L1) {  // axis 2 (rows), occupied rows only
-    cplx<T>* row = S + p * PS + occ_row<N>(lane, M1, L1) * LDS;
-    cplx<T> x[N];
-    rdft_detail::StaticFor<0, N>::run([&](auto qc) { x[decltype(qc)::value] = row[decltype(qc)::value]; });
-    rdft<N, +1>(x);
-    rdft_detail::StaticFor<0, N>::run([&](auto qc) { row[decltype(qc)::value] = x[decltype(qc)::value]; });
-  }
-  __syncthreads();
-  if (p < np) {  // axis 1 (columns): the whole column out to W
-    const cplx<T>* col = S + p * PS + lane;
-    cplx<T> x[N];
-    rdft_detail::StaticFor<0, N>::run([&](auto rc) {
-      constexpr int r = decltype(rc)::value;
-      x[r] = col[r * LDS];
-    });
-    rdft<N, +1>(x);
-    cplx<T>* dst = W + (((size_t)k * nbc + bl) * L0 + jb + p) * (size_t)(N * N) + lane;
-    rdft_detail::StaticFor<0, N>::run([&](auto rc) {
-      constexpr int r = decltype(rc)::value;
-      dst[r * N] = x[r];
-    });
-  }
-}
-
-template <typename T, typename SIO, int N>
-__global__ void __launch_bounds__(PLR * N) k_plane_forward_reg(
-    FftGeom g, const int* __restrict__ plane_ptr, const int* __restrict__ plane_g, const int* __restrict__ plane_pos,
-    const int* __restrict__ npw, const SIO* __restrict__ c, SIO* __restrict__ out, const cplx<T>* __restrict__ W,
-    const T* __restrict__ t, int64_t ck, int64_t ok, int b0, int nbc, int npw_max) {
-  constexpr int LDS = N + 1, PS = N * LDS;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  cplx<T>* S = reinterpret_cast<cplx<T>*>(smem_raw);  // [PLR][N][LDS]
-  const int L0 = g.L[0], L1 = g.L[1], M1 = g.M[1];
-  const int jb = blockIdx.x * PLR, bl = blockIdx.y, k = blockIdx.z;
-  const int np = min(PLR, L0 - jb);
-  const int p = threadIdx.x / N, lane = threadIdx.x - p * N;
-  const int hi1 = N - (L1 - M1 - 1);
-  if (p < np) {  // axis 1 (columns) forward; keep the occupied rows
-    const cplx<T>* src = W + (((size_t)k * nbc + bl) * L0 + jb + p) * (size_t)(N * N) + lane;
-    cplx<T> x[N];
-    rdft_detail::StaticFor<0, N>::run([&](auto rc) {
-      constexpr int r = decltype(rc)::value;
-      x[r] = src[r * N];
-    });
-    rdft<N, -1>(x);
-    cplx<T>* col = S + p * PS + lane;
-    rdft_detail::StaticFor<0, N>::run([&](auto rc) {
-      constexpr int r = decltype(rc)::value;
-      if (r <= M1 || r >= hi1) col[r * LDS] = x[r];
-    });
-  }
-  __syncthreads();
-  if (p < np && lane < L1) {  // axis 2 (rows) forward, occupied rows only
-    cplx<T>* row = S + p * PS + occ_row<N>(lane, M1, L1) * LDS;
-    cplx<T> x[N];
-    rdft_detail::StaticFor<0, N>::run([&](auto qc) { x[decltype(qc)::value] = row[decltype(qc)::value]; });
-    rdft<N, -1>(x);
-    rdft_detail::StaticFor<0, N>::run([&](auto qc) { row[decltype(qc)::value] = x[decltype(qc)::value]; });
-  }
-  __syncthreads();
-  const size_t crow = (size_t)k * ck + (size_t)(b0 + bl) * npw_max;
-  const size_t orow = (size_t)k * ok + (size_t)(b0 + bl) * npw_max;
-  const T* tk = t + (size_t)k * npw_max;
-  const int* pp = plane_ptr + k * L0 + jb;
-  const int e0 = pp[0], e1 = pp[np];
-  for (int e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
-    int q = 0;
-#pragma unroll
-    for (int qq = 1; qq < PLR; ++qq) q += (qq < np && e >= pp[qq]) ? 1 : 0;
-    const int pos = plane_pos[e], i1 = pos / N, i2 = pos - i1 * N;
-    const int gi = plane_g[e];
-    const cplx<T> cv = ld<T>(c, crow + gi);
-    st(out, orow + gi, S[q * PS + i1 * LDS + i2] + scale(cv, tk[gi]));
-  }
-  if (jb == 0) {
-    for (int gi = npw[k] + threadIdx.x; gi < npw_max; gi += blockDim.x) st(out, orow + gi, mk<T>(0, 0));
-  }
-}
-
-// K3: forward FFT along axes 1 and 2, sphere gather, + t c, padding zeroed.
-template <typename T, typename SIO, unsigned C1, unsigned C2, int NT = 256>
-__global__ void __launch_bounds__(NT, (fft_minb<T, NT, (C1 && C2)>())) k_plane_forward(
-    FftGeom g, const int* __restrict__ plane_ptr, const int* __restrict__ plane_g,
-    const int* __restrict__ plane_pos, const int* __restrict__ npw, const SIO* __restrict__ c,
-    SIO* __restrict__ out, const cplx<T>* __restrict__ W, const T* __restrict__ t,
-    const cplx<T>* __restrict__ tw1, const cplx<T>* __restrict__ tw2, int64_t ck, int64_t ok, int b0, int nbc,
-    int npw_max) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int n1 = g.n[1], n2 = g.n[2], L0 = g.L[0];
-  const int j0 = blockIdx.x, bl = blockIdx.y, k = blockIdx.z;
-  cplx<T>* S = reinterpret_cast<cplx<T>*>(smem_raw);
-  cplx<T>* t1 = S + n1 * n2;
-  cplx<T>* t2 = t1 + n1;
-  for (int i = threadIdx.x; i < n1; i += blockDim.x) t1[i] = tw1[i];
-  for (int i = threadIdx.x; i < n2; i += blockDim.x) t2[i] = tw2[i];
-  const cplx<T>* src = W + (((size_t)k * nbc + bl) * L0 + j0) * (size_t)(n1 * n2);
-  for (int i = threadIdx.x; i < n1 * n2; i += blockDim.x) S[i] = src[i];
-  __syncthreads();
-  fft_any<T, true, -1, C1>(S, n2, g.plan[1], 1, n2, n2, n2, t1);
-  fft_any<T, false, -1, C2>(S, g.L[1], g.plan[2], n2, 1, g.M[1], n1, t2);
-  const size_t crow = (size_t)k * ck + (size_t)(b0 + bl) * npw_max;
-  const size_t orow = (size_t)k * ok + (size_t)(b0 + bl) * npw_max;
-  const int e0 = plane_ptr[k * L0 + j0], e1 = plane_ptr[k * L0 + j0 + 1];
-  const T* tk = t + (size_t)k * npw_max;
-  for (int e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
-    const int gi = plane_g[e];
-    cplx<T> cv = ld<T>(c, crow + gi);
-    st(out, orow + gi, S[plane_pos[e]] + scale(cv, tk[gi]));
-  }
-  if (j0 == 0) {
-    for (int gi = npw[k] + threadIdx.x; gi < npw_max; gi += blockDim.x) st(out, orow + gi, mk<T>(0, 0));
+// Sphere slots that name the box cell of another slot of the same k (not met
+// in a sphere of distinct G): the transforms read and write the last such slot,
+// the others get its local term with their own kinetic term here.
+template <typename T, typename SIO>
+__global__ void k_duplicate_slots(const int* __restrict__ dup, int ndup, const SIO* __restrict__ c, int64_t ck,
+                                  SIO* __restrict__ out, int64_t ok, const T* __restrict__ t, int nb, int npw_max) {
+  const int total = ndup * nb;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    const int* d = dup + 3 * (i / nb);
+    const int b = i % nb, k = d[0], g = d[1], h = d[2];
+    const size_t ci = (size_t)k * ck + (size_t)b * npw_max, oi = (size_t)k * ok + (size_t)b * npw_max;
+    const T* tk = t + (size_t)k * npw_max;
+    const cplx<T> local = ld<T>(out, oi + h) - scale(ld<T>(c, ci + h), tk[h]);
+    st(out, oi + g, local + scale(ld<T>(c, ci + g), tk[g]));
   }
 }
 
@@ -766,13 +415,6 @@ static int ensure_buf(void** p, size_t* have, size_t need) {
   return GWB_OK;
 }
 
-static size_t plane_smem(const FftGeom& g, size_t es) {
-  return (size_t)(g.n[1] * g.n[2] + g.n[1] + g.n[2]) * es;
-}
-static size_t pencil_smem(const FftGeom& g, size_t es) {
-  return (size_t)(g.n[0] * g.n[2] + g.n[0]) * es;
-}
-
 // G slices of the becp reduction: enough CTAs to fill the GPU (4 per SM)
 // with every slice at least 256 plane waves long.
 static int nl_slices(const gwb_ham* h, int nb) {
@@ -783,87 +425,47 @@ static int nl_slices(const gwb_ham* h, int nb) {
   return std::max(1, std::min(want, cap));
 }
 
-// Compile-time FFT plans instantiated for the cubic boxes of the workloads
-// (24 = 8*3, 36 = 4*3*3, 72 = 8*3*3, 96 = 8*4*3); any other box runs the
-// runtime-plan kernels.
-constexpr unsigned kCode24 = 0x38u, kCode36 = 0x334u, kCode72 = 0x338u, kCode96 = 0x348u;
-
-// The shared-memory kernels of one band chunk (K1, K2, K3) with NT threads per block.
-template <typename T, typename SIO, unsigned C, int NT>
-static int local_shared(gwb_ham* h, const SIO* c, int64_t ck, SIO* out, int64_t ok, cplx<T>* W, const T* v,
-                        const T* t, const cplx<T>* tw0, const cplx<T>* tw1, const cplx<T>* tw2, int b0, int cb,
-                        cudaStream_t st, size_t smA, size_t smB) {
+// Bands per chunk and the chunk's scratch (W: L0 planes, W2: the disc's rows):
+// as few chunks as the budget allows, all of (nearly) equal size. When the
+// device has no room for that scratch, chunks of kWBudgetLowMB.
+static int chunk_scratch(gwb_ham* h, int nb, size_t es, int* nbc) {
   const FftGeom& g = h->g;
-  GWB_CUDA_TRY(allow_smem(k_plane_inverse<T, SIO, C, C, NT>));
-  GWB_CUDA_TRY(allow_smem(k_plane_forward<T, SIO, C, C, NT>));
-  GWB_CUDA_TRY(allow_smem(k_pencil_vloc<T, C, NT>));
-  dim3 gA(g.L[0], cb, h->nk), gB(g.n[1], cb, h->nk);
-  k_plane_inverse<T, SIO, C, C, NT><<<gA, NT, smA, st>>>(g, h->d_plane_ptr, h->d_plane_g, h->d_plane_pos, c, W, tw1,
-                                                        tw2, ck, b0, cb, h->npw_max);
-  k_pencil_vloc<T, C, NT><<<gB, NT, smB, st>>>(g, W, v, tw0, cb);
-  k_plane_forward<T, SIO, C, C, NT><<<gA, NT, smA, st>>>(g, h->d_plane_ptr, h->d_plane_g, h->d_plane_pos, h->d_npw,
-                                                        c, out, W, t, tw1, tw2, ck, ok, b0, cb, h->npw_max);
-  return GWB_OK;
+  const size_t per_band = (size_t)h->nk * ((size_t)g.L[0] * g.n[1] + g.nrow) * g.n[2] * es;
+  auto bands = [&](size_t budget) {
+    const size_t most = std::max<size_t>(1, budget / per_band);
+    const size_t nchunks = ((size_t)nb + most - 1) / most;
+    return (int)(((size_t)nb + nchunks - 1) / nchunks);
+  };
+  *nbc = bands(h->w_budget ? h->w_budget : w_budget_bytes());
+  int rc = ensure_buf(&h->d_W, &h->W_bytes, per_band * *nbc);
+  const int low = bands((size_t)kWBudgetLowMB << 20);
+  if (rc == GWB_ERR_ALLOC && low < *nbc) {
+    *nbc = low;
+    rc = ensure_buf(&h->d_W, &h->W_bytes, per_band * *nbc);
+  }
+  return rc;
 }
 
-template <typename T, typename SIO, unsigned C>
-static int local_chunks(gwb_ham* h, const SIO* c, int64_t ck, SIO* out, int64_t ok, int nb, int nbc,
-                        cudaStream_t st, size_t smA, size_t smB) {
+template <typename T> static FftRun<T> fft_run(const gwb_ham* h, int nbc) {
   const FftGeom& g = h->g;
   const bool dbl = sizeof(T) == 8;
-  const cplx<T>* tw0 = dbl ? (const cplx<T>*)h->d_tw64[0] : (const cplx<T>*)h->d_tw32[0];
-  const cplx<T>* tw1 = dbl ? (const cplx<T>*)h->d_tw64[1] : (const cplx<T>*)h->d_tw32[1];
-  const cplx<T>* tw2 = dbl ? (const cplx<T>*)h->d_tw64[2] : (const cplx<T>*)h->d_tw32[2];
-  const T* v = dbl ? (const T*)h->d_v64 : (const T*)h->d_v32;
-  const T* t = dbl ? (const T*)h->d_t64 : (const T*)h->d_t32;
-  cplx<T>* W = (cplx<T>*)h->d_W;
-  const bool cubic = g.n[0] == g.n[1] && g.n[1] == g.n[2];
-  const int nreg = (cubic && g.n[0] == 36 && C == kCode36) ? 36 : ((cubic && g.n[0] == 24 && C == kCode24) ? 24 : 0);
-  const size_t smR = (size_t)PLR * nreg * (nreg + 1) * sizeof(cplx<T>);
-  if (nreg == 36) {
-    GWB_CUDA_TRY(allow_smem(k_plane_inverse_reg<T, SIO, 36>));
-    GWB_CUDA_TRY(allow_smem(k_plane_forward_reg<T, SIO, 36>));
-  } else if (nreg == 24) {
-    GWB_CUDA_TRY(allow_smem(k_plane_inverse_reg<T, SIO, 24>));
-    GWB_CUDA_TRY(allow_smem(k_plane_forward_reg<T, SIO, 24>));
-  }
-  for (int b0 = 0; b0 < nb; b0 += nbc) {
-    const int cb = std::min(nbc, nb - b0);
-    dim3 gA(g.L[0], cb, h->nk), gB(g.n[1], cb, h->nk), gP((g.L[0] + PLR - 1) / PLR, cb, h->nk);
-    dim3 gR((g.n[1] * g.n[2] + 127) / 128, cb, h->nk);
-    if (nreg == 36) {
-      k_plane_inverse_reg<T, SIO, 36><<<gP, PLR * 36, smR, st>>>(g, h->d_plane_ptr, h->d_plane_g, h->d_plane_pos, c,
-                                                                 W, ck, b0, cb, h->npw_max);
-      k_pencil_vloc_reg<T, 36><<<gR, 128, 0, st>>>(g, W, v, cb);
-      k_plane_forward_reg<T, SIO, 36><<<gP, PLR * 36, smR, st>>>(g, h->d_plane_ptr, h->d_plane_g, h->d_plane_pos,
-                                                                 h->d_npw, c, out, W, t, ck, ok, b0, cb, h->npw_max);
-    } else if (nreg == 24) {
-      k_plane_inverse_reg<T, SIO, 24><<<gP, PLR * 24, smR, st>>>(g, h->d_plane_ptr, h->d_plane_g, h->d_plane_pos, c,
-                                                                 W, ck, b0, cb, h->npw_max);
-      k_pencil_vloc_reg<T, 24><<<gR, 128, 0, st>>>(g, W, v, cb);
-      k_plane_forward_reg<T, SIO, 24><<<gP, PLR * 24, smR, st>>>(g, h->d_plane_ptr, h->d_plane_g, h->d_plane_pos,
-                                                                 h->d_npw, c, out, W, t, ck, ok, b0, cb, h->npw_max);
-    } else {
-      // threads per block of the large compile-time boxes (72^3, 96^3):
-      // gwb_ham_set_fft_threads, else 512 (float32: two 73 KB planes per SM)
-      // and 1024 (float64: one 147 KB plane per SM). Measured on the 96^3
-      // box of si216, 480 bands: float32 6.35 -> 6.26 ms, float64 16.7 ->
-      // 12.0 ms against 256 threads.
-      const int nt = h->fft_nt[dbl ? 1 : 0] ? h->fft_nt[dbl ? 1 : 0] : (dbl ? 1024 : 512);
-      int rc = GWB_OK;
-      if constexpr (C == kCode96 || C == kCode72) {
-        if (nt == 1024) rc = local_shared<T, SIO, C, 1024>(h, c, ck, out, ok, W, v, t, tw0, tw1, tw2, b0, cb, st, smA, smB);
-        else if (nt == 512) rc = local_shared<T, SIO, C, 512>(h, c, ck, out, ok, W, v, t, tw0, tw1, tw2, b0, cb, st, smA, smB);
-        else rc = local_shared<T, SIO, C, 256>(h, c, ck, out, ok, W, v, t, tw0, tw1, tw2, b0, cb, st, smA, smB);
-      } else {
-        rc = local_shared<T, SIO, C, 256>(h, c, ck, out, ok, W, v, t, tw0, tw1, tw2, b0, cb, st, smA, smB);
-      }
-      if (rc != GWB_OK) return rc;
-    }
-    GWB_LAUNCH_CHECK();
-    count_launches(3);
-  }
-  return GWB_OK;
+  FftRun<T> f{};
+  f.n0 = g.n[0], f.n1 = g.n[1], f.n2 = g.n[2];
+  f.M0 = g.M[0], f.L0 = g.L[0], f.M2 = g.M[2];
+  f.nk = h->nk, f.nrow = g.nrow, f.nbc = nbc, f.npw_max = h->npw_max;
+  f.map = h->d_map, f.rowof = h->d_rowof, f.npw = h->d_npw;
+  f.tw0 = dbl ? (const cplx<T>*)h->d_tw64[0] : (const cplx<T>*)h->d_tw32[0];
+  f.tw1 = dbl ? (const cplx<T>*)h->d_tw64[1] : (const cplx<T>*)h->d_tw32[1];
+  f.tw2 = dbl ? (const cplx<T>*)h->d_tw64[2] : (const cplx<T>*)h->d_tw32[2];
+  f.v = dbl ? (const T*)h->d_v64 : (const T*)h->d_v32;
+  f.t = dbl ? (const T*)h->d_t64 : (const T*)h->d_t32;
+  f.W = (cplx<T>*)h->d_W;
+  return f;
+}
+
+// rows' scratch of a chunk: behind its planes
+template <typename T> static void place_rows(const gwb_ham* h, FftRun<T>* f) {
+  f->W2 = f->W + (size_t)h->nk * f->nbc * f->L0 * f->n1 * f->n2;
 }
 
 int tc_becp_d_planes(int nk, int nb, int nproj, const cplx<double>* becp, const double* D, void* planes, int64_t ldq,
@@ -919,28 +521,30 @@ static int nonlocal_tc(gwb_ham* h, const cplx<double>* c, int64_t ck, cplx<doubl
 // out = T c + local(c): the kinetic and FFT local terms, band chunks sized to L2.
 template <typename T, typename SIO>
 static int local_term(gwb_ham* h, const SIO* c, int64_t ck, SIO* out, int64_t ok, int nb, cudaStream_t st) {
-  const FftGeom& g = h->g;
-  const size_t es = sizeof(cplx<T>);
-  const size_t plane_elems = (size_t)g.n[1] * g.n[2];
-  const size_t per_band = (size_t)h->nk * g.L[0] * plane_elems * es;
-  // balanced chunks: as few as the L2 budget allows, all of (nearly) equal size
-  const size_t budget = std::max(h->w_budget ? h->w_budget : w_budget_bytes(), per_band);
-  const size_t max_nbc = std::max<size_t>(1, budget / per_band);
-  const size_t nchunks = ((size_t)nb + max_nbc - 1) / max_nbc;
-  int nbc = (int)(((size_t)nb + nchunks - 1) / nchunks);
-  if (nbc < 1) nbc = 1;
-  int rc = ensure_buf(&h->d_W, &h->W_bytes, per_band * nbc);
+  int nbc = 0;
+  const int rc = chunk_scratch(h, nb, sizeof(cplx<T>), &nbc);
   if (rc) return rc;
-  const size_t smA = plane_smem(g, es), smB = pencil_smem(g, es);
-  const unsigned c0 = g.plan[0].code, c1 = g.plan[1].code, c2 = g.plan[2].code;
-  const bool cubic = c0 == c1 && c1 == c2;
-  int rcl;
-  if (cubic && c0 == kCode24) rcl = local_chunks<T, SIO, kCode24>(h, c, ck, out, ok, nb, nbc, st, smA, smB);
-  else if (cubic && c0 == kCode36) rcl = local_chunks<T, SIO, kCode36>(h, c, ck, out, ok, nb, nbc, st, smA, smB);
-  else if (cubic && c0 == kCode72) rcl = local_chunks<T, SIO, kCode72>(h, c, ck, out, ok, nb, nbc, st, smA, smB);
-  else if (cubic && c0 == kCode96) rcl = local_chunks<T, SIO, kCode96>(h, c, ck, out, ok, nb, nbc, st, smA, smB);
-  else rcl = local_chunks<T, SIO, 0u>(h, c, ck, out, ok, nb, nbc, st, smA, smB);
-  return rcl;
+  FftRun<T> f = fft_run<T>(h, nbc);
+  f.c = c, f.out = out, f.ck = ck, f.ok = ok;
+  f.io64 = sizeof(SIO) == 16;
+  for (int b0 = 0; b0 < nb; b0 += nbc) {
+    f.b0 = b0;
+    f.nbc = std::min(nbc, nb - b0);
+    place_rows(h, &f);
+    GWB_CUDA_TRY(fft_rows_inverse(f, st));
+    GWB_CUDA_TRY(fft_cols_inverse(f, st));
+    GWB_CUDA_TRY(fft_pencil_vloc(f, st));
+    GWB_CUDA_TRY(fft_cols_forward(f, st));
+    GWB_CUDA_TRY(fft_rows_forward(f, st));
+    count_launches(5);
+  }
+  if (h->ndup) {
+    k_duplicate_slots<T, SIO><<<std::min(148 * 4, (h->ndup * nb + 255) / 256), 256, 0, st>>>(
+        h->d_dup, h->ndup, c, ck, out, ok, f.t, nb, h->npw_max);
+    GWB_LAUNCH_CHECK();
+    count_launches(1);
+  }
+  return GWB_OK;
 }
 
 // The nonlocal slices: enough G slices to fill the GPU for this band count.
@@ -1014,75 +618,37 @@ static int apply_hs_impl(gwb_ham* h, const SIO* c, int64_t ck, SIO* out_h, int64
   return GWB_OK;
 }
 
-// Density of nb bands (float64 FFTs): K1 per band chunk into W, then the
-// pencil kernel accumulating w |psi|^2 into rho_k, finally the k sum.
-template <typename SIO, unsigned C>
-static int density_chunks(gwb_ham* h, const SIO* c, int64_t ck, int nb, int nbc, const double* w, int64_t wk,
-                          cudaStream_t st, size_t smA, size_t smB) {
-  using T = double;
-  const FftGeom& g = h->g;
-  const cplx<T>* tw0 = (const cplx<T>*)h->d_tw64[0];
-  const cplx<T>* tw1 = (const cplx<T>*)h->d_tw64[1];
-  const cplx<T>* tw2 = (const cplx<T>*)h->d_tw64[2];
-  cplx<T>* W = (cplx<T>*)h->d_W;
-  const bool cubic = g.n[0] == g.n[1] && g.n[1] == g.n[2];
-  const int nreg = (cubic && g.n[0] == 36 && C == kCode36) ? 36 : ((cubic && g.n[0] == 24 && C == kCode24) ? 24 : 0);
-  const size_t smR = (size_t)PLR * nreg * (nreg + 1) * sizeof(cplx<T>);
-  GWB_CUDA_TRY(allow_smem(k_plane_inverse<T, SIO, C, C>));
-  GWB_CUDA_TRY(allow_smem(k_pencil_density<T, C>));
-  if (nreg == 36) GWB_CUDA_TRY(allow_smem(k_plane_inverse_reg<T, SIO, 36>));
-  if (nreg == 24) GWB_CUDA_TRY(allow_smem(k_plane_inverse_reg<T, SIO, 24>));
-  for (int b0 = 0; b0 < nb; b0 += nbc) {
-    const int cb = std::min(nbc, nb - b0);
-    const int first = b0 == 0;
-    dim3 gA(g.L[0], cb, h->nk), gP((g.L[0] + PLR - 1) / PLR, cb, h->nk);
-    dim3 gR((g.n[1] * g.n[2] + 127) / 128, 1, h->nk), gB(g.n[1], 1, h->nk);
-    if (nreg == 36) {
-      k_plane_inverse_reg<T, SIO, 36><<<gP, PLR * 36, smR, st>>>(g, h->d_plane_ptr, h->d_plane_g, h->d_plane_pos, c,
-                                                                 W, ck, b0, cb, h->npw_max);
-      k_pencil_density_reg<T, 36><<<gR, 128, 0, st>>>(g, W, w, wk, b0, cb, h->d_rhok, first);
-    } else if (nreg == 24) {
-      k_plane_inverse_reg<T, SIO, 24><<<gP, PLR * 24, smR, st>>>(g, h->d_plane_ptr, h->d_plane_g, h->d_plane_pos, c,
-                                                                 W, ck, b0, cb, h->npw_max);
-      k_pencil_density_reg<T, 24><<<gR, 128, 0, st>>>(g, W, w, wk, b0, cb, h->d_rhok, first);
-    } else {
-      k_plane_inverse<T, SIO, C, C><<<gA, 256, smA, st>>>(g, h->d_plane_ptr, h->d_plane_g, h->d_plane_pos, c, W,
-                                                         tw1, tw2, ck, b0, cb, h->npw_max);
-      k_pencil_density<T, C><<<gB, 256, smB, st>>>(g, W, tw0, w, wk, b0, cb, h->d_rhok, first);
-    }
-    GWB_LAUNCH_CHECK();
-    count_launches(2);
-  }
-  return GWB_OK;
-}
-
+// Density of nb bands (float64 FFTs): axes 2 and 1 of a band chunk into W, then
+// the pencil kernel accumulating w |psi|^2 per k and band group, finally their sum.
 template <typename SIO>
 static int density_impl(gwb_ham* h, const SIO* c, int64_t ck, int nb, const double* w, int64_t wk, double scale,
                         double* rho, cudaStream_t st) {
   const FftGeom& g = h->g;
-  const size_t es = sizeof(cplx<double>);
   const size_t N = (size_t)g.n[0] * g.n[1] * g.n[2];
-  const size_t per_band = (size_t)h->nk * g.L[0] * g.n[1] * g.n[2] * es;
-  const size_t budget = std::max(h->w_budget ? h->w_budget : w_budget_bytes(), per_band);
-  const size_t max_nbc = std::max<size_t>(1, budget / per_band);
-  const size_t nchunks = ((size_t)nb + max_nbc - 1) / max_nbc;
-  int nbc = (int)(((size_t)nb + nchunks - 1) / nchunks);
-  if (nbc < 1) nbc = 1;
-  int rc = ensure_buf(&h->d_W, &h->W_bytes, per_band * nbc);
+  int nbc = 0;
+  int rc = chunk_scratch(h, nb, sizeof(cplx<double>), &nbc);
   if (rc) return rc;
-  rc = ensure_buf((void**)&h->d_rhok, &h->rhok_bytes, (size_t)h->nk * N * sizeof(double));
+  // band groups: about 8 blocks of 16 pencils per SM, at least two bands each;
+  // the same for every chunking, so that chunks do not change the sums
+  const int64_t blocks = (int64_t)h->nk * ((g.n[1] * g.n[2] + 15) / 16);
+  const int ngrp = (int)std::max<int64_t>(1, std::min<int64_t>((8 * 148 + blocks - 1) / blocks, nb / 2));
+  rc = ensure_buf((void**)&h->d_rhok, &h->rhok_bytes, (size_t)h->nk * ngrp * N * sizeof(double));
   if (rc) return rc;
-  const size_t smA = plane_smem(g, es), smB = pencil_smem(g, es);
-  const unsigned c0 = g.plan[0].code, c1 = g.plan[1].code, c2 = g.plan[2].code;
-  const bool cubic = c0 == c1 && c1 == c2;
-  if (cubic && c0 == kCode24) rc = density_chunks<SIO, kCode24>(h, c, ck, nb, nbc, w, wk, st, smA, smB);
-  else if (cubic && c0 == kCode36) rc = density_chunks<SIO, kCode36>(h, c, ck, nb, nbc, w, wk, st, smA, smB);
-  else if (cubic && c0 == kCode72) rc = density_chunks<SIO, kCode72>(h, c, ck, nb, nbc, w, wk, st, smA, smB);
-  else if (cubic && c0 == kCode96) rc = density_chunks<SIO, kCode96>(h, c, ck, nb, nbc, w, wk, st, smA, smB);
-  else rc = density_chunks<SIO, 0u>(h, c, ck, nb, nbc, w, wk, st, smA, smB);
-  if (rc) return rc;
-  const int blocks = (int)std::min<size_t>((N + 255) / 256, 148 * 8);
-  k_density_sum<<<blocks, 256, 0, st>>>(h->nk, (int64_t)N, h->d_rhok, scale, rho);
+  FftRun<double> f = fft_run<double>(h, nbc);
+  f.c = c, f.ck = ck, f.io64 = sizeof(SIO) == 16;
+  f.w = w, f.wk = wk, f.rho = h->d_rhok, f.ngrp = ngrp;
+  for (int b0 = 0; b0 < nb; b0 += nbc) {
+    f.b0 = b0;
+    f.nbc = std::min(nbc, nb - b0);
+    f.first = b0 == 0;
+    place_rows(h, &f);
+    GWB_CUDA_TRY(fft_rows_inverse(f, st));
+    GWB_CUDA_TRY(fft_cols_inverse(f, st));
+    GWB_CUDA_TRY(fft_pencil_density(f, st));
+    count_launches(3);
+  }
+  const int sum_blocks = (int)std::min<size_t>((N + 255) / 256, 148 * 8);
+  k_density_sum<<<sum_blocks, 256, 0, st>>>(h->nk * ngrp, (int64_t)N, h->d_rhok, scale, rho);
   GWB_LAUNCH_CHECK();
   count_launches(1);
   return GWB_OK;
@@ -1110,7 +676,7 @@ int gwb_ham_create(const gwb_ham_geometry* geom, int device, gwb_ham** out) {
   FftGeom& g = h->g;
   for (int a = 0; a < 3; ++a) {
     g.n[a] = geom->n[a];
-    if (!plan_axis(g.n[a], &g.plan[a])) {
+    if (!axis_ok(g.n[a])) {
       delete h;
       set_error("FFT axis length " + std::to_string(geom->n[a]) + " unsupported (need <=128, factors 2,3,5,7)");
       return GWB_ERR_ARG;
@@ -1119,7 +685,11 @@ int gwb_ham_create(const gwb_ham_geometry* geom, int device, gwb_ham** out) {
   const int n0 = g.n[0], n1 = g.n[1], n2 = g.n[2];
   const int64_t nbox = (int64_t)n0 * n1 * n2;
   h->npw_host.assign(geom->npw, geom->npw + geom->nk);
-  // Miller extents over all k
+  // box coordinates of every sphere point, Miller extents over all k
+  struct Cell {
+    uint8_t i0, i1, i2;
+  };
+  std::vector<Cell> cell((size_t)h->nk * h->npw_max);
   int M[3] = {0, 0, 0};
   for (int k = 0; k < h->nk; ++k) {
     const int64_t np_k = h->npw_host[k];
@@ -1135,7 +705,9 @@ int gwb_ham_create(const gwb_ham_geometry* geom, int device, gwb_ham** out) {
         set_error("flat_idx out of the box");
         return GWB_ERR_ARG;
       }
-      const int idx[3] = {(int)(f / ((int64_t)n1 * n2)), (int)((f / n2) % n1), (int)(f % n2)};
+      const unsigned u = (unsigned)f, q = u / (unsigned)n2, i0 = q / (unsigned)n1;
+      const int idx[3] = {(int)i0, (int)(q - i0 * n1), (int)(u - q * n2)};
+      cell[(size_t)k * h->npw_max + gi] = {(uint8_t)idx[0], (uint8_t)idx[1], (uint8_t)idx[2]};
       for (int a = 0; a < 3; ++a) {
         const int m = idx[a] <= g.n[a] / 2 ? idx[a] : idx[a] - g.n[a];
         M[a] = std::max(M[a], std::abs(m));
@@ -1147,29 +719,28 @@ int gwb_ham_create(const gwb_ham_geometry* geom, int device, gwb_ham** out) {
     g.M[a] = g.L[a] == g.n[a] ? g.n[a] : M[a];
   }
   const int L0 = g.L[0];
-  // sphere points grouped by compact axis-0 plane
-  std::vector<int> cnt((size_t)h->nk * L0 + 1, 0);
-  auto compact0 = [&](int i0) -> int {
-    if (g.L[0] == n0) return i0;
-    if (i0 <= g.M[0]) return i0;
-    return i0 - (n0 - L0);
-  };
+  // row slots of the occupied (j0, i1) of each k, and the sphere index of each row point
+  auto compact0 = [&](int i0) -> int { return g.L[0] == n0 || i0 <= g.M[0] ? i0 : i0 - (n0 - L0); };
+  std::vector<int> rowof((size_t)h->nk * L0 * n1, -1);
+  std::vector<int> nrow_k(h->nk, 0);
+  for (int k = 0; k < h->nk; ++k) {
+    int* ro = rowof.data() + (size_t)k * L0 * n1;
+    const Cell* ck = cell.data() + (size_t)k * h->npw_max;
+    for (int64_t gi = 0; gi < h->npw_host[k]; ++gi) ro[compact0(ck[gi].i0) * n1 + ck[gi].i1] = 0;
+    for (int i = 0; i < L0 * n1; ++i)
+      if (ro[i] == 0) ro[i] = nrow_k[k]++;
+  }
+  g.nrow = std::max(1, *std::max_element(nrow_k.begin(), nrow_k.end()));
+  std::vector<int> map((size_t)h->nk * g.nrow * n2, -1), dup;
   for (int k = 0; k < h->nk; ++k)
-    for (int64_t gi = 0; gi < h->npw_host[k]; ++gi) {
-      const int64_t f = geom->flat_idx[(size_t)k * h->npw_max + gi];
-      cnt[(size_t)k * L0 + compact0((int)(f / ((int64_t)n1 * n2))) + 1]++;
+    for (int64_t gi = h->npw_host[k] - 1; gi >= 0; --gi) {
+      const Cell p = cell[(size_t)k * h->npw_max + gi];
+      const int row = rowof[((size_t)k * L0 + compact0(p.i0)) * n1 + p.i1];
+      int& slot = map[((size_t)k * g.nrow + row) * n2 + p.i2];
+      if (slot < 0) slot = (int)gi;
+      else dup.insert(dup.end(), {k, (int)gi, slot});
     }
-  for (size_t i = 1; i < cnt.size(); ++i) cnt[i] += cnt[i - 1];
-  const int total = cnt.back();
-  std::vector<int> pg(std::max(total, 1)), pp(std::max(total, 1));
-  std::vector<int> fill(cnt.begin(), cnt.end() - 1);
-  for (int k = 0; k < h->nk; ++k)
-    for (int64_t gi = 0; gi < h->npw_host[k]; ++gi) {
-      const int64_t f = geom->flat_idx[(size_t)k * h->npw_max + gi];
-      const int slot = fill[(size_t)k * L0 + compact0((int)(f / ((int64_t)n1 * n2)))]++;
-      pg[slot] = (int)gi;
-      pp[slot] = (int)(f % ((int64_t)n1 * n2));
-    }
+  h->ndup = (int)(dup.size() / 3);
   std::vector<int> npw32(h->npw_host.begin(), h->npw_host.end());
   // twiddles exp(-2 pi i t / n), computed in double on the host
   std::vector<cplx<double>> tw64[3];
@@ -1195,9 +766,9 @@ int gwb_ham_create(const gwb_ham_geometry* geom, int device, gwb_ham** out) {
     e = cudaMemcpy((dst), (vec).data(), (vec).size() * sizeof((vec)[0]), cudaMemcpyHostToDevice); \
     if (e != cudaSuccess) return fail(e);                                                   \
   } while (0)
-  GWB_ALLOC_COPY(h->d_plane_ptr, cnt);
-  GWB_ALLOC_COPY(h->d_plane_g, pg);
-  GWB_ALLOC_COPY(h->d_plane_pos, pp);
+  GWB_ALLOC_COPY(h->d_map, map);
+  GWB_ALLOC_COPY(h->d_rowof, rowof);
+  if (h->ndup) GWB_ALLOC_COPY(h->d_dup, dup);
   GWB_ALLOC_COPY(h->d_npw, npw32);
   for (int a = 0; a < 3; ++a) {
     GWB_ALLOC_COPY(h->d_tw64[a], tw64[a]);
@@ -1222,7 +793,7 @@ int gwb_ham_create(const gwb_ham_geometry* geom, int device, gwb_ham** out) {
 
 int gwb_ham_destroy(gwb_ham* h) {
   if (!h) return GWB_OK;
-  void* ptrs[] = {h->d_npw, h->d_plane_ptr, h->d_plane_g, h->d_plane_pos, h->d_t64, h->d_t32, h->d_v64,
+  void* ptrs[] = {h->d_npw, h->d_map, h->d_rowof, h->d_dup, h->d_t64, h->d_t32, h->d_v64,
                   h->d_v32, h->d_p64, h->d_p32, h->d_d64, h->d_d32, h->d_q64, h->d_q32, h->d_W, h->d_part, h->d_bd, h->d_bq,
                   h->d_pplanes, h->d_cplanes, h->d_becp, h->d_bdplanes, h->d_tcwork, h->d_tcstatus, h->d_rhok,
                   h->d_tw64[0], h->d_tw64[1], h->d_tw64[2], h->d_tw32[0], h->d_tw32[1], h->d_tw32[2]};
@@ -1325,9 +896,7 @@ int gwb_ham_set_fft_threads(gwb_ham* h, int32_t threads_fp32, int32_t threads_fp
   GWB_REQUIRE(h, "null handle");
   auto ok = [](int32_t n) { return n == 0 || n == 256 || n == 512 || n == 1024; };
   GWB_REQUIRE(ok(threads_fp32) && ok(threads_fp64), "FFT block threads must be 0, 256, 512 or 1024");
-  h->fft_nt[0] = threads_fp32;
-  h->fft_nt[1] = threads_fp64;
-  return GWB_OK;
+  return GWB_OK;  // a hint: the block sizes of the FFT kernels follow from the axis lengths
 }
 
 int gwb_ham_set_overlap(gwb_ham* h, const double* q, void* stream) {

@@ -6,8 +6,8 @@
 // FFT", 1992, sec. 2.3). The recursion works in place on strided views of the
 // one array, every index and every twiddle is a compile-time constant, so the
 // array lives in registers and a twiddle is an immediate operand; no shared
-// memory, no barriers. Meant for the short box axes (N <= 48) where a thread
-// can hold a whole pencil.
+// memory, no barriers. Meant for the factors (up to 25 points) of the box axes
+// that one thread holds.
 //
 // The twiddle constants cos/sin(2 pi k / N) come from a constexpr evaluator
 // (octant reduction on the integer ratio k/N, then Taylor series on
@@ -62,7 +62,9 @@ constexpr double cis(long k, long n, int which) {
   return which == 0 ? cc : ss;
 }
 
-constexpr int first_radix(int n) { return n % 4 == 0 ? 4 : (n % 3 == 0 ? 3 : (n % 2 == 0 ? 2 : n)); }
+constexpr int first_radix(int n) {
+  return n % 4 == 0 ? 4 : (n % 3 == 0 ? 3 : (n % 2 == 0 ? 2 : (n % 5 == 0 ? 5 : (n % 7 == 0 ? 7 : n))));
+}
 
 template <int I, int N>
 struct StaticFor {
@@ -117,6 +119,33 @@ __host__ __device__ __forceinline__ void small_dft(cplx<T> (&t)[R]) {
     t[2] = a0 - b0;
     t[1] = a1 + b1;
     t[3] = a1 - b1;
+  } else if constexpr (R == 5 || R == 7) {
+    // odd prime length: with s_j = t_j + t_(R-j), d_j = t_j - t_(R-j),
+    // X_k = t_0 + sum_j cos(2 pi j k / R) s_j + SIGN i sum_j sin(2 pi j k / R) d_j
+    // and X_(R-k) the same with the second sum subtracted
+    constexpr int H = (R - 1) / 2;
+    cplx<T> s[H], d[H];
+    const cplx<T> t0 = t[0];
+    cplx<T> sum = t0;
+    StaticFor<0, H>::run([&](auto jc) {
+      constexpr int j = decltype(jc)::value;
+      s[j] = t[j + 1] + t[R - 1 - j];
+      d[j] = t[j + 1] - t[R - 1 - j];
+      sum = sum + s[j];
+    });
+    t[0] = sum;
+    StaticFor<0, H>::run([&](auto kc) {
+      constexpr int k = decltype(kc)::value + 1;
+      cplx<T> a = t0, b = mk<T>((T)0, (T)0);
+      StaticFor<0, H>::run([&](auto jc) {
+        constexpr int j = decltype(jc)::value;
+        constexpr double cd = cis((long)(j + 1) * k, R, 0), sd = SIGN * cis((long)(j + 1) * k, R, 1);
+        a = mk<T>(a.x + (T)cd * s[j].x, a.y + (T)cd * s[j].y);
+        b = mk<T>(b.x + (T)sd * d[j].x, b.y + (T)sd * d[j].y);
+      });
+      t[k] = mk<T>(a.x - b.y, a.y + b.x);
+      t[R - k] = mk<T>(a.x + b.y, a.y - b.x);
+    });
   }
 }
 
@@ -124,7 +153,7 @@ __host__ __device__ __forceinline__ void small_dft(cplx<T> (&t)[R]) {
 // leaves output X[k]: for N = R M, X[kk + M q] lands where sub-DFT q kept its
 // output kk, i.e. at q + R pos_M(kk) (digit reversal over the radix chain).
 constexpr int out_pos(int n, int k) {
-  if (n <= 4) return k;
+  if (n <= 5 || n == 7) return k;
   const int r = first_radix(n), m = n / r;
   return (k / m) + r * out_pos(m, k % m);
 }
@@ -135,7 +164,7 @@ template <int N, int SIGN, int OFF, int STRIDE, typename T, int NT>
 __host__ __device__ __forceinline__ void dit_ip(cplx<T> (&x)[NT]) {
   if constexpr (N == 1) {
     return;
-  } else if constexpr (N <= 4) {
+  } else if constexpr (N <= 5 || N == 7) {
     cplx<T> t[N];
     StaticFor<0, N>::run([&](auto ic) { t[decltype(ic)::value] = x[OFF + STRIDE * decltype(ic)::value]; });
     small_dft<N, SIGN>(t);
@@ -143,7 +172,7 @@ __host__ __device__ __forceinline__ void dit_ip(cplx<T> (&x)[NT]) {
   } else {
     constexpr int R = first_radix(N);
     constexpr int M = N / R;
-    static_assert(R * M == N && R <= 4, "rdft: lengths with prime factors 2 and 3 only");
+    static_assert(R * M == N && R <= 7, "rdft: lengths with prime factors 2, 3, 5 and 7 only");
     StaticFor<0, R>::run([&](auto rc) {
       constexpr int r = decltype(rc)::value;
       dit_ip<M, SIGN, OFF + STRIDE * r, STRIDE * R>(x);

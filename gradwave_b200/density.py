@@ -17,6 +17,7 @@ eigenvectors (the reference would add them to the G = 0 component).
 from __future__ import annotations
 
 import ctypes
+import weakref
 
 import numpy as np
 import torch
@@ -86,8 +87,9 @@ def density_b(coeffs: torch.Tensor, occ: torch.Tensor, kweights: torch.Tensor, b
     dev = coeffs.device
     key = (id(bk), tuple(int(s) for s in shape), dev.index)
     h = _HANDLES.get(key)
-    if h is None or h[1] is not bk:
-        h = (_GeometryHandle(bk, shape, dev), bk)
+    if h is None or h[1]() is not bk:
+        # the handle (and its scratch) goes when bk does
+        h = (_GeometryHandle(bk, shape, dev), weakref.ref(bk, lambda _, key=key: _HANDLES.pop(key, None)))
         _HANDLES[key] = h
     g = h[0]
     return density_from_handle(g._h, g.nk, g.npw_max, g.shape, coeffs, occ, kweights, volume)

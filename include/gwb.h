@@ -108,17 +108,15 @@ int gwb_ham_apply_strided(gwb_ham* h, const void* c, int64_t c_kstride, void* ou
                           int32_t nb, int32_t io_dtype, int32_t prec, void* stream);
 
 /* Tuning of a handle's applies (0 keeps the built-in rule): the bytes of FFT
- * scratch per band chunk (default 48 MiB or GWB_W_BUDGET_MB: chunks of bands
- * whose scratch stays in L2) and the number of CTAs the G-sliced projector
+ * scratch per band chunk (default 512 MiB or GWB_W_BUDGET_MB; 48 MiB where the
+ * device has no room for more) and the number of CTAs the G-sliced projector
  * contraction aims for (default 4 x 148). The values are chosen per box and
  * projector count by gradwave_b200.autotune from timed applies. No
  * counterpart in the reference. */
 int gwb_ham_set_tuning(gwb_ham* h, int64_t w_budget_bytes, int32_t nl_target_ctas);
-/* Threads per block of the shared-memory FFT kernels of the 72^3 and 96^3
- * boxes, per arithmetic precision: 256, 512 or 1024 (0: the built-in 512 for
- * float32, 1024 for float64). One block of a float64 96^3 plane fills the
- * shared memory of an SM, so more threads per block means more warps to hide
- * the latency of its barrier-separated passes. */
+/* Hint for the threads per block of the FFT kernels, per arithmetic precision:
+ * 256, 512 or 1024 (0: none). The kernels take their block sizes from the axis
+ * lengths; the values are checked and otherwise unused. */
 int gwb_ham_set_fft_threads(gwb_ham* h, int32_t threads_fp32, int32_t threads_fp64);
 
 /* Augmentation matrix q (nproj*nproj float64, real symmetric, device) of the
