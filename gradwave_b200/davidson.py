@@ -63,6 +63,10 @@ logger = logging.getLogger(__name__)
 
 _FP32_CERT_FLOOR_EPS = 32 * torch.finfo(torch.float32).eps
 _FP32_CERT_STALL = 0.7
+# norm of the noise on the unit rows of the first expansion of a cold start
+# (largest residual above _COLD_START_EV)
+_START_NOISE = 0.25
+_COLD_START_EV = 1.0
 _N, _T, _H = 0, 1, 2
 
 
@@ -573,6 +577,8 @@ class _Solver:
             with self.prof("precond"):
                 _lib.call("gwb_select_worst", nk, nb, _ptr(ws.rn), n_add, _ptr(ws.sel), self.stream)
                 self.precondition(n_add, eig)
+                if it == 1 and self.max_dim > self.heev_max and rnmax > _COLD_START_EV:
+                    self.break_symmetry(n_add)
             if m + n_add > md:
                 # restart: re-orthonormalise the Ritz block, images by the same
                 # transform (no re-application), keep the new directions
@@ -602,6 +608,21 @@ class _Solver:
             logger.debug("batched Davidson hit max_iter=%d (max res=%.3e > tol=%.1e)", self.max_iter,
                          float(ws.rn.max()), self.tol)
         return self.result(eig, self.max_iter)
+
+    def break_symmetry(self, n_add: int):
+        """Seeded noise on the first expansion rows of a cold start. A start
+        block of plane waves on a symmetric cell has no component in some
+        irreducible representations, and no step of the solver brings one in
+        but round-off: a solve may then converge to eigenpairs that skip a
+        level (64-atom cell, float64, identity start with 1e-15 of noise: 6 of
+        8 solves skip one at the block's upper edge; with the noise none of 45).
+        Rounds to 1e-10 eV by its norm (float64 / mixed / mixed with the
+        network): 3e-6 49-53 / 87-208 / 37-38, 3e-4 45-165 / 61-230 / 41-125,
+        0.03 78-100 / 79-137 / 38-44, 0.27 52-55 / 51-78 / 40."""
+        gen = torch.Generator(device=self.dev).manual_seed(20260 + n_add)
+        noise = torch.randn(self.nk, n_add, self.npw, 2, dtype=torch.float64, device=self.dev, generator=gen)
+        self.ws.D[:, :n_add].add_(torch.view_as_complex(noise) * self.mask[:, None, :], 
+                                      alpha=_START_NOISE / math.sqrt(2.0 * self.npw))
 
     def precondition(self, n_add: int, eig: torch.Tensor):
         """D[:, :n_add] = preconditioned, unit-normalised worst residuals."""
