@@ -25,6 +25,7 @@
 
 #include "common.cuh"
 #include "fft_axis.cuh"
+#include "zmma.cuh"
 
 namespace gwb {
 
@@ -547,16 +548,40 @@ static int local_term(gwb_ham* h, const SIO* c, int64_t ck, SIO* out, int64_t ok
   return GWB_OK;
 }
 
-// The nonlocal slices: enough G slices to fill the GPU for this band count.
-template <typename T>
-static int nl_geometry(gwb_ham* h, int nb, int* gslice, int* nsl) {
-  const int ns = nl_slices(h, nb);
-  *gslice = ((h->npw_max + ns - 1) / ns + NL_TG - 1) / NL_TG * NL_TG;
-  *nsl = (h->npw_max + *gslice - 1) / *gslice;
+// float64 arithmetic on complex128 rows: the float64 tensor instruction
+// (zmma.cuh); anything else the CUDA-core kernels above. Measured with 256
+// projectors, 2 k x 129 bands x 37,000 plane waves: becp 1908 -> 880 us, update
+// 1369 -> 720 us.
+template <typename T, typename SIO>
+constexpr bool nl_zmma = std::is_same<T, double>::value && std::is_same<SIO, cplx<double>>::value;
+
+// becp partial sums over G slices into d_part (slice, k, band, projector).
+template <typename T, typename SIO>
+static int becp_slices(gwb_ham* h, const SIO* c, int64_t ck, int nb, int* nsl, cudaStream_t st) {
   const size_t es = sizeof(cplx<T>);
-  int rc = ensure_buf(&h->d_part, &h->part_bytes, (size_t)*nsl * h->nk * nb * h->nproj * es);
+  const int npw = h->npw_max, np = h->nproj;
+  int gslice = 0;
+  if constexpr (nl_zmma<T, SIO>) {
+    *nsl = zmma_nh_slices(nb, np, npw, h->nk, npw, h->nl_target > 0 ? h->nl_target : 4 * 148, &gslice);
+  } else {
+    const int ns = nl_slices(h, nb);
+    gslice = ((npw + ns - 1) / ns + NL_TG - 1) / NL_TG * NL_TG;
+    *nsl = (npw + gslice - 1) / gslice;
+  }
+  int rc = ensure_buf(&h->d_part, &h->part_bytes, (size_t)*nsl * h->nk * nb * np * es);
   if (rc) return rc;
-  return ensure_buf(&h->d_bd, &h->bd_bytes, (size_t)h->nk * nb * h->nproj * es);
+  if ((rc = ensure_buf(&h->d_bd, &h->bd_bytes, (size_t)h->nk * nb * np * es))) return rc;
+  if constexpr (nl_zmma<T, SIO>) {
+    GWB_CUDA_TRY(zmma_nh(nb, np, npw, gslice, *nsl, c, npw, ck, h->d_p64, npw, (int64_t)np * npw,
+                         (cplx<double>*)h->d_part, h->nk, st));
+  } else {
+    const cplx<T>* P = sizeof(T) == 8 ? (const cplx<T>*)h->d_p64 : (const cplx<T>*)h->d_p32;
+    dim3 g4((np + NL_TP - 1) / NL_TP, (nb + NL_TB - 1) / NL_TB, h->nk * *nsl);
+    k_becp_partial<T, SIO><<<g4, 256, 0, st>>>(c, P, (cplx<T>*)h->d_part, h->nk, nb, np, npw, gslice, ck);
+    GWB_LAUNCH_CHECK();
+  }
+  count_launches(1);
+  return GWB_OK;
 }
 
 template <typename T, typename SIO>
@@ -569,23 +594,26 @@ static int apply_impl(gwb_ham* h, const SIO* c, int64_t ck, SIO* out, int64_t ok
     if (h->nproj > 0 && tc_nonlocal_enabled(h)) return nonlocal_tc(h, c, ck, out, ok, nb, st);
   }
   if (h->nproj > 0) {
-    int gslice = 0, nsl = 0;
-    if ((rc = nl_geometry<T>(h, nb, &gslice, &nsl))) return rc;
-    const cplx<T>* P = dbl ? (const cplx<T>*)h->d_p64 : (const cplx<T>*)h->d_p32;
+    int nsl = 0;
+    if ((rc = becp_slices<T, SIO>(h, c, ck, nb, &nsl, st))) return rc;
     const T* D = dbl ? (const T*)h->d_d64 : (const T*)h->d_d32;
-    dim3 g4((h->nproj + NL_TP - 1) / NL_TP, (nb + NL_TB - 1) / NL_TB, h->nk * nsl);
-    k_becp_partial<T, SIO><<<g4, 256, 0, st>>>(c, P, (cplx<T>*)h->d_part, h->nk, nb, h->nproj, h->npw_max, gslice, ck);
     const int ngrp = std::max(1, 128 / h->nproj);
     k_becp_reduce_d<T><<<h->nk * nb, 128, (size_t)h->nproj * (1 + ngrp) * es, st>>>(
         (const cplx<T>*)h->d_part, D, (cplx<T>*)h->d_bd, h->nk, nb, h->nproj, nsl);
-    dim3 g6((h->npw_max + 63) / 64, (nb + NL_TB - 1) / NL_TB, h->nk);
-    k_nl_add<T, SIO><<<g6, 256, 0, st>>>((const cplx<T>*)h->d_bd, P, out, h->nk, nb, h->nproj, h->npw_max, ok);
     GWB_LAUNCH_CHECK();
-    count_launches(3);
+    if constexpr (nl_zmma<T, SIO>) {
+      GWB_CUDA_TRY(zmma_nn(nb, h->npw_max, h->nproj, (const cplx<double>*)h->d_bd, nullptr, h->d_p64, nullptr, 0, out,
+                           ok, nullptr, 0, nullptr, h->nk, st));
+    } else {
+      const cplx<T>* P = dbl ? (const cplx<T>*)h->d_p64 : (const cplx<T>*)h->d_p32;
+      dim3 g6((h->npw_max + 63) / 64, (nb + NL_TB - 1) / NL_TB, h->nk);
+      k_nl_add<T, SIO><<<g6, 256, 0, st>>>((const cplx<T>*)h->d_bd, P, out, h->nk, nb, h->nproj, h->npw_max, ok);
+      GWB_LAUNCH_CHECK();
+    }
+    count_launches(2);
   }
   return GWB_OK;
 }
-
 
 // Generalized apply: out_h = H c and out_s = S c = (c + sum_pq |p> q_pq <q|c>)
 // masked, from one becp contraction (CUDA cores, every precision).
@@ -596,24 +624,30 @@ static int apply_hs_impl(gwb_ham* h, const SIO* c, int64_t ck, SIO* out_h, int64
   const bool dbl = sizeof(T) == 8;
   int rc = local_term<T, SIO>(h, c, ck, out_h, ohk, nb, st);
   if (rc) return rc;
-  const cplx<T>* P = dbl ? (const cplx<T>*)h->d_p64 : (const cplx<T>*)h->d_p32;
   if (h->nproj > 0) {
-    int gslice = 0, nsl = 0;
-    if ((rc = nl_geometry<T>(h, nb, &gslice, &nsl))) return rc;
+    int nsl = 0;
+    if ((rc = becp_slices<T, SIO>(h, c, ck, nb, &nsl, st))) return rc;
     if ((rc = ensure_buf(&h->d_bq, &h->bq_bytes, (size_t)h->nk * nb * h->nproj * es))) return rc;
     const T* D = dbl ? (const T*)h->d_d64 : (const T*)h->d_d32;
     const T* Q = dbl ? (const T*)h->d_q64 : (const T*)h->d_q32;
-    dim3 g4((h->nproj + NL_TP - 1) / NL_TP, (nb + NL_TB - 1) / NL_TB, h->nk * nsl);
-    k_becp_partial<T, SIO><<<g4, 256, 0, st>>>(c, P, (cplx<T>*)h->d_part, h->nk, nb, h->nproj, h->npw_max, gslice, ck);
     const int ngrp = std::max(1, 128 / h->nproj);
     k_becp_reduce_dq<T><<<h->nk * nb, 128, (size_t)h->nproj * (1 + ngrp) * es, st>>>(
         (const cplx<T>*)h->d_part, D, Q, (cplx<T>*)h->d_bd, (cplx<T>*)h->d_bq, h->nk, nb, h->nproj, nsl);
-    count_launches(2);
+    GWB_LAUNCH_CHECK();
+    count_launches(1);
   }
-  dim3 g6((h->npw_max + 63) / 64, (nb + NL_TB - 1) / NL_TB, h->nk);
-  k_nl_add_hs<T, SIO><<<g6, 256, 0, st>>>((const cplx<T>*)h->d_bd, (const cplx<T>*)h->d_bq, P, c, ck, out_h, ohk,
-                                          out_s, osk, h->d_npw, h->nk, nb, h->nproj, h->npw_max);
-  GWB_LAUNCH_CHECK();
+  if constexpr (nl_zmma<T, SIO>) {
+    // with no projectors nothing is read from bq, but it still asks for S c = masked c
+    const cplx<double>* bq = h->nproj > 0 ? (const cplx<double>*)h->d_bq : c;
+    GWB_CUDA_TRY(zmma_nn(nb, h->npw_max, h->nproj, (const cplx<double>*)h->d_bd, bq, h->d_p64, c, ck, out_h, ohk, out_s,
+                         osk, h->d_npw, h->nk, st));
+  } else {
+    const cplx<T>* P = dbl ? (const cplx<T>*)h->d_p64 : (const cplx<T>*)h->d_p32;
+    dim3 g6((h->npw_max + 63) / 64, (nb + NL_TB - 1) / NL_TB, h->nk);
+    k_nl_add_hs<T, SIO><<<g6, 256, 0, st>>>((const cplx<T>*)h->d_bd, (const cplx<T>*)h->d_bq, P, c, ck, out_h, ohk,
+                                            out_s, osk, h->d_npw, h->nk, nb, h->nproj, h->npw_max);
+    GWB_LAUNCH_CHECK();
+  }
   count_launches(1);
   return GWB_OK;
 }
