@@ -582,14 +582,20 @@ __global__ void k_precond_normalize(int npw, int n_add, int chunks, const double
 // true): half-sphere coefficient c_G = phi[2G-1] + i phi[2G] (c_0 = phi[0]),
 // which are the sqrt(w)-scaled half rows, so sums over them are full-sphere
 // sums; the output is written back in the same embedding.
-constexpr int PU_THREADS = 128;
+// Warpgroups per CTA, each with its own tile, A rows, accumulator and barriers,
+// all on one copy of the weights: eight tiles in flight per SM where CTAs of one
+// tile each fitted five (their weights took half of the shared memory). Bound by
+// the latency of a tile's three MMA rounds and by the tanh unit (192 per plane
+// wave, 0.66 ms of it here); 404 rows of 37,000 plane waves: 1410 -> 1261 us.
+constexpr int PU_WG = 4;
+constexpr int PU_THREADS = 128 * PU_WG;
 constexpr int PU_TILE = 128;
 constexpr int PU_K1 = 16, PU_K = 80;
 constexpr int PU_A = PU_TILE * PU_K * 2;   // 20480 B
 constexpr int PU_B1 = HID * PU_K1 * 2;      // 2048 B
 constexpr int PU_B = HID * PU_K * 2;        // 10240 B
-constexpr int PU_SMEM = PU_A + PU_B1 + 2 * PU_B + 16;  // 43 KB: five CTAs per SM
-constexpr int PU_TMEM_COLS = 64;
+constexpr int PU_SMEM = PU_WG * PU_A + PU_B1 + 2 * PU_B + 16;  // 102 KB: two CTAs per SM
+constexpr int PU_TMEM_COLS = 64 * PU_WG;
 // kind::f16 instruction descriptor: F32 accumulator, BF16 A and B, both
 // K-major, N = 64, M = 128
 constexpr uint32_t PU_IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(HID >> 3) << 17) |
@@ -665,34 +671,38 @@ __device__ __forceinline__ float pu_hidden(uint32_t taddr, uint8_t* sA, int row,
 }
 
 template <bool GAMMA>
-__global__ void __launch_bounds__(PU_THREADS, 5) k_precond_learned_umma(PuArgs a) {
+__global__ void __launch_bounds__(PU_THREADS, 2) k_precond_learned_umma(PuArgs a) {
   extern __shared__ uint8_t pu_raw[];
   __shared__ float sW4[HID];
   __shared__ float sB4;
-  __shared__ __align__(8) uint64_t bar;
+  __shared__ __align__(8) uint64_t bars[PU_WG];
   __shared__ uint32_t tmem_slot;
-  __shared__ double red[PU_THREADS / 32];
-  __shared__ int abort_f;
-  uint8_t* sA = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(pu_raw) + 15) & ~(uintptr_t)15);
-  uint8_t* sB1 = sA + PU_A;
+  __shared__ double reds[PU_WG][4];
+  __shared__ int abort_fs[PU_WG];
+  uint8_t* sB1 = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(pu_raw) + 15) & ~(uintptr_t)15);
   uint8_t* sB2 = sB1 + PU_B1;
   uint8_t* sB3 = sB2 + PU_B;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int wg = threadIdx.x >> 7, tid = threadIdx.x & 127, warp = tid >> 5, lane = tid & 31;
+  uint8_t* sA = sB3 + PU_B + wg * PU_A;
+  uint64_t& bar = bars[wg];
+  double* red = reds[wg];
+  int& abort_f = abort_fs[wg];
+  auto wg_sync = [&] { asm volatile("bar.sync %0, 128;" ::"r"(wg + 1) : "memory"); };
   const float* P = a.P;
-  for (int i = tid; i < HID * PU_K1; i += PU_THREADS) {
+  for (int i = threadIdx.x; i < HID * PU_K1; i += PU_THREADS) {
     const int n = i / PU_K1, k = i % PU_K1;
     const float v = k < NIN ? P[O_W1 + n * NIN + k] : (k == NIN ? P[O_B1 + n] : 0.f);
     *reinterpret_cast<__nv_bfloat16*>(sB1 + pu_off(n, k, PU_K1)) = __float2bfloat16_rn(v);
   }
-  for (int i = tid; i < HID * PU_K; i += PU_THREADS) {
+  for (int i = threadIdx.x; i < HID * PU_K; i += PU_THREADS) {
     const int n = i / PU_K, k = i % PU_K;
     const float v2 = k < HID ? P[O_W2 + n * HID + k] : (k == HID ? P[O_B2 + n] : 0.f);
     const float v3 = k < HID ? P[O_W3 + n * HID + k] : (k == HID ? P[O_B3 + n] : 0.f);
     *reinterpret_cast<__nv_bfloat16*>(sB2 + pu_off(n, k, PU_K)) = __float2bfloat16_rn(v2);
     *reinterpret_cast<__nv_bfloat16*>(sB3 + pu_off(n, k, PU_K)) = __float2bfloat16_rn(v3);
   }
-  for (int i = tid; i < HID; i += PU_THREADS) sW4[i] = bf(P[O_W4 + i]);
-  if (tid == 0) sB4 = bf(P[O_B4]);
+  for (int i = threadIdx.x; i < HID; i += PU_THREADS) sW4[i] = bf(P[O_W4 + i]);
+  if (threadIdx.x == 0) sB4 = bf(P[O_B4]);
   // the constant columns of this thread's A row for layers 2 and 3: k = 64 holds 1
   {
     const uint32_t one = 0x3F80u;  // BF16 1.0
@@ -704,7 +714,7 @@ __global__ void __launch_bounds__(PU_THREADS, 5) k_precond_learned_umma(PuArgs a
     abort_f = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 0) {
+  if (threadIdx.x < 32) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
                  "r"((uint32_t)PU_TMEM_COLS)
                  : "memory");
@@ -714,7 +724,7 @@ __global__ void __launch_bounds__(PU_THREADS, 5) k_precond_learned_umma(PuArgs a
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = tmem_slot;
+  const uint32_t tmem = tmem_slot + 64 * wg;  // this warpgroup's accumulator columns
   const uint32_t taddr = tmem + ((uint32_t)(32 * warp) << 16);  // this warp's 32 lanes
   const uint32_t bar_a = smem_u32(&bar);
   // layer 1 reads the first 16 columns of A (its features, a 1 at k = 4, zeros)
@@ -727,7 +737,7 @@ __global__ void __launch_bounds__(PU_THREADS, 5) k_precond_learned_umma(PuArgs a
   auto layer = [&](int which) {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
+    wg_sync();
     if (tid == 0) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (which == 1) {
@@ -748,7 +758,8 @@ __global__ void __launch_bounds__(PU_THREADS, 5) k_precond_learned_umma(PuArgs a
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   };
 
-  for (int w = blockIdx.x; w < a.total; w += gridDim.x) {
+  // the first items go to different CTAs, so that few items spread over the SMs
+  for (int w = wg * gridDim.x + blockIdx.x; w < a.total; w += PU_WG * gridDim.x) {
     const int row = w / a.tiles, tile = w - row * a.tiles;
     const int k = row / a.n_add, s = row - k * a.n_add;
     const int b = a.sel[(int64_t)k * a.n_add + s];
@@ -801,9 +812,9 @@ __global__ void __launch_bounds__(PU_THREADS, 5) k_precond_learned_umma(PuArgs a
       }
     }
     for (int o = 16; o > 0; o >>= 1) nn += __shfl_xor_sync(0xffffffffu, nn, o);
-    __syncthreads();  // red from the previous tile is read
+    wg_sync();  // red from the previous tile is read
     if (lane == 0) red[warp] = nn;
-    __syncthreads();
+    wg_sync();
     if (tid == 0) a.partial[(int64_t)row * a.tiles + tile] = red[0] + red[1] + red[2] + red[3];
     if (abort_f) break;
   }
@@ -812,7 +823,7 @@ __global__ void __launch_bounds__(PU_THREADS, 5) k_precond_learned_umma(PuArgs a
   if (abort_f && tid == 0) mbar_wait(bar_a, parity ^ 1u, a.wait_cycles);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == 0) {
+  if (threadIdx.x < 32) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)PU_TMEM_COLS)
                  : "memory");
@@ -899,7 +910,7 @@ __global__ void k_stall_update(const double* __restrict__ rn, double* __restrict
 }
 
 // The tcgen05 inference kernel over all (row, tile) items: a persistent grid
-// of up to five CTAs per SM (43 KB of shared memory and 64 TMEM columns each).
+// of up to two CTAs per SM (102 KB of shared memory and 256 TMEM columns each).
 template <bool GAMMA>
 int precond_umma(const float* params, int nb, int n_add, int npw, const void* r, int64_t rk, int64_t r_row,
                  const double* t, const double* eig, const int* sel, const uint8_t* tpa_only, const double* stats,
@@ -931,7 +942,7 @@ int precond_umma(const float* params, int nb, int n_add, int npw, const void* r,
   GWB_CUDA_TRY(cudaFuncSetAttribute(k_precond_learned_umma<GAMMA>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     PU_SMEM));
   GWB_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int), st));
-  const int grid = std::min(a.total, 5 * sms);
+  const int grid = std::min(a.total, 2 * sms);
   k_precond_learned_umma<GAMMA><<<grid, PU_THREADS, PU_SMEM, st>>>(a);
   GWB_LAUNCH_CHECK();
   return GWB_OK;
