@@ -87,6 +87,8 @@ __global__ void k_zgemm_nh_reduce(int M, int N, int nslice, int batch, const cpl
                                   cplx<double> alpha, cplx<double> beta, cplx<double>* __restrict__ C, int64_t ldc,
                                   int64_t sC) {
   const int64_t total = (int64_t)batch * M * N;
+  chain_wait();
+  part = after_wait(part);
   for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
        idx += (int64_t)gridDim.x * blockDim.x) {
     const int b = (int)(idx / ((int64_t)M * N));
@@ -119,11 +121,9 @@ extern "C" int gwb_zgemm_nh(int64_t M, int64_t N, int64_t K, double alpha_re, do
                        ldb, strideB, (cplx<double>*)work, (int)batch, st));
   const int64_t total = M * N * batch;
   const int blocks = (int)std::min<int64_t>((total + 255) / 256, 4096);
-  k_zgemm_nh_reduce<<<blocks, 256, 0, st>>>((int)M, (int)N, ns, (int)batch,
-                                            (const cplx<double>*)work, mk<double>(alpha_re, alpha_im),
-                                                              mk<double>(beta_re, beta_im), (cplx<double>*)C, ldc,
-                                                              strideC);
-  GWB_LAUNCH_CHECK();
+  GWB_CUDA_TRY(launch_chained(k_zgemm_nh_reduce, dim3(blocks), 256, 0, st, (int)M, (int)N, ns, (int)batch,
+                              (const cplx<double>*)work, mk<double>(alpha_re, alpha_im), mk<double>(beta_re, beta_im),
+                              (cplx<double>*)C, ldc, strideC));
   count_launches(2);
   return GWB_OK;
 }

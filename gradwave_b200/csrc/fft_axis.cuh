@@ -154,6 +154,7 @@ __global__ void __launch_bounds__(AxisCfg<T, N>::NTR, AxisCfg<T, N>::minb(AxisCf
         const int i2 = a + R2 * b;
         idx[b] = (i2 <= f.M2 || i2 >= N - f.M2) ? mp[i2] : -1;
       });
+      chain_wait();
       cplx<T> x[R1];
       StaticFor<0, R1>::run([&](auto bc) {
         constexpr int b = decltype(bc)::value;
@@ -196,6 +197,7 @@ __global__ void __launch_bounds__(AxisCfg<T, N>::NTR, AxisCfg<T, N>::minb(AxisCf
   const size_t crow = (size_t)k * f.ck + (size_t)(f.b0 + bl) * f.npw_max;
   const size_t orow = (size_t)k * f.ok + (size_t)(f.b0 + bl) * f.npw_max;
   const T* tk = f.t + (size_t)k * f.npw_max;
+  chain_wait();
   auto store = [&](int g, cplx<T> val) {
     const cplx<T> cv = load_io<T>(f.c, f.io64, crow + g);
     const cplx<T> o = val + scale(cv, tk[g]);
@@ -267,6 +269,7 @@ __global__ void __launch_bounds__(AxisCfg<T, N>::NT, AxisCfg<T, N>::minb(AxisCfg
     const cplx<T>* src = f.W2 + kb * f.nrow * n2 + i2;
     int idx[R1];
     StaticFor<0, R1>::run([&](auto bc) { idx[decltype(bc)::value] = ro[R2 * decltype(bc)::value]; });
+    chain_wait();
     cplx<T> x[R1];
     StaticFor<0, R1>::run([&](auto bc) {
       constexpr int b = decltype(bc)::value;
@@ -310,6 +313,7 @@ __global__ void __launch_bounds__(AxisCfg<T, N>::NT, AxisCfg<T, N>::minb(AxisCfg
   const size_t kb = (size_t)k * f.nbc + bl;
   cplx<T>* dst = f.W2 + kb * f.nrow * n2 + i2;
   const int* ro = f.rowof + ((size_t)k * f.L0 + j0) * N;
+  chain_wait();
   if (live) {
     const cplx<T>* src = f.W + (kb * f.L0 + j0) * (size_t)(N * n2) + (size_t)s * n2 + i2;
     cplx<T> x[R1];
@@ -363,6 +367,7 @@ __global__ void __launch_bounds__(AxisCfg<T, N>::NT, AxisCfg<T, N>::minb(AxisCfg
   const bool live = p < plane;
   const int M0 = f.M0, L0 = f.L0;
   const int bl0 = blockIdx.y * bands_per_block, bl1 = min(f.nbc, bl0 + bands_per_block);
+  chain_wait();
   for (int bl = bl0; bl < bl1; ++bl) {
     // opaque per band: hoisted out of the loop, the twiddles and the 2 R1 + R2
     // addresses take more registers than there are
@@ -449,6 +454,7 @@ __global__ void __launch_bounds__(AxisCfg<T, N>::NT, AxisCfg<T, N>::minb(AxisCfg
   const bool own = live && s < SV;
   double* rk = f.rho + ((size_t)k * f.ngrp + grp) * N * plane + p + (R2 == 1 ? 0 : s * plane);
   double acc[RV];
+  chain_wait();
   StaticFor<0, RV>::run([&](auto kc) {
     acc[decltype(kc)::value] = own && !f.first ? rk[SV * decltype(kc)::value * plane] : 0.0;
   });
@@ -504,18 +510,16 @@ cudaError_t fft_pencil_density(const FftRun<double>& f, cudaStream_t st);
 
 namespace fft_detail {
 
-template <typename T, int N, class K> cudaError_t launch_rows(K* kern, const FftRun<T>& f, cudaStream_t st) {
+template <typename T, int N> cudaError_t launch_rows(void (*kern)(FftRun<T>), const FftRun<T>& f, cudaStream_t st) {
   using C = AxisCfg<T, N>;
   dim3 g((f.nrow + C::RB - 1) / C::RB, f.nbc, f.nk);
-  kern<<<g, C::NTR, C::smem_rows, st>>>(f);
-  return cudaGetLastError();
+  return launch_chained(kern, g, C::NTR, C::smem_rows, st, f);
 }
 
-template <typename T, int N, class K> cudaError_t launch_cols(K* kern, const FftRun<T>& f, cudaStream_t st) {
+template <typename T, int N> cudaError_t launch_cols(void (*kern)(FftRun<T>), const FftRun<T>& f, cudaStream_t st) {
   using C = AxisCfg<T, N>;
   dim3 g((f.L0 * f.n2 + C::PB - 1) / C::PB, f.nbc, f.nk);
-  kern<<<g, C::NT, C::smem_strided, st>>>(f);
-  return cudaGetLastError();
+  return launch_chained(kern, g, C::NT, C::smem_strided, st, f);
 }
 
 template <typename T, int N> cudaError_t launch_vloc(const FftRun<T>& f, cudaStream_t st) {
@@ -531,8 +535,7 @@ template <typename T, int N> cudaError_t launch_vloc(const FftRun<T>& f, cudaStr
     const cudaError_t e = allow_smem(k_pencil_vloc<T, N>);
     if (e != cudaSuccess) return e;
   }
-  k_pencil_vloc<T, N><<<g, C::NT, 2 * C::smem_strided, st>>>(f, bpb);
-  return cudaGetLastError();
+  return launch_chained(k_pencil_vloc<T, N>, g, C::NT, 2 * C::smem_strided, st, f, bpb);
 }
 
 template <typename T, int N> cudaError_t launch_density(const FftRun<T>& f, cudaStream_t st) {
@@ -542,8 +545,7 @@ template <typename T, int N> cudaError_t launch_density(const FftRun<T>& f, cuda
     const cudaError_t e = allow_smem(k_pencil_density<T, N>);
     if (e != cudaSuccess) return e;
   }
-  k_pencil_density<T, N><<<g, C::NT, 2 * C::smem_strided, st>>>(f);
-  return cudaGetLastError();
+  return launch_chained(k_pencil_density<T, N>, g, C::NT, 2 * C::smem_strided, st, f);
 }
 
 }  // namespace fft_detail

@@ -36,6 +36,8 @@ __global__ void k_gamma_pack(int nb, int nphi, int npw, const double* __restrict
                              cplx<double>* __restrict__ z) {
   const int npair = (nb + 1) / 2;
   const int64_t total = (int64_t)npair * npw;
+  chain_wait();
+  phi = after_wait(phi);
   for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
        idx += (int64_t)gridDim.x * blockDim.x) {
     const int p = (int)(idx / npw), g = (int)(idx % npw);
@@ -58,6 +60,8 @@ __global__ void k_gamma_unpack(int nb, int nhalf, int npw, const cplx<double>* _
                                double* __restrict__ out, int64_t ldout) {
   const int npair = (nb + 1) / 2;
   const int64_t total = (int64_t)npair * nhalf;
+  chain_wait();
+  hz = after_wait(hz);
   for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
        idx += (int64_t)gridDim.x * blockDim.x) {
     const int p = (int)(idx / nhalf), j = (int)(idx % nhalf);
@@ -110,17 +114,14 @@ extern "C" int gwb_gamma_apply(gwb_ham* h, int32_t nb, int32_t nhalf, int32_t np
   cplx<double>* hz = z + (size_t)npair * npw;
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t t1 = (int64_t)npair * npw, t2 = (int64_t)npair * nhalf;
-  k_gamma_pack<<<(unsigned)std::min<int64_t>((t1 + 255) / 256, 148 * 16), 256, 0, st>>>(nb, nphi, npw, phi, ldphi,
-                                                                                      src_half, conj_full, z);
-  GWB_LAUNCH_CHECK();
+  GWB_CUDA_TRY(launch_chained(k_gamma_pack, dim3((unsigned)std::min<int64_t>((t1 + 255) / 256, 148 * 16)), 256, 0, st, nb,
+                              nphi, npw, phi, ldphi, src_half, conj_full, z));
   count_launches(1);
   const int rc = gwb_ham_apply_strided(h, z, (int64_t)npair * npw, hz, (int64_t)npair * npw, npair, GWB_C128, prec,
                                        stream);
   if (rc != GWB_OK) return rc;
-  k_gamma_unpack<<<(unsigned)std::min<int64_t>((t2 + 255) / 256, 148 * 16), 256, 0, st>>>(nb, nhalf, npw, hz,
-                                                                                        rep_full, partner_rep, out,
-                                                                                        ldout);
-  GWB_LAUNCH_CHECK();
+  GWB_CUDA_TRY(launch_chained(k_gamma_unpack, dim3((unsigned)std::min<int64_t>((t2 + 255) / 256, 148 * 16)), 256, 0, st, nb,
+                              nhalf, npw, (const cplx<double>*)hz, rep_full, partner_rep, out, ldout));
   count_launches(1);
   return GWB_OK;
 }

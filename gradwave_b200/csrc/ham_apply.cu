@@ -19,6 +19,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <atomic>
+#include <map>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -62,6 +63,7 @@ struct gwb_ham {
   gwb::cplx<float>* d_p32 = nullptr;
   double* d_d64 = nullptr;
   float* d_d32 = nullptr;
+  gwb::ColumnLists d_cols, q_cols;  // nonzeros of D and q per column
   double* d_q64 = nullptr;  // augmentation q_pq of the overlap S (USPP/PAW), when set
   float* d_q32 = nullptr;
   gwb::cplx<double>* d_tw64[3] = {nullptr, nullptr, nullptr};
@@ -69,6 +71,7 @@ struct gwb_ham {
   // scratch
   void* d_W = nullptr;  // planes of a band chunk, then its rows
   size_t W_bytes = 0;
+  bool counted = false;  // among its device's live handles (gwb_ham_create completed)
   void* d_part = nullptr;  // becp partials
   size_t part_bytes = 0;
   void* d_bd = nullptr;  // becp * D
@@ -180,6 +183,8 @@ __global__ void __launch_bounds__(256) k_becp_partial(const SIO* __restrict__ c,
       rp[q] = (p < nproj && gi < g_end) ? P[((size_t)k * nproj + p) * npw_max + gi] : mk<T>(0, 0);
     }
   };
+  chain_wait();
+  c = after_wait(c);
   if (g_begin < g_end) fetch(g_begin);
   for (int gb = g_begin; gb < g_end; gb += NL_TG) {
 #pragma unroll
@@ -211,23 +216,19 @@ __global__ void __launch_bounds__(256) k_becp_partial(const SIO* __restrict__ c,
   }
 }
 
-// K5: bd[k][b][q] = sum_p (sum_s part[s][k][b][p]) D[p][q]. The slice sums
-// are split over the threads (projector p, slice group) and combined in a
-// fixed order (deterministic).
+// Sum of the slice partials of one (k, band) into becp (shared memory): the
+// slices are split over the threads (projector p, slice group) and combined in
+// a fixed order (deterministic).
 template <typename T>
-__global__ void __launch_bounds__(128) k_becp_reduce_d(const cplx<T>* __restrict__ part, const T* __restrict__ D,
-                                                       cplx<T>* __restrict__ bd, int nk, int nb, int nproj,
-                                                       int nslice) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  cplx<T>* becp = reinterpret_cast<cplx<T>*>(smem_raw);  // nproj
-  cplx<T>* grp = becp + nproj;                            // nproj * ngrp partial sums
-  const int kb = blockIdx.x;                               // k*nb + b
-  const size_t stride = (size_t)nk * nb * nproj;
+__device__ __forceinline__ void sum_slices(const cplx<T>* part, cplx<T>* becp, cplx<T>* grp, size_t stride,
+                                           size_t row, int nproj, int nslice) {
   const int ngrp = max(1, (int)blockDim.x / nproj);
+  chain_wait();
+  part = after_wait(part);
   for (int idx = threadIdx.x; idx < nproj * ngrp; idx += blockDim.x) {
     const int p = idx % nproj, gq = idx / nproj;
     cplx<T> a = mk<T>(0, 0);
-    for (int s = gq; s < nslice; s += ngrp) a = a + part[s * stride + (size_t)kb * nproj + p];
+    for (int s = gq; s < nslice; s += ngrp) a = a + part[s * stride + row + p];
     grp[gq * nproj + p] = a;
   }
   __syncthreads();
@@ -237,11 +238,18 @@ __global__ void __launch_bounds__(128) k_becp_reduce_d(const cplx<T>* __restrict
     becp[p] = a;
   }
   __syncthreads();
-  for (int q = threadIdx.x; q < nproj; q += blockDim.x) {
-    cplx<T> a = mk<T>(0, 0);
-    for (int p = 0; p < nproj; ++p) a = a + scale(becp[p], D[(size_t)p * nproj + q]);
-    bd[(size_t)kb * nproj + q] = a;
-  }
+}
+
+// K5: bd[k][b][q] = sum_p (sum_s part[s][k][b][p]) D[p][q].
+template <typename T>
+__global__ void __launch_bounds__(128) k_becp_reduce_d(const cplx<T>* __restrict__ part, const T* __restrict__ D,
+                                                       ColumnLists cols, cplx<T>* __restrict__ bd, int nk, int nb,
+                                                       int nproj, int nslice) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  cplx<T>* becp = reinterpret_cast<cplx<T>*>(smem_raw);  // nproj
+  const size_t row = (size_t)blockIdx.x * nproj;         // blockIdx.x = k*nb + b
+  sum_slices(part, becp, becp + nproj, (size_t)nk * nb * nproj, row, nproj, nslice);
+  for (int q = threadIdx.x; q < nproj; q += blockDim.x) bd[row + q] = column_sum(cols, D, nproj, q, becp);
 }
 
 // K6: out[k][b][g] += sum_q bd[k][b][q] P[k][q][g]; tiles TB bands x 64 G.
@@ -258,6 +266,8 @@ __global__ void __launch_bounds__(256) k_nl_add(const cplx<T>* __restrict__ bd,
   const int lg = tid % TGO, lb0 = tid / TGO;  // 4 band groups x 64 g; each thread 4 bands
   cplx<T> acc[4];
   const int gi_o = gt * TGO + lg;
+  chain_wait();
+  bd = after_wait(bd);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {  // the output rows first: their loads overlap the tile staging below
     const int b = bt * NL_TB + lb0 * 4 + i;
@@ -293,39 +303,19 @@ __global__ void __launch_bounds__(256) k_nl_add(const cplx<T>* __restrict__ bd,
 }
 
 // K5 of the generalized apply: one pass over the slice partials gives both
-// bd = becp D (H) and bq = becp q (S). Same fixed-order reduction as K5.
+// bd = becp D (H) and bq = becp q (S).
 template <typename T>
 __global__ void __launch_bounds__(128) k_becp_reduce_dq(const cplx<T>* __restrict__ part, const T* __restrict__ D,
-                                                        const T* __restrict__ Q, cplx<T>* __restrict__ bd,
-                                                        cplx<T>* __restrict__ bq, int nk, int nb, int nproj,
-                                                        int nslice) {
+                                                        ColumnLists dcols, const T* __restrict__ Q, ColumnLists qcols,
+                                                        cplx<T>* __restrict__ bd, cplx<T>* __restrict__ bq, int nk,
+                                                        int nb, int nproj, int nslice) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cplx<T>* becp = reinterpret_cast<cplx<T>*>(smem_raw);
-  cplx<T>* grp = becp + nproj;
-  const int kb = blockIdx.x;
-  const size_t stride = (size_t)nk * nb * nproj;
-  const int ngrp = max(1, (int)blockDim.x / nproj);
-  for (int idx = threadIdx.x; idx < nproj * ngrp; idx += blockDim.x) {
-    const int p = idx % nproj, gq = idx / nproj;
-    cplx<T> a = mk<T>(0, 0);
-    for (int s = gq; s < nslice; s += ngrp) a = a + part[s * stride + (size_t)kb * nproj + p];
-    grp[gq * nproj + p] = a;
-  }
-  __syncthreads();
-  for (int p = threadIdx.x; p < nproj; p += blockDim.x) {
-    cplx<T> a = mk<T>(0, 0);
-    for (int gq = 0; gq < ngrp; ++gq) a = a + grp[gq * nproj + p];
-    becp[p] = a;
-  }
-  __syncthreads();
+  const size_t row = (size_t)blockIdx.x * nproj;
+  sum_slices(part, becp, becp + nproj, (size_t)nk * nb * nproj, row, nproj, nslice);
   for (int q = threadIdx.x; q < nproj; q += blockDim.x) {
-    cplx<T> a = mk<T>(0, 0), b = mk<T>(0, 0);
-    for (int p = 0; p < nproj; ++p) {
-      a = a + scale(becp[p], D[(size_t)p * nproj + q]);
-      b = b + scale(becp[p], Q[(size_t)p * nproj + q]);
-    }
-    bd[(size_t)kb * nproj + q] = a;
-    bq[(size_t)kb * nproj + q] = b;
+    bd[row + q] = column_sum(dcols, D, nproj, q, becp);
+    bq[row + q] = column_sum(qcols, Q, nproj, q, becp);
   }
 }
 
@@ -349,6 +339,9 @@ __global__ void __launch_bounds__(256) k_nl_add_hs(const cplx<T>* __restrict__ b
   const int gi_o = gt * TGO + lg;
   const bool on_sphere = gi_o < npw_k[k];
   cplx<T> ah[4], as[4];
+  chain_wait();
+  bd = after_wait(bd);
+  bq = after_wait(bq);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int b = bt * NL_TB + lb0 * 4 + i;
@@ -397,9 +390,78 @@ template <typename T> __global__ void k_scale_copy(const double* src, T* dst, si
   size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (i < n) dst[i] = (T)(src[i] * s);
 }
+// Nonzeros of each column of the n x n matrix D, rows ascending.
+__global__ void k_column_lists(const double* __restrict__ D, int n, int* __restrict__ cnt, int* __restrict__ idx) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= n) return;
+  int c = 0;
+#pragma unroll 8
+  for (int p = 0; p < n; ++p)
+    if (D[(size_t)p * n + q] != 0.0) idx[(size_t)c++ * n + q] = p;
+  cnt[q] = c;
+}
+
+static cudaError_t alloc_columns(ColumnLists* c, int n) {
+  const cudaError_t e = cudaMalloc((void**)&c->cnt, (size_t)n * sizeof(int));
+  return e != cudaSuccess ? e : cudaMalloc((void**)&c->idx, (size_t)n * n * sizeof(int));
+}
+
 __global__ void k_c128_to_c64(const cplx<double>* src, cplx<float>* dst, size_t n) {
   size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (i < n) dst[i] = mk<float>((float)src[i].x, (float)src[i].y);
+}
+
+// The band-chunk scratch of a destroyed handle waits here for the next handle
+// on the device (mapping half a GB takes milliseconds, as long as many an
+// apply): at most one buffer per device, kept only while a handle lives there
+// and given back when an allocation fails.
+struct ScratchSlot {
+  int handles = 0;
+  void* p = nullptr;
+  size_t bytes = 0;
+};
+static std::mutex g_scratch_mu;
+static std::map<int, ScratchSlot> g_scratch;
+
+static void scratch_handle(int dev, int n) {
+  void* drop = nullptr;
+  {
+    std::lock_guard<std::mutex> lk(g_scratch_mu);
+    ScratchSlot& s = g_scratch[dev];
+    s.handles += n;
+    if (s.handles == 0) {
+      drop = s.p;
+      s.p = nullptr;
+      s.bytes = 0;
+    }
+  }
+  if (drop) cudaFree(drop);
+}
+
+// A kept buffer of at least need bytes (need = 0: any), or null.
+static void* scratch_take(int dev, size_t need, size_t* bytes) {
+  std::lock_guard<std::mutex> lk(g_scratch_mu);
+  ScratchSlot& s = g_scratch[dev];
+  if (!s.p || s.bytes < need) return nullptr;
+  void* p = s.p;
+  *bytes = s.bytes;
+  s.p = nullptr;
+  s.bytes = 0;
+  return p;
+}
+
+// p is idle (its device has been synchronised). The larger of it and the kept
+// buffer stays.
+static void scratch_give(int dev, void* p, size_t bytes) {
+  {
+    std::lock_guard<std::mutex> lk(g_scratch_mu);
+    ScratchSlot& s = g_scratch[dev];
+    if (s.handles > 0 && bytes > s.bytes) {
+      std::swap(p, s.p);
+      s.bytes = bytes;
+    }
+  }
+  if (p) cudaFree(p);
 }
 
 static int ensure_buf(void** p, size_t* have, size_t need) {
@@ -432,17 +494,34 @@ static int nl_slices(const gwb_ham* h, int nb) {
 static int chunk_scratch(gwb_ham* h, int nb, size_t es, int* nbc) {
   const FftGeom& g = h->g;
   const size_t per_band = (size_t)h->nk * ((size_t)g.L[0] * g.n[1] + g.nrow) * g.n[2] * es;
+  auto ensure = [&](size_t need) {
+    if (h->W_bytes >= need) return GWB_OK;
+    if (void* p = scratch_take(h->device, need, &need)) {
+      if (h->d_W) cudaFree(h->d_W);
+      h->d_W = p;
+      h->W_bytes = need;
+      return GWB_OK;
+    }
+    int rc = ensure_buf(&h->d_W, &h->W_bytes, need);
+    size_t n = 0;
+    void* kept = rc == GWB_ERR_ALLOC ? scratch_take(h->device, 0, &n) : nullptr;
+    if (kept) {
+      cudaFree(kept);
+      rc = ensure_buf(&h->d_W, &h->W_bytes, need);
+    }
+    return rc;
+  };
   auto bands = [&](size_t budget) {
     const size_t most = std::max<size_t>(1, budget / per_band);
     const size_t nchunks = ((size_t)nb + most - 1) / most;
     return (int)(((size_t)nb + nchunks - 1) / nchunks);
   };
   *nbc = bands(h->w_budget ? h->w_budget : w_budget_bytes());
-  int rc = ensure_buf(&h->d_W, &h->W_bytes, per_band * *nbc);
+  int rc = ensure(per_band * *nbc);
   const int low = bands((size_t)kWBudgetLowMB << 20);
   if (rc == GWB_ERR_ALLOC && low < *nbc) {
     *nbc = low;
-    rc = ensure_buf(&h->d_W, &h->W_bytes, per_band * *nbc);
+    rc = ensure(per_band * *nbc);
   }
   return rc;
 }
@@ -469,8 +548,8 @@ template <typename T> static void place_rows(const gwb_ham* h, FftRun<T>* f) {
   f->W2 = f->W + (size_t)h->nk * f->nbc * f->L0 * f->n1 * f->n2;
 }
 
-int tc_becp_d_planes(int nk, int nb, int nproj, const cplx<double>* becp, const double* D, void* planes, int64_t ldq,
-                     cudaStream_t st);
+int tc_becp_d_planes(int nk, int nb, int nproj, const cplx<double>* becp, const double* D, const ColumnLists& cols,
+                     void* planes, int64_t ldq, cudaStream_t st);
 
 // Projector counts from which the float32 apply of complex128 blocks runs its
 // nonlocal term on the tensor cores (GWB_TC_NONLOCAL=0 keeps the CUDA-core
@@ -514,7 +593,7 @@ static int nonlocal_tc(gwb_ham* h, const cplx<double>* c, int64_t ck, cplx<doubl
   if ((rc = gwb_zgemm_tc(2, nb, np, npw, 1.0, 0.0, h->d_cplanes, ldp, nb, h->d_pplanes, ldp, np, 0.0, 0.0, h->d_becp,
                          np, (int64_t)nb * np, nk, h->d_tcwork, h->tcwork_bytes, h->d_tcstatus, st)))
     return rc;
-  if ((rc = tc_becp_d_planes(nk, nb, np, (const cplx<double>*)h->d_becp, h->d_d64, h->d_bdplanes, ldq, st))) return rc;
+  if ((rc = tc_becp_d_planes(nk, nb, np, (const cplx<double>*)h->d_becp, h->d_d64, h->d_cols, h->d_bdplanes, ldq, st))) return rc;
   return gwb_zgemm_tc(0, nb, npw, np, 1.0, 0.0, h->d_bdplanes, ldq, nb, h->d_pplanes, ldp, np, 1.0, 0.0, out, npw, ok,
                       nk, nullptr, 0, h->d_tcstatus, st);
 }
@@ -577,8 +656,8 @@ static int becp_slices(gwb_ham* h, const SIO* c, int64_t ck, int nb, int* nsl, c
   } else {
     const cplx<T>* P = sizeof(T) == 8 ? (const cplx<T>*)h->d_p64 : (const cplx<T>*)h->d_p32;
     dim3 g4((np + NL_TP - 1) / NL_TP, (nb + NL_TB - 1) / NL_TB, h->nk * *nsl);
-    k_becp_partial<T, SIO><<<g4, 256, 0, st>>>(c, P, (cplx<T>*)h->d_part, h->nk, nb, np, npw, gslice, ck);
-    GWB_LAUNCH_CHECK();
+    GWB_CUDA_TRY(launch_chained(k_becp_partial<T, SIO>, g4, 256, 0, st, c, P, (cplx<T>*)h->d_part, h->nk, nb, np, npw,
+                                gslice, ck));
   }
   count_launches(1);
   return GWB_OK;
@@ -598,17 +677,16 @@ static int apply_impl(gwb_ham* h, const SIO* c, int64_t ck, SIO* out, int64_t ok
     if ((rc = becp_slices<T, SIO>(h, c, ck, nb, &nsl, st))) return rc;
     const T* D = dbl ? (const T*)h->d_d64 : (const T*)h->d_d32;
     const int ngrp = std::max(1, 128 / h->nproj);
-    k_becp_reduce_d<T><<<h->nk * nb, 128, (size_t)h->nproj * (1 + ngrp) * es, st>>>(
-        (const cplx<T>*)h->d_part, D, (cplx<T>*)h->d_bd, h->nk, nb, h->nproj, nsl);
-    GWB_LAUNCH_CHECK();
+    GWB_CUDA_TRY(launch_chained(k_becp_reduce_d<T>, dim3(h->nk * nb), 128, (size_t)h->nproj * (1 + ngrp) * es, st,
+                                (const cplx<T>*)h->d_part, D, h->d_cols, (cplx<T>*)h->d_bd, h->nk, nb, h->nproj, nsl));
     if constexpr (nl_zmma<T, SIO>) {
       GWB_CUDA_TRY(zmma_nn(nb, h->npw_max, h->nproj, (const cplx<double>*)h->d_bd, nullptr, h->d_p64, nullptr, 0, out,
                            ok, nullptr, 0, nullptr, h->nk, st));
     } else {
       const cplx<T>* P = dbl ? (const cplx<T>*)h->d_p64 : (const cplx<T>*)h->d_p32;
       dim3 g6((h->npw_max + 63) / 64, (nb + NL_TB - 1) / NL_TB, h->nk);
-      k_nl_add<T, SIO><<<g6, 256, 0, st>>>((const cplx<T>*)h->d_bd, P, out, h->nk, nb, h->nproj, h->npw_max, ok);
-      GWB_LAUNCH_CHECK();
+      GWB_CUDA_TRY(launch_chained(k_nl_add<T, SIO>, g6, 256, 0, st, (const cplx<T>*)h->d_bd, P, out, h->nk, nb, h->nproj,
+                                  h->npw_max, ok));
     }
     count_launches(2);
   }
@@ -631,9 +709,9 @@ static int apply_hs_impl(gwb_ham* h, const SIO* c, int64_t ck, SIO* out_h, int64
     const T* D = dbl ? (const T*)h->d_d64 : (const T*)h->d_d32;
     const T* Q = dbl ? (const T*)h->d_q64 : (const T*)h->d_q32;
     const int ngrp = std::max(1, 128 / h->nproj);
-    k_becp_reduce_dq<T><<<h->nk * nb, 128, (size_t)h->nproj * (1 + ngrp) * es, st>>>(
-        (const cplx<T>*)h->d_part, D, Q, (cplx<T>*)h->d_bd, (cplx<T>*)h->d_bq, h->nk, nb, h->nproj, nsl);
-    GWB_LAUNCH_CHECK();
+    GWB_CUDA_TRY(launch_chained(k_becp_reduce_dq<T>, dim3(h->nk * nb), 128, (size_t)h->nproj * (1 + ngrp) * es, st,
+                                (const cplx<T>*)h->d_part, D, h->d_cols, Q, h->q_cols, (cplx<T>*)h->d_bd,
+                                (cplx<T>*)h->d_bq, h->nk, nb, h->nproj, nsl));
     count_launches(1);
   }
   if constexpr (nl_zmma<T, SIO>) {
@@ -644,9 +722,8 @@ static int apply_hs_impl(gwb_ham* h, const SIO* c, int64_t ck, SIO* out_h, int64
   } else {
     const cplx<T>* P = dbl ? (const cplx<T>*)h->d_p64 : (const cplx<T>*)h->d_p32;
     dim3 g6((h->npw_max + 63) / 64, (nb + NL_TB - 1) / NL_TB, h->nk);
-    k_nl_add_hs<T, SIO><<<g6, 256, 0, st>>>((const cplx<T>*)h->d_bd, (const cplx<T>*)h->d_bq, P, c, ck, out_h, ohk,
-                                            out_s, osk, h->d_npw, h->nk, nb, h->nproj, h->npw_max);
-    GWB_LAUNCH_CHECK();
+    GWB_CUDA_TRY(launch_chained(k_nl_add_hs<T, SIO>, g6, 256, 0, st, (const cplx<T>*)h->d_bd, (const cplx<T>*)h->d_bq, P,
+                                c, ck, out_h, ohk, out_s, osk, h->d_npw, h->nk, nb, h->nproj, h->npw_max));
   }
   count_launches(1);
   return GWB_OK;
@@ -820,15 +897,31 @@ int gwb_ham_create(const gwb_ham_geometry* geom, int device, gwb_ham** out) {
     if ((e = cudaMalloc((void**)&h->d_p32, np * 8)) != cudaSuccess) return fail(e);
     if ((e = cudaMalloc((void**)&h->d_d64, (size_t)h->nproj * h->nproj * 8)) != cudaSuccess) return fail(e);
     if ((e = cudaMalloc((void**)&h->d_d32, (size_t)h->nproj * h->nproj * 4)) != cudaSuccess) return fail(e);
+    if ((e = alloc_columns(&h->d_cols, h->nproj)) != cudaSuccess) return fail(e);
   }
+  scratch_handle(device, 1);
+  h->counted = true;
   *out = h;
   return GWB_OK;
 }
 
 int gwb_ham_destroy(gwb_ham* h) {
   if (!h) return GWB_OK;
+  if (h->d_W) {
+    // the scratch may serve the next handle once nothing in flight uses it
+    int cur = 0;
+    const bool idle = cudaGetDevice(&cur) == cudaSuccess && cudaSetDevice(h->device) == cudaSuccess &&
+                      cudaDeviceSynchronize() == cudaSuccess;
+    if (idle) {
+      scratch_give(h->device, h->d_W, h->W_bytes);
+      h->d_W = nullptr;
+    }
+    cudaSetDevice(cur);
+  }
+  if (h->counted) scratch_handle(h->device, -1);
   void* ptrs[] = {h->d_npw, h->d_map, h->d_rowof, h->d_dup, h->d_t64, h->d_t32, h->d_v64,
-                  h->d_v32, h->d_p64, h->d_p32, h->d_d64, h->d_d32, h->d_q64, h->d_q32, h->d_W, h->d_part, h->d_bd, h->d_bq,
+                  h->d_v32, h->d_p64, h->d_p32, h->d_d64, h->d_d32, h->d_q64, h->d_q32, h->d_cols.cnt, h->d_cols.idx,
+                  h->q_cols.cnt, h->q_cols.idx, h->d_W, h->d_part, h->d_bd, h->d_bq,
                   h->d_pplanes, h->d_cplanes, h->d_becp, h->d_bdplanes, h->d_tcwork, h->d_tcstatus, h->d_rhok,
                   h->d_tw64[0], h->d_tw64[1], h->d_tw64[2], h->d_tw32[0], h->d_tw32[1], h->d_tw32[2]};
   for (void* p : ptrs)
@@ -877,6 +970,7 @@ int gwb_ham_set_projectors(gwb_ham* h, const void* p, const double* dij, void* s
   GWB_CUDA_TRY(cudaMemcpyAsync(h->d_d64, dij, nd * 8, cudaMemcpyDeviceToDevice, st));
   h->pplanes_ok = false;  // the tensor-core planes of P are rebuilt on next use
   k_scale_copy<float><<<blocks_for(nd, 256), 256, 0, st>>>(dij, h->d_d32, nd, 1.0);
+  k_column_lists<<<blocks_for(h->nproj, 64), 64, 0, st>>>(dij, h->nproj, h->d_cols.cnt, h->d_cols.idx);
   GWB_LAUNCH_CHECK();
   h->have_p = true;
   return GWB_OK;
@@ -947,9 +1041,11 @@ int gwb_ham_set_overlap(gwb_ham* h, const double* q, void* stream) {
   if (!h->d_q64) {
     GWB_CUDA_TRY(cudaMalloc((void**)&h->d_q64, nd * 8));
     GWB_CUDA_TRY(cudaMalloc((void**)&h->d_q32, nd * 4));
+    GWB_CUDA_TRY(alloc_columns(&h->q_cols, h->nproj));
   }
   GWB_CUDA_TRY(cudaMemcpyAsync(h->d_q64, q, nd * 8, cudaMemcpyDeviceToDevice, st));
   k_scale_copy<float><<<blocks_for(nd, 256), 256, 0, st>>>(q, h->d_q32, nd, 1.0);
+  k_column_lists<<<blocks_for(h->nproj, 64), 64, 0, st>>>(q, h->nproj, h->q_cols.cnt, h->q_cols.idx);
   GWB_LAUNCH_CHECK();
   h->have_q = true;
   return GWB_OK;

@@ -58,6 +58,7 @@ __global__ void __launch_bounds__(ZN_TN * 4) k_zmma_nn(int nb, int N, int K, con
     }
     cp_async_commit();
   };
+  chain_wait();
 #pragma unroll
   for (int p = 0; p < ZM_STAGES - 1; ++p) load(p);
 
@@ -124,13 +125,14 @@ cudaError_t zmma_nh(int M, int N, int K, int kslice, int ns, const cplx<double>*
       const cudaError_t e = allow_smem(k_zmma_nh<tm, tn>);                                                \
       if (e != cudaSuccess) return e;                                                                     \
     }                                                                                                     \
-    k_zmma_nh<tm, tn><<<grid, tn * 4, smem, st>>>(M, N, K, kslice, A, lda, sA, B, ldb, sB, part, batch);  \
+    return launch_chained(k_zmma_nh<tm, tn>, grid, tn * 4, smem, st, M, N, K, kslice, A, lda, sA, B, ldb, sB, \
+                          part, batch);                                                                   \
   }
 #define GWB_ZM_ROW(tm) GWB_ZM_CASE(tm, 8) GWB_ZM_CASE(tm, 16) GWB_ZM_CASE(tm, 24) GWB_ZM_CASE(tm, 32) GWB_ZM_CASE(tm, 64)
   GWB_ZM_ROW(8) GWB_ZM_ROW(16) GWB_ZM_ROW(24) GWB_ZM_ROW(32)
 #undef GWB_ZM_ROW
 #undef GWB_ZM_CASE
-  return cudaGetLastError();
+  return cudaErrorInvalidValue;
 }
 
 cudaError_t zmma_nn(int nb, int N, int K, const cplx<double>* A, const cplx<double>* A2, const cplx<double>* P,
@@ -139,18 +141,13 @@ cudaError_t zmma_nn(int nb, int N, int K, const cplx<double>* A, const cplx<doub
   const int rows = A2 ? 2 * nb : nb;
   const int TM = zmma_edge(rows, 32);
   const dim3 grid((unsigned)((N + ZN_TN - 1) / ZN_TN), (unsigned)((rows + TM - 1) / TM), batch);
-#define GWB_ZN_CASE(tm)                                                                                         \
-  if (TM == tm) {                                                                                               \
-    if (A2)                                                                                                     \
-      k_zmma_nn<tm, true><<<grid, ZN_TN * 4, zmma_nn_smem<tm>(), st>>>(nb, N, K, A, A2, P, c, ck, out_h, hk, out_s, \
-                                                                       sk, npw_k);                              \
-    else                                                                                                        \
-      k_zmma_nn<tm, false><<<grid, ZN_TN * 4, zmma_nn_smem<tm>(), st>>>(nb, N, K, A, A2, P, c, ck, out_h, hk,    \
-                                                                        out_s, sk, npw_k);                      \
-  }
+#define GWB_ZN_CASE(tm)                                                                                            \
+  if (TM == tm)                                                                                                    \
+    return launch_chained(A2 ? k_zmma_nn<tm, true> : k_zmma_nn<tm, false>, grid, ZN_TN * 4, zmma_nn_smem<tm>(), st, \
+                          nb, N, K, A, A2, P, c, ck, out_h, hk, out_s, sk, npw_k);
   GWB_ZN_CASE(8) GWB_ZN_CASE(16) GWB_ZN_CASE(24) GWB_ZN_CASE(32)
 #undef GWB_ZN_CASE
-  return cudaGetLastError();
+  return cudaErrorInvalidValue;
 }
 
 }  // namespace gwb

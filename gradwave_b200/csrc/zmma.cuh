@@ -97,6 +97,7 @@ __global__ void __launch_bounds__(TN * 4) k_zmma_nh(int M, int N, int K, int ksl
   for (int t = 0; t < MT; ++t)
 #pragma unroll
     for (int e = 0; e < 2; ++e) re[t][e] = im[t][e] = sr[t][e] = si[t][e] = 0.0;
+  chain_wait();
 #pragma unroll
   for (int p = 0; p < ZM_STAGES - 1; ++p) load(p);
   for (int step = 0; step < nsteps; ++step) {
