@@ -138,6 +138,12 @@ template <typename T> __device__ __forceinline__ T* after_wait(T* p) {
   return p;
 }
 
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
+
 // Raise a kernel's dynamic shared-memory cap to the device's opt-in maximum
 // (less its static shared memory), once per (kernel, device). The cap is a
 // process-wide attribute of the kernel: setting it to each launch's own size

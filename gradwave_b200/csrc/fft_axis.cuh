@@ -54,7 +54,7 @@ template <typename T> struct FftRun {
   const int* map;        // (nk, nrow, n2) sphere index of each row point, -1: none
   const int* rowof;      // (nk, L0, n1) row slot of (j0, i1), -1: none
   const int* npw;        // (nk)
-  const cplx<T>* tw0;    // exp(-2 pi i t / n) per axis
+  const cplx<T>* tw0;    // per axis, n = R1 R2: exp(-2 pi i a k / n) at k R2 + a, a < R2, k < R1
   const cplx<T>* tw1;
   const cplx<T>* tw2;
   cplx<T>* W2;           // (nk, nbc, nrow, n2)
@@ -96,7 +96,8 @@ template <typename T, int N> struct AxisCfg {
   // blocks per SM the registers are limited for (at most 113 registers in
   // float64, 64 in float32; the 25-point pass of 125 needs more)
   static constexpr int minb(int nt, int threads = sizeof(T) == 8 ? 576 : 1024) {
-    return R2 > 16 || threads < nt ? 1 : threads / nt;
+    const int t = R2 == 1 ? threads * 5 / 8 : threads;  // one pass holds all N points
+    return R2 > 16 || t < nt ? 1 : t / nt;
   }
   static constexpr size_t smem_strided = R2 == 1 ? 0 : (size_t)N * PB * sizeof(cplx<T>);
   static constexpr size_t smem_rows = R2 == 1 ? 0 : (size_t)RB * R1 * P2 * sizeof(cplx<T>);
@@ -106,23 +107,71 @@ namespace fft_detail {
 
 using rdft_detail::StaticFor;
 
-template <int SIGN, typename T> __device__ __forceinline__ cplx<T> tw_at(const cplx<T>* __restrict__ tw, int i) {
-  const cplx<T> w = tw[i];
+template <int SIGN, typename T> __device__ __forceinline__ cplx<T> tw_at(const cplx<T>* tw) {
+  const cplx<T> w = *tw;
   return SIGN > 0 ? conj(w) : w;
 }
 
-// First pass: R1 points x[a + R2 b] -> exchange slots [k1][a], twiddled.
-template <typename T, int R1, int SIGN, class PUT>
-__device__ __forceinline__ void pass1(cplx<T> (&x)[R1], int a, const cplx<T>* __restrict__ tw, PUT&& put) {
+// First pass: R1 points x[a + R2 b] -> exchange slots [k1][a], twiddled; twa =
+// the axis table at column a (row k1: w_N^(a k1)), so that every twiddle is a
+// load at a constant offset.
+template <typename T, int R1, int R2, int SIGN, class PUT>
+__device__ __forceinline__ void pass1(cplx<T> (&x)[R1], const cplx<T>* __restrict__ twa, PUT&& put) {
   rdft<R1, SIGN>(x);
   StaticFor<0, R1>::run([&](auto kc) {
     constexpr int k1 = decltype(kc)::value;
-    put(k1, k1 == 0 ? x[0] : x[k1] * tw_at<SIGN>(tw, a * k1));
+    put(k1, k1 == 0 ? x[0] : x[k1] * tw_at<SIGN>(twa + k1 * R2));
   });
 }
 
-template <typename T> __device__ __forceinline__ cplx<T> load_io(const void* p, int io64, size_t i) {
-  return io64 ? ld<T>((const cplx<double>*)p, i) : ld<T>((const cplx<float>*)p, i);
+// Loads (0 where p is false) and stores under a predicate: written as branches
+// they took 40 % of the branch unit's cycles and a third of the issue slots of
+// the float32 kernels.
+__device__ __forceinline__ cplx<double> ld_if(bool p, const cplx<double>* a) {
+  cplx<double> v;
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %3, 0;\n\tmov.f64 %0, 0d0000000000000000;\n\t"
+      "mov.f64 %1, 0d0000000000000000;\n\t@q ld.global.v2.f64 {%0, %1}, [%2];\n\t}"
+      : "=&d"(v.x), "=&d"(v.y)
+      : "l"(a), "r"((int)p)
+      : "memory");
+  return v;
+}
+__device__ __forceinline__ cplx<float> ld_if(bool p, const cplx<float>* a) {
+  cplx<float> v;
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %3, 0;\n\tmov.f32 %0, 0f00000000;\n\t"
+      "mov.f32 %1, 0f00000000;\n\t@q ld.global.v2.f32 {%0, %1}, [%2];\n\t}"
+      : "=&f"(v.x), "=&f"(v.y)
+      : "l"(a), "r"((int)p)
+      : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_if(bool p, cplx<double>* a, cplx<double> v) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %3, 0;\n\t@q st.global.v2.f64 [%0], {%1, %2};\n\t}" ::"l"(a),
+               "d"(v.x), "d"(v.y), "r"((int)p)
+               : "memory");
+}
+__device__ __forceinline__ void st_if(bool p, cplx<float>* a, cplx<float> v) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %3, 0;\n\t@q st.global.v2.f32 [%0], {%1, %2};\n\t}" ::"l"(a),
+               "f"(v.x), "f"(v.y), "r"((int)p)
+               : "memory");
+}
+
+// element i of a complex128 or complex64 array (0 where i < 0) in precision T
+template <typename T, typename SIO> __device__ __forceinline__ cplx<T> load_io(const SIO* p, int i) {
+  const SIO v = ld_if(i >= 0, p + i);
+  return mk<T>((T)v.x, (T)v.y);
+}
+
+// one complex element, global to shared memory, asynchronously (0 where p is false)
+template <typename T> __device__ __forceinline__ void cp_async_elem(bool p, cplx<T>* dst, const cplx<T>* src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  const int n = p ? (int)sizeof(cplx<T>) : 0;
+  if constexpr (sizeof(cplx<T>) == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
 }
 
 // memory row r of axis 0 -> offset of its occupied plane in W, or -1
@@ -156,17 +205,20 @@ __global__ void __launch_bounds__(AxisCfg<T, N>::NTR, AxisCfg<T, N>::minb(AxisCf
       });
       chain_wait();
       cplx<T> x[R1];
-      StaticFor<0, R1>::run([&](auto bc) {
-        constexpr int b = decltype(bc)::value;
-        x[b] = idx[b] >= 0 ? load_io<T>(f.c, f.io64, crow + idx[b]) : mk<T>(0, 0);
-      });
+      if (f.io64) {
+        const cplx<double>* c = (const cplx<double>*)f.c + crow;
+        StaticFor<0, R1>::run([&](auto bc) { x[decltype(bc)::value] = load_io<T>(c, idx[decltype(bc)::value]); });
+      } else {
+        const cplx<float>* c = (const cplx<float>*)f.c + crow;
+        StaticFor<0, R1>::run([&](auto bc) { x[decltype(bc)::value] = load_io<T>(c, idx[decltype(bc)::value]); });
+      }
       if constexpr (R2 == 1) {
         rdft<R1, +1>(x);
         cplx<T>* dst = f.W2 + (((size_t)k * f.nbc + bl) * f.nrow + row) * N;
         StaticFor<0, R1>::run([&](auto bc) { dst[decltype(bc)::value] = x[decltype(bc)::value]; });
       } else {
         cplx<T>* e = ex + r * (R1 * P2) + a;
-        pass1<T, R1, +1>(x, a, f.tw2, [&](int k1, cplx<T> v) { e[k1 * P2] = v; });
+        pass1<T, R1, R2, +1>(x, f.tw2 + a, [&](int k1, cplx<T> v) { e[k1 * P2] = v; });
       }
     }
   }
@@ -198,11 +250,15 @@ __global__ void __launch_bounds__(AxisCfg<T, N>::NTR, AxisCfg<T, N>::minb(AxisCf
   const size_t orow = (size_t)k * f.ok + (size_t)(f.b0 + bl) * f.npw_max;
   const T* tk = f.t + (size_t)k * f.npw_max;
   chain_wait();
-  auto store = [&](int g, cplx<T> val) {
-    const cplx<T> cv = load_io<T>(f.c, f.io64, crow + g);
-    const cplx<T> o = val + scale(cv, tk[g]);
-    if (f.io64) st((cplx<double>*)f.out, orow + g, o);
-    else st((cplx<float>*)f.out, orow + g, o);
+  auto store = [&](int g, cplx<T> val) {  // where g >= 0
+    const T tg = g >= 0 ? tk[g] : (T)0;
+    if (f.io64) {
+      const cplx<T> o = val + scale(load_io<T>((const cplx<double>*)f.c + crow, g), tg);
+      st_if(g >= 0, (cplx<double>*)f.out + orow + g, mk<double>(o.x, o.y));
+    } else {
+      const cplx<T> o = val + scale(load_io<T>((const cplx<float>*)f.c + crow, g), tg);
+      st_if(g >= 0, (cplx<float>*)f.out + orow + g, mk<float>((float)o.x, (float)o.y));
+    }
   };
   {
     const int a = tid % R2, r = tid / R2, row = row0 + r;
@@ -214,12 +270,11 @@ __global__ void __launch_bounds__(AxisCfg<T, N>::NTR, AxisCfg<T, N>::minb(AxisCf
         rdft<R1, -1>(x);
         const int* mp = f.map + ((size_t)k * f.nrow + row) * N;
         StaticFor<0, R1>::run([&](auto bc) {
-          const int g = mp[decltype(bc)::value];
-          if (g >= 0) store(g, x[decltype(bc)::value]);
+          store(mp[decltype(bc)::value], x[decltype(bc)::value]);
         });
       } else {
         cplx<T>* e = ex + r * (R1 * P2) + a;
-        pass1<T, R1, -1>(x, a, f.tw2, [&](int k1, cplx<T> v) { e[k1 * P2] = v; });
+        pass1<T, R1, R2, -1>(x, f.tw2 + a, [&](int k1, cplx<T> v) { e[k1 * P2] = v; });
       }
     }
   }
@@ -236,7 +291,7 @@ __global__ void __launch_bounds__(AxisCfg<T, N>::NTR, AxisCfg<T, N>::minb(AxisCf
         constexpr int o = R1 * decltype(kc)::value;
         const int i2 = k1 + o;
         const int g = (i2 <= f.M2 || i2 >= N - f.M2) ? mp[o] : -1;
-        if (g >= 0) store(g, y[decltype(kc)::value]);
+        store(g, y[decltype(kc)::value]);
       });
     }
   }
@@ -273,7 +328,7 @@ __global__ void __launch_bounds__(AxisCfg<T, N>::NT, AxisCfg<T, N>::minb(AxisCfg
     cplx<T> x[R1];
     StaticFor<0, R1>::run([&](auto bc) {
       constexpr int b = decltype(bc)::value;
-      x[b] = idx[b] >= 0 ? src[idx[b] * n2] : mk<T>(0, 0);
+      x[b] = ld_if(idx[b] >= 0, src + idx[b] * n2);
     });
     if constexpr (R2 == 1) {
       rdft<R1, +1>(x);
@@ -281,7 +336,7 @@ __global__ void __launch_bounds__(AxisCfg<T, N>::NT, AxisCfg<T, N>::minb(AxisCfg
       StaticFor<0, R1>::run([&](auto bc) { dst[decltype(bc)::value * n2] = x[decltype(bc)::value]; });
     } else {
       cplx<T>* e = ex + s * PB + c;
-      pass1<T, R1, +1>(x, s, f.tw1, [&](int k1, cplx<T> v) { e[k1 * (R2 * PB)] = v; });
+      pass1<T, R1, R2, +1>(x, f.tw1 + s, [&](int k1, cplx<T> v) { e[k1 * (R2 * PB)] = v; });
     }
   }
   if constexpr (R2 > 1) {
@@ -322,11 +377,11 @@ __global__ void __launch_bounds__(AxisCfg<T, N>::NT, AxisCfg<T, N>::minb(AxisCfg
       rdft<R1, -1>(x);
       StaticFor<0, R1>::run([&](auto bc) {
         const int row = ro[decltype(bc)::value];
-        if (row >= 0) dst[row * n2] = x[decltype(bc)::value];
+        st_if(row >= 0, dst + row * n2, x[decltype(bc)::value]);
       });
     } else {
       cplx<T>* e = ex + s * PB + c;
-      pass1<T, R1, -1>(x, s, f.tw1, [&](int k1, cplx<T> v) { e[k1 * (R2 * PB)] = v; });
+      pass1<T, R1, R2, -1>(x, f.tw1 + s, [&](int k1, cplx<T> v) { e[k1 * (R2 * PB)] = v; });
     }
   }
   if constexpr (R2 > 1) {
@@ -339,7 +394,7 @@ __global__ void __launch_bounds__(AxisCfg<T, N>::NT, AxisCfg<T, N>::minb(AxisCfg
       StaticFor<0, R2>::run([&](auto kc) {
         constexpr int k2 = decltype(kc)::value;
         const int row = ro[s + R1 * k2];
-        if (row >= 0) dst[row * n2] = y[k2];
+        st_if(row >= 0, dst + row * n2, y[k2]);
       });
     }
   }
@@ -349,8 +404,10 @@ __global__ void __launch_bounds__(AxisCfg<T, N>::NT, AxisCfg<T, N>::minb(AxisCfg
 // v(r)/N, forward. After the inverse a thread holds the R2 points
 // i0 = k1 + R1 k2 of its pencil; the forward transform starts on exactly these
 // (DFT over k2 first, twiddle w_N^(k1 m2), exchange, DFT over k1), so the pair
-// costs two exchanges. v is read from L1 after the first band of the group
-// (kept in registers it made the float64 kernels spill).
+// costs two exchanges, in place in one buffer. v is read from L1 after the
+// first band of the group (kept in registers it made the float64 kernels
+// spill). The next band's points travel to shared memory while this band is
+// transformed.
 template <typename T, int N>
 __global__ void __launch_bounds__(AxisCfg<T, N>::NT, AxisCfg<T, N>::minb(AxisCfg<T, N>::NT))
     k_pencil_vloc(const FftRun<T> f, int bands_per_block) {
@@ -358,8 +415,8 @@ __global__ void __launch_bounds__(AxisCfg<T, N>::NT, AxisCfg<T, N>::minb(AxisCfg
   using namespace fft_detail;
   constexpr int R1 = C::R1, R2 = C::R2, PB = C::PB;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  cplx<T>* ex1 = reinterpret_cast<cplx<T>*>(smem_raw);
-  cplx<T>* ex2 = ex1 + N * PB;
+  cplx<T>* ex = reinterpret_cast<cplx<T>*>(smem_raw);
+  cplx<T>* in = ex + N * PB + threadIdx.x;  // this thread's R1 points of the next band, NT apart
   const int k = blockIdx.z;
   const int plane = f.n1 * f.n2;  // box indices fit 32 bits (axes <= 128)
   const int c = threadIdx.x % PB, s = threadIdx.x / PB;
@@ -367,23 +424,38 @@ __global__ void __launch_bounds__(AxisCfg<T, N>::NT, AxisCfg<T, N>::minb(AxisCfg
   const bool live = p < plane;
   const int M0 = f.M0, L0 = f.L0;
   const int bl0 = blockIdx.y * bands_per_block, bl1 = min(f.nbc, bl0 + bands_per_block);
-  chain_wait();
-  for (int bl = bl0; bl < bl1; ++bl) {
-    // opaque per band: hoisted out of the loop, the twiddles and the 2 R1 + R2
-    // addresses take more registers than there are
-    const T* vp = f.v + p + s * plane;
-    const cplx<T>* tw = f.tw0;
-    int s_ = s;
-    asm volatile("" : "+l"(vp), "+l"(tw), "+r"(s_));
-    cplx<T>* base = f.W + ((size_t)k * f.nbc + bl) * (size_t)(L0 * plane) + p;
-    if (live) {
-      cplx<T> x[R1];
+  int off[R1];  // planes of the pencil's points s + R2 b in W
+  StaticFor<0, R1>::run([&](auto bc) {
+    constexpr int b = decltype(bc)::value;
+    off[b] = plane_of(s + R2 * b, M0, L0, N, plane);
+  });
+  auto band = [&](int bl) { return f.W + ((size_t)k * f.nbc + bl) * (size_t)(L0 * plane) + p; };
+  auto fetch = [&](int bl) {
+    if (live && bl < bl1) {
+      const cplx<T>* base = band(bl);
       StaticFor<0, R1>::run([&](auto bc) {
         constexpr int b = decltype(bc)::value;
-        const int o = plane_of(s_ + R2 * b, M0, L0, N, plane);
-        x[b] = o >= 0 ? base[o] : mk<T>(0, 0);
+        cp_async_elem(off[b] >= 0, in + b * C::NT, base + max(off[b], 0));
       });
-      if constexpr (R2 == 1) {
+    }
+    cp_async_commit();
+  };
+  chain_wait();
+  if constexpr (R2 > 1) fetch(bl0);
+  for (int bl = bl0; bl < bl1; ++bl) {
+    // opaque per band: hoisted out of the loop, the twiddles and the addresses
+    // take more registers than there are
+    const T* vp = f.v + p + s * plane;
+    const cplx<T>* tw = f.tw0;
+    asm volatile("" : "+l"(vp), "+l"(tw));
+    cplx<T>* base = band(bl);
+    if constexpr (R2 == 1) {
+      if (live) {
+        cplx<T> x[R1];
+        StaticFor<0, R1>::run([&](auto bc) {
+          constexpr int b = decltype(bc)::value;
+          x[b] = ld_if(off[b] >= 0, base + off[b]);
+        });
         rdft<R1, +1>(x);
         StaticFor<0, R1>::run([&](auto bc) {
           x[decltype(bc)::value] = scale(x[decltype(bc)::value], vp[decltype(bc)::value * plane]);
@@ -391,18 +463,25 @@ __global__ void __launch_bounds__(AxisCfg<T, N>::NT, AxisCfg<T, N>::minb(AxisCfg
         rdft<R1, -1>(x);
         StaticFor<0, R1>::run([&](auto bc) {
           constexpr int b = decltype(bc)::value;
-          const int o = plane_of(b, M0, L0, N, plane);
-          if (o >= 0) base[o] = x[b];
+          st_if(off[b] >= 0, base + off[b], x[b]);
         });
-      } else {
-        cplx<T>* e = ex1 + s * PB + c;
-        pass1<T, R1, +1>(x, s_, tw, [&](int k1, cplx<T> v) { e[k1 * (R2 * PB)] = v; });
       }
-    }
-    if constexpr (R2 > 1) {
-      __syncthreads();  // also: every thread has read ex2 of the band before
+    } else {
+      cp_async_wait<0>();  // the points are this thread's own: no barrier
+      if (live) {
+        cplx<T> x[R1];
+        StaticFor<0, R1>::run([&](auto bc) {
+          constexpr int b = decltype(bc)::value;
+          x[b] = in[b * C::NT];
+        });
+        cplx<T>* e = ex + s * PB + c;
+        pass1<T, R1, R2, +1>(x, tw + s, [&](int k1, cplx<T> v) { e[k1 * (R2 * PB)] = v; });
+      }
+      fetch(bl + 1);
+      __syncthreads();
+      // the R2 points of one k1 are read and written by one thread: in place
       if (s < R1 && live) {
-        const cplx<T>* e = ex1 + s * (R2 * PB) + c;
+        cplx<T>* e = ex + s * (R2 * PB) + c;
         cplx<T> y[R2];
         StaticFor<0, R2>::run([&](auto ac) { y[decltype(ac)::value] = e[decltype(ac)::value * PB]; });
         rdft<R2, +1>(y);
@@ -410,22 +489,22 @@ __global__ void __launch_bounds__(AxisCfg<T, N>::NT, AxisCfg<T, N>::minb(AxisCfg
           y[decltype(kc)::value] = scale(y[decltype(kc)::value], vp[R1 * decltype(kc)::value * plane]);
         });
         rdft<R2, -1>(y);
-        cplx<T>* o = ex2 + s * (R2 * PB) + c;
         StaticFor<0, R2>::run([&](auto mc) {
           constexpr int m2 = decltype(mc)::value;
-          o[m2 * PB] = m2 == 0 ? y[0] : y[m2] * tw_at<-1>(tw, s_ * m2);
+          e[m2 * PB] = m2 == 0 ? y[0] : y[m2] * tw_at<-1>(tw + s * R2 + m2);
         });
       }
-      __syncthreads();  // also: every thread has read ex1 before the next band fills it
+      __syncthreads();
+      // column s of the exchange is read here and written by the next band's
+      // first pass, both by this thread
       if (live) {
-        const cplx<T>* e = ex2 + s * PB + c;
+        const cplx<T>* e = ex + s * PB + c;
         cplx<T> x[R1];
         StaticFor<0, R1>::run([&](auto kc) { x[decltype(kc)::value] = e[decltype(kc)::value * (R2 * PB)]; });
         rdft<R1, -1>(x);
         StaticFor<0, R1>::run([&](auto bc) {
           constexpr int b = decltype(bc)::value;
-          const int o = plane_of(s_ + R2 * b, M0, L0, N, plane);
-          if (o >= 0) base[o] = x[b];
+          st_if(off[b] >= 0, base + off[b], x[b]);
         });
       }
     }
@@ -474,14 +553,14 @@ __global__ void __launch_bounds__(AxisCfg<T, N>::NT, AxisCfg<T, N>::minb(AxisCfg
       StaticFor<0, R1>::run([&](auto bc) {
         constexpr int b = decltype(bc)::value;
         const int o = plane_of(s_ + R2 * b, M0, L0, N, plane);
-        x[b] = o >= 0 ? base[o] : mk<T>(0, 0);
+        x[b] = ld_if(o >= 0, base + o);
       });
       if constexpr (R2 == 1) {
         rdft<R1, +1>(x);
         StaticFor<0, R1>::run([&](auto bc) { add(acc[decltype(bc)::value], x[decltype(bc)::value]); });
       } else {
         cplx<T>* e = exb + s * PB + c;
-        pass1<T, R1, +1>(x, s_, tw, [&](int k1, cplx<T> v) { e[k1 * (R2 * PB)] = v; });
+        pass1<T, R1, R2, +1>(x, tw + s, [&](int k1, cplx<T> v) { e[k1 * (R2 * PB)] = v; });
       }
     }
     if constexpr (R2 > 1) {
@@ -531,11 +610,12 @@ template <typename T, int N> cudaError_t launch_vloc(const FftRun<T>& f, cudaStr
   while (groups < f.nbc && (int64_t)blocks * f.nk * groups < 4 * 148) ++groups;
   const int bpb = (f.nbc + groups - 1) / groups;
   dim3 g(blocks, (f.nbc + bpb - 1) / bpb, f.nk);
-  if (2 * C::smem_strided > 48 * 1024) {
+  constexpr size_t smem = C::R2 == 1 ? 0 : C::smem_strided + (size_t)C::R1 * C::NT * sizeof(cplx<T>);
+  if (smem > 48 * 1024) {
     const cudaError_t e = allow_smem(k_pencil_vloc<T, N>);
     if (e != cudaSuccess) return e;
   }
-  return launch_chained(k_pencil_vloc<T, N>, g, C::NT, 2 * C::smem_strided, st, f, bpb);
+  return launch_chained(k_pencil_vloc<T, N>, g, C::NT, smem, st, f, bpb);
 }
 
 template <typename T, int N> cudaError_t launch_density(const FftRun<T>& f, cudaStream_t st) {

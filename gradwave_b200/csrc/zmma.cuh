@@ -33,12 +33,6 @@ __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc, boo
   const int n = valid ? 16 : 0;  // 0: zero-fill, nothing read
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(gsrc), "r"(n) : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
-
 // d += a b for one 8x8x4 tile: lane l holds a[l / 4][l % 4], b[l % 4][l / 4] and
 // d[l / 4][2 (l % 4) + {0, 1}].
 __device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
