@@ -585,8 +585,9 @@ __global__ void k_precond_normalize(int npw, int n_add, int chunks, const double
 // Warpgroups per CTA, each with its own tile, A rows, accumulator and barriers,
 // all on one copy of the weights: eight tiles in flight per SM where CTAs of one
 // tile each fitted five (their weights took half of the shared memory). Bound by
-// the latency of a tile's three MMA rounds and by the tanh unit (192 per plane
-// wave, 0.66 ms of it here); 404 rows of 37,000 plane waves: 1410 -> 1261 us.
+// the latency of a tile's three MMA rounds and by the special-function unit (192
+// tanh per plane wave, 0.66 ms of it here); 404 rows of 37,000 plane waves:
+// 1410 -> 1261 us, 1105 with the roundings off that unit (silu_bf16_2).
 constexpr int PU_WG = 4;
 constexpr int PU_THREADS = 128 * PU_WG;
 constexpr int PU_TILE = 128;
@@ -639,6 +640,49 @@ struct PuArgs {
   long long wait_cycles;
 };
 
+// Packed float32 pairs.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pk2(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void un2(f32x2 v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+// SiLU of two activations (silu_fast) and its rounding to BF16, still as
+// float32: the upper part of a split at 16 bits (Dekker, Numer. Math. 18 (1971)
+// 224), g = 65537 h, h + (g - h) rounded, is the nearest BF16 value. A
+// conversion instruction would take the special-function unit, which the tanh
+// has to itself here: with the conversions it ran 300 instead of about 205
+// operations per plane wave at 80 % of its rate.
+__device__ __forceinline__ f32x2 silu_bf16_2(uint32_t z0, uint32_t z1) {
+  const f32x2 h = mul2(pk2(__uint_as_float(z0), __uint_as_float(z1)), pk2(0.5f, 0.5f));
+  float h0, h1;
+  un2(h, h0, h1);
+  const f32x2 y = fma2(h, pk2(tanh_approx(h0), tanh_approx(h1)), h);
+  const f32x2 g = mul2(y, pk2(65537.f, 65537.f));
+  const f32x2 d = fma2(g, pk2(-1.f, -1.f), y);
+  return fma2(g, pk2(1.f, 1.f), d);
+}
+// the pair as two BF16 (its low halves are zero)
+__device__ __forceinline__ uint32_t pack_hi(f32x2 v) {
+  float a, b;
+  un2(v, a, b);
+  return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
+}
+
 // This warp's 32 rows of the 64 accumulator columns, 16 at a time: SiLU,
 // then either the BF16 chunks of the next A (hidden layers) or, for the last
 // hidden layer, layer 4's dot product with w4 added to o in column order.
@@ -649,20 +693,22 @@ __device__ __forceinline__ float pu_hidden(uint32_t taddr, uint8_t* sA, int row,
     uint32_t r[16];
     tmem_ld16(taddr + 16 * q, r);
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-    float h[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) h[i] = silu_fast(__uint_as_float(r[i]));
     if (last) {
 #pragma unroll
-      for (int i = 0; i < 16; ++i) o = fmaf(bf(h[i]), w4[16 * q + i], o);
+      for (int i = 0; i < 16; i += 2) {
+        float h0, h1;
+        un2(silu_bf16_2(r[i], r[i + 1]), h0, h1);
+        o = fmaf(h0, w4[16 * q + i], o);
+        o = fmaf(h1, w4[16 * q + i + 1], o);
+      }
     } else {
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         uint4 v;
-        v.x = pack_bf16(h[8 * c + 0], h[8 * c + 1]);
-        v.y = pack_bf16(h[8 * c + 2], h[8 * c + 3]);
-        v.z = pack_bf16(h[8 * c + 4], h[8 * c + 5]);
-        v.w = pack_bf16(h[8 * c + 6], h[8 * c + 7]);
+        v.x = pack_hi(silu_bf16_2(r[8 * c + 0], r[8 * c + 1]));
+        v.y = pack_hi(silu_bf16_2(r[8 * c + 2], r[8 * c + 3]));
+        v.z = pack_hi(silu_bf16_2(r[8 * c + 4], r[8 * c + 5]));
+        v.w = pack_hi(silu_bf16_2(r[8 * c + 6], r[8 * c + 7]));
         *reinterpret_cast<uint4*>(sA + pu_off(row, 16 * q + 8 * c, PU_K)) = v;
       }
     }
