@@ -37,6 +37,8 @@ int blas_handle(cublasHandle_t* out) {
   return GWB_OK;
 }
 
+constexpr int64_t kShortRows = 64;
+
 static cublasOperation_t to_op(int op) {
   return op == 0 ? CUBLAS_OP_N : (op == 1 ? CUBLAS_OP_T : CUBLAS_OP_C);
 }
@@ -53,6 +55,16 @@ extern "C" int gwb_zgemm(int opA, int opB, int64_t M, int64_t N, int64_t K, doub
   GWB_REQUIRE(M >= 0 && N >= 0 && K >= 0 && batch >= 0, "negative size");
   if (M == 0 || N == 0 || batch == 0) return GWB_OK;
   GWB_REQUIRE(A && B && C, "null matrix");
+  // few rows against long ones (the solver's triangular transforms, projections
+  // and Ritz vectors of small blocks): own tiles, launched in chain; cuBLAS for
+  // the rest, whose larger tiles load less
+  if (opB == 0 && opA <= 1 && M <= kShortRows && N >= 8 * M && K > 0 && batch <= 65535) {
+    GWB_CUDA_TRY(zmma_ab(opA == 1, (int)M, (int)N, (int)K, mk<double>(alpha_re, alpha_im), (const cplx<double>*)A, lda,
+                         strideA, (const cplx<double>*)B, ldb, strideB, mk<double>(beta_re, beta_im), (cplx<double>*)C,
+                         ldc, strideC, (int)batch, (cudaStream_t)stream));
+    count_launches(1);
+    return GWB_OK;
+  }
   cublasHandle_t h;
   int rc = blas_handle(&h);
   if (rc) return rc;

@@ -39,12 +39,17 @@ __global__ void __launch_bounds__(256) k_residual(int npw, const cplx<double>* _
                                                   cplx<double>* __restrict__ r, int64_t rk,
                                                   double* __restrict__ rn, int nb) {
   __shared__ double red[8];
+  chain_wait();
+  x = after_wait(x);
+  hx = after_wait(hx);
+  eig = after_wait(eig);
   const int k = blockIdx.x / nb, b = blockIdx.x % nb;
   const double e = eig[k * ek + b];
   const cplx<double>* xr = x + k * xk + (int64_t)b * npw;
   const cplx<double>* hr = hx + k * hk + (int64_t)b * npw;
   cplx<double>* rr = r + k * rk + (int64_t)b * npw;
   double acc = 0.0;
+#pragma unroll 4
   for (int g = threadIdx.x; g < npw; g += blockDim.x) {
     const cplx<double> v = hr[g] - scale(xr[g], e);
     rr[g] = v;
@@ -57,6 +62,8 @@ __global__ void __launch_bounds__(256) k_residual(int npw, const cplx<double>* _
 __global__ void k_conv_stats(const double* __restrict__ rn, int nk, int nb, double tol, double* __restrict__ out) {
   __shared__ double smax[32];
   __shared__ int scnt[32];
+  chain_wait();
+  rn = after_wait(rn);
   // thread t handles k = t (nk <= 1024 per launch chunk loop)
   double mx = 0.0;
   int best = 0;
@@ -92,6 +99,8 @@ __global__ void k_conv_stats(const double* __restrict__ rn, int nk, int nb, doub
 
 // Stable descending order by |r|: rank = #(larger) + #(equal and earlier).
 __global__ void k_select_worst(const double* __restrict__ rn, int nb, int n_add, int* __restrict__ sel) {
+  chain_wait();
+  rn = after_wait(rn);
   const int k = blockIdx.x;
   const double* row = rn + (int64_t)k * nb;
   for (int b = threadIdx.x; b < nb; b += blockDim.x) {
@@ -121,6 +130,10 @@ __global__ void __launch_bounds__(256) k_precond_teter(int npw, int nb, int n_ad
                                                        const int* __restrict__ sel,
                                                        cplx<double>* __restrict__ d, int64_t dk) {
   __shared__ double red[8];
+  chain_wait();
+  x = after_wait(x);
+  r = after_wait(r);
+  sel = after_wait(sel);
   const int k = blockIdx.x / n_add, s = blockIdx.x % n_add;
   const int b = sel[(int64_t)k * n_add + s];
   const cplx<double>* xr = x + k * xk + (int64_t)b * npw;
@@ -128,9 +141,11 @@ __global__ void __launch_bounds__(256) k_precond_teter(int npw, int nb, int n_ad
   const double* tk = t + (int64_t)k * npw;
   cplx<double>* dr = d + k * dk + (int64_t)s * npw;
   double tb = 0.0;
+#pragma unroll 4
   for (int g = threadIdx.x; g < npw; g += blockDim.x) tb += tk[g] * norm2(xr[g]);
   tb = block_sum<256>(tb, red);
   double nn = 0.0;
+#pragma unroll 4
   for (int g = threadIdx.x; g < npw; g += blockDim.x) {
     const cplx<double> v = scale(rr[g], tpa(tk[g], tb));
     dr[g] = v;
@@ -139,6 +154,7 @@ __global__ void __launch_bounds__(256) k_precond_teter(int npw, int nb, int n_ad
   nn = sqrt(block_sum<256>(nn, red));
   if (nn > 1e-300) {
     const double inv = 1.0 / nn;
+#pragma unroll 4
     for (int g = threadIdx.x; g < npw; g += blockDim.x) dr[g] = scale(dr[g], inv);
   }
 }
@@ -147,6 +163,8 @@ __global__ void __launch_bounds__(256) k_precond_teter(int npw, int nb, int n_ad
 // columns j >= m0 and their mirrored rows; the new diagonal block is Hermitised.
 __global__ void k_subspace_insert(const cplx<double>* __restrict__ C, int m, int m0, cplx<double>* __restrict__ S,
                                   int lds, int64_t sk) {
+  chain_wait();
+  C = after_wait(C);
   const int k = blockIdx.y;
   const int nnew = m - m0;
   const int64_t total = (int64_t)m * nnew;
@@ -221,69 +239,64 @@ __global__ void __launch_bounds__(256) k_chol_inv(cplx<double>* __restrict__ G, 
   }
 }
 
-// Shared-memory version for n <= CHOL_SMEM_MAX: the same column-by-column
-// Cholesky and forward substitution, with L and L^-1 kept on chip (the global
-// version is bound by L2 latency on these tiny dependent loops). The inverse
-// runs row by row: row i of L^-1 needs rows < i only, all columns in parallel.
+// Shared-memory version for n <= CHOL_SMEM_MAX, right-looking, with the inverse
+// carried along: step j scales row j of W (W starts as the identity, W = L^-1
+// at the end) and subtracts l_ij times column j of L from the trailing matrix
+// and row j of W from the rows below, all entries at once. Two barriers and one
+// square root per column; dot products per entry with a block reduction per
+// column took 22 us at n = 24 (bound by their dependent loads).
 constexpr int CHOL_SMEM_MAX = 64;
-__global__ void __launch_bounds__(256) k_chol_inv_smem(cplx<double>* __restrict__ G, int n, int ld, int64_t gk,
+__global__ void __launch_bounds__(256) k_chol_inv_smem(cplx<double>* G, int n, int ld, int64_t gk,
                                                        cplx<double>* __restrict__ Linv, int64_t lk,
                                                        int* __restrict__ info, int* __restrict__ flag) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  cplx<double>* A = reinterpret_cast<cplx<double>*>(smem_raw);  // n*n
-  cplx<double>* Li = A + n * n;                                 // n*n
-  __shared__ double red[8];
+  cplx<double>* A = reinterpret_cast<cplx<double>*>(smem_raw);  // n*n, L in the lower triangle
+  cplx<double>* W = A + n * n;                                  // n*n
   __shared__ int bad;
-  const int k = blockIdx.x;
-  for (int i = threadIdx.x; i < n * n; i += blockDim.x) A[i] = G[k * gk + (int64_t)(i / n) * ld + (i % n)];
-  if (threadIdx.x == 0) bad = 0;
+  const int k = blockIdx.x, tid = threadIdx.x;
+  chain_wait();
+  for (int i = tid; i < n * n; i += blockDim.x) {
+    const int r = i / n, c = i - r * n;
+    A[i] = G[k * gk + (int64_t)r * ld + c];
+    W[i] = mk<double>(r == c ? 1.0 : 0.0, 0.0);
+  }
+  if (tid == 0) bad = 0;
   __syncthreads();
+  const int ti = tid >> 4, tc = tid & 15;  // 16 x 16 threads over rows and columns
   for (int j = 0; j < n; ++j) {
-    double s = 0.0;
-    for (int q = threadIdx.x; q < j; q += blockDim.x) s += norm2(A[j * n + q]);
-    s = block_sum<256>(s, red);
-    const double dj = A[j * n + j].x - s;
-    if (!(dj > 0.0) || !isfinite(dj)) {
-      if (threadIdx.x == 0) bad = j + 1;
-      __syncthreads();
+    const double dj = A[j * n + j].x;
+    if (!(dj > 0.0) || !isfinite(dj)) {  // the same for every thread
+      if (tid == 0) bad = j + 1;
       break;
     }
-    const double ljj = sqrt(dj), inv = 1.0 / ljj;
-    for (int i = j + 1 + threadIdx.x; i < n; i += blockDim.x) {
-      cplx<double> acc = A[i * n + j];
-      for (int q = 0; q < j; ++q) acc = acc - mul_conj(A[i * n + q], A[j * n + q]);
-      A[i * n + j] = scale(acc, inv);
+    const double inv = rsqrt(dj);
+    // row j of W and column j of L take their scale; the pivot itself stays
+    // untouched until every thread has read it
+    if (tid < n) {
+      if (tid <= j) W[j * n + tid] = scale(W[j * n + tid], inv);
+      else A[tid * n + j] = scale(A[tid * n + j], inv);
     }
     __syncthreads();
-    if (threadIdx.x == 0) A[j * n + j] = mk<double>(ljj, 0.0);
+    for (int i = j + 1 + ti; i < n; i += 16) {
+      const cplx<double> l = A[i * n + j];
+      for (int c = tc; c < n; c += 16) {
+        if (c <= j) W[i * n + c] = W[i * n + c] - l * W[j * n + c];
+        else if (c <= i) A[i * n + c] = A[i * n + c] - mul_conj(l, A[c * n + j]);
+      }
+    }
+    if (tid == 0) A[j * n + j] = mk<double>(dj * inv, 0.0);
     __syncthreads();
   }
-  if (threadIdx.x == 0) {
+  __syncthreads();
+  if (tid == 0) {
     info[k] = bad;
     if (bad && flag) atomicOr(flag, 2);
   }
   if (bad) return;
-  for (int i = 0; i < n; ++i) {
-    const double dinv = 1.0 / A[i * n + i].x;
-    for (int jc = threadIdx.x; jc < n; jc += blockDim.x) {
-      cplx<double> v;
-      if (jc > i) {
-        v = mk<double>(0.0, 0.0);
-      } else if (jc == i) {
-        v = mk<double>(dinv, 0.0);
-      } else {
-        cplx<double> acc = mk<double>(0.0, 0.0);
-        for (int q = jc; q < i; ++q) acc = acc + A[i * n + q] * Li[q * n + jc];
-        v = scale(acc, -dinv);
-      }
-      Li[i * n + jc] = v;
-    }
-    __syncthreads();
-  }
   cplx<double>* Lo = Linv + k * lk;
   cplx<double>* Gw = G + k * gk;
-  for (int i = threadIdx.x; i < n * n; i += blockDim.x) {
-    Lo[i] = Li[i];
+  for (int i = tid; i < n * n; i += blockDim.x) {
+    Lo[i] = W[i];
     const int r = i / n, c = i % n;
     if (c <= r) Gw[(int64_t)r * ld + c] = A[i];  // the factor in place, as the global version
   }
@@ -307,14 +320,17 @@ __global__ void __launch_bounds__(256) k_row_repair(int npw, int n, cplx<double>
                                                     const unsigned char* __restrict__ mask, double thresh,
                                                     int* __restrict__ flag) {
   __shared__ double red[8];
+  chain_wait();
+  D = after_wait(D);
   const int k = blockIdx.x / n, s = blockIdx.x % n;
   cplx<double>* row = D + k * dk + (int64_t)s * npw;
   double nn = 0.0;
+#pragma unroll 4
   for (int g = threadIdx.x; g < npw; g += blockDim.x) nn += norm2(row[g]);
   nn = block_sum<256>(nn, red);
   if (sqrt(nn) < thresh) {
     const unsigned long long base = ((unsigned long long)k * 4099ull + (unsigned long long)s) * 1000003ull;
-    for (int g = threadIdx.x; g < npw; g += blockDim.x) {
+      for (int g = threadIdx.x; g < npw; g += blockDim.x) {
       const unsigned long long key = (base + (unsigned long long)g) * 2ull;
       row[g] = mask[(int64_t)k * npw + g] ? mk<double>(hash_unit(key), hash_unit(key + 1)) : mk<double>(0.0, 0.0);
     }
@@ -334,26 +350,21 @@ int gwb_residual(int32_t nk, int32_t nb, int32_t npw, const void* x, int64_t x_k
   GWB_REQUIRE(nk >= 0 && nb >= 0 && npw > 0, "bad sizes");
   if (nk == 0 || nb == 0) return GWB_OK;
   GWB_REQUIRE(x && hx && eig && r && rn, "null pointer");
-  k_residual<<<nk * nb, 256, 0, (cudaStream_t)stream>>>(npw, (const cplx<double>*)x, x_kstride,
-                                                       (const cplx<double>*)hx, hx_kstride, eig, eig_kstride,
-                                                       (cplx<double>*)r, r_kstride, rn, nb);
-  GWB_LAUNCH_CHECK();
+  GWB_CUDA_TRY(launch_chained(k_residual, dim3(nk * nb), 256, 0, (cudaStream_t)stream, npw, (const cplx<double>*)x, x_kstride, (const cplx<double>*)hx, hx_kstride, eig, eig_kstride, (cplx<double>*)r, r_kstride, rn, nb));
   count_launches(1);
   return GWB_OK;
 }
 
 int gwb_conv_stats(int32_t nk, int32_t nb, const double* rn, double tol, double* out, void* stream) {
   GWB_REQUIRE(nk > 0 && nb > 0 && rn && out, "bad arguments");
-  k_conv_stats<<<1, 256, 0, (cudaStream_t)stream>>>(rn, nk, nb, tol, out);
-  GWB_LAUNCH_CHECK();
+  GWB_CUDA_TRY(launch_chained(k_conv_stats, dim3(1), 256, 0, (cudaStream_t)stream, rn, nk, nb, tol, out));
   count_launches(1);
   return GWB_OK;
 }
 
 int gwb_select_worst(int32_t nk, int32_t nb, const double* rn, int32_t n_add, int32_t* sel, void* stream) {
   GWB_REQUIRE(nk > 0 && nb > 0 && n_add > 0 && n_add <= nb && rn && sel, "bad arguments");
-  k_select_worst<<<nk, 256, 0, (cudaStream_t)stream>>>(rn, nb, n_add, sel);
-  GWB_LAUNCH_CHECK();
+  GWB_CUDA_TRY(launch_chained(k_select_worst, dim3(nk), 256, 0, (cudaStream_t)stream, rn, nb, n_add, sel));
   count_launches(1);
   return GWB_OK;
 }
@@ -363,10 +374,7 @@ int gwb_precond_teter(int32_t nk, int32_t nb, int32_t n_add, int32_t npw, const 
                       int64_t d_kstride, void* stream) {
   GWB_REQUIRE(nk > 0 && nb > 0 && n_add > 0 && n_add <= nb && npw > 0, "bad sizes");
   GWB_REQUIRE(x && r && t && sel && d, "null pointer");
-  k_precond_teter<<<nk * n_add, 256, 0, (cudaStream_t)stream>>>(npw, nb, n_add, (const cplx<double>*)x, x_kstride,
-                                                               (const cplx<double>*)r, r_kstride, t, sel,
-                                                               (cplx<double>*)d, d_kstride);
-  GWB_LAUNCH_CHECK();
+  GWB_CUDA_TRY(launch_chained(k_precond_teter, dim3(nk * n_add), 256, 0, (cudaStream_t)stream, npw, nb, n_add, (const cplx<double>*)x, x_kstride, (const cplx<double>*)r, r_kstride, t, sel, (cplx<double>*)d, d_kstride));
   count_launches(1);
   return GWB_OK;
 }
@@ -378,9 +386,7 @@ int gwb_subspace_insert(int32_t nk, int32_t m, int32_t m0, const void* C, void* 
   const int64_t total = (int64_t)m * (m - m0);
   const int blocks = (int)std::min<int64_t>((total + 255) / 256, 1024);
   dim3 grid(blocks, nk);
-  k_subspace_insert<<<grid, 256, 0, (cudaStream_t)stream>>>((const cplx<double>*)C, m, m0, (cplx<double>*)S, lds,
-                                                           s_kstride);
-  GWB_LAUNCH_CHECK();
+  GWB_CUDA_TRY(launch_chained(k_subspace_insert, grid, 256, 0, (cudaStream_t)stream, (const cplx<double>*)C, m, m0, (cplx<double>*)S, lds, s_kstride));
   count_launches(1);
   return GWB_OK;
 }
@@ -392,8 +398,8 @@ int gwb_chol_inv(int32_t nk, int32_t n, void* G, int32_t ldg, int64_t g_kstride,
   if (n <= CHOL_SMEM_MAX) {
     const size_t sm = (size_t)2 * n * n * sizeof(cplx<double>);
     GWB_CUDA_TRY(allow_smem(k_chol_inv_smem));
-    k_chol_inv_smem<<<nk, 256, sm, (cudaStream_t)stream>>>((cplx<double>*)G, n, ldg, g_kstride,
-                                                          (cplx<double>*)Linv, linv_kstride, info, flag);
+    GWB_CUDA_TRY(launch_chained(k_chol_inv_smem, dim3(nk), 256, sm, (cudaStream_t)stream, (cplx<double>*)G, n, ldg,
+                                g_kstride, (cplx<double>*)Linv, linv_kstride, info, flag));
   } else {
     k_chol_inv<<<nk, 256, 0, (cudaStream_t)stream>>>((cplx<double>*)G, n, ldg, g_kstride, (cplx<double>*)Linv,
                                                     linv_kstride, info, flag);
@@ -407,8 +413,7 @@ int gwb_row_repair(int32_t nk, int32_t n, int32_t npw, void* D, int64_t d_kstrid
                    double thresh, int32_t* flag, void* stream) {
   GWB_REQUIRE(nk > 0 && n > 0 && npw > 0, "bad sizes");
   GWB_REQUIRE(D && mask && flag, "null pointer");
-  k_row_repair<<<nk * n, 256, 0, (cudaStream_t)stream>>>(npw, n, (cplx<double>*)D, d_kstride, mask, thresh, flag);
-  GWB_LAUNCH_CHECK();
+  GWB_CUDA_TRY(launch_chained(k_row_repair, dim3(nk * n), 256, 0, (cudaStream_t)stream, npw, n, (cplx<double>*)D, d_kstride, mask, thresh, flag));
   count_launches(1);
   return GWB_OK;
 }

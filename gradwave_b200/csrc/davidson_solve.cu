@@ -209,12 +209,11 @@ class Solver {
     // initial block: masked copy, orthonormalised with host-checked CholQR2
     GWB_TRY(masked_copy(static_cast<const Z16*>(x0), nbp, w_.D, nbp, nb_));
     int ok = 0;
-    GWB_TRY(cholqr2(w_.D, nbp, nb_, w_.D2, nullptr, nullptr, /*sync=*/true, &ok));
+    GWB_TRY(cholqr2(w_.D, nbp, nb_, w_.D2, w_.V, mdp, nullptr, nullptr, /*sync=*/true, &ok));
     if (!ok) {
       set_error("initial block is rank deficient (Cholesky breakdown)");
       return GWB_ERR_BREAKDOWN;
     }
-    GWB_TRY(copy_rows(w_.V, mdp, w_.D, nbp, nb_));
     GWB_TRY(apply(w_.V, mdp, w_.HV, mdp, nb_, fp32_exp_));
     int m = nb_, m0 = 0, m_prev = nb_;
     const double eps32 = 1.1920928955078125e-07;
@@ -276,7 +275,7 @@ class Solver {
       GWB_TRY(precondition(n_add, eig));
       if (m + n_add > md_) {
         ++n_restart_;
-        GWB_TRY(cholqr2(w_.X, nbp, nb_, w_.D2, w_.HX, w_.R, /*sync=*/true, &ok));
+        GWB_TRY(cholqr2(w_.X, nbp, nb_, w_.D2, w_.X, nbp, w_.HX, w_.R, /*sync=*/true, &ok));
         if (!ok) {
           set_error("Ritz block lost rank at restart");
           return GWB_ERR_BREAKDOWN;
@@ -287,7 +286,6 @@ class Solver {
         m0 = 0;
       }
       GWB_TRY(orthonormalize_new(n_add, m));
-      GWB_TRY(copy_rows(w_.V + (int64_t)m * npw_, mdp, w_.D, nbp, n_add));
       GWB_TRY(apply(w_.V + (int64_t)m * npw_, mdp, w_.HV + (int64_t)m * npw_, mdp, n_add, fp32_exp_));
       m_prev = m;
       m += n_add;
@@ -462,14 +460,18 @@ class Solver {
     return gwb_precond_teter(nk_, nb_, n_add, npw_, w_.X, nbp, w_.R, nbp, t_, w_.sel, w_.D, nbp, st_);
   }
 
-  // Two rounds of Gram -> Cholesky -> L^-1 on n rows of Y (k stride ys); the
-  // companion Z (if any) gets the same transform. sync: check breakdown on the
-  // host (ok = 0 on failure); else breakdown only raises bit 1 of flags.
-  int cholqr2(Z16* Y, int64_t ys, int n, Z16* Ytmp, Z16* Z, Z16* Ztmp, bool sync, int* ok) {
-    const int64_t nn = (int64_t)n * n;
+  // Two rounds of Gram -> Cholesky -> L^-1 on n rows of Y (k stride ys): the
+  // first into Ytmp, the second into out (k stride os; Y itself or elsewhere).
+  // The companion Z (if any; k stride ys, result in place) gets the same
+  // transform. sync: check breakdown on the host (ok = 0 on failure); else
+  // breakdown only raises bit 1 of flags.
+  int cholqr2(Z16* Y, int64_t ys, int n, Z16* Ytmp, Z16* out, int64_t os, Z16* Z, Z16* Ztmp, bool sync, int* ok) {
+    const int64_t nn = (int64_t)n * n, ts = (int64_t)nb_ * npw_;
     *ok = 1;
     for (int pass = 0; pass < 2; ++pass) {
-      GWB_TRY(zgemm(0, 2, n, n, npw_, Y, npw_, ys, Y, npw_, ys, w_.G, n, nn));
+      const Z16* src = pass ? Ytmp : Y;
+      const int64_t ss = pass ? ts : ys;
+      GWB_TRY(zgemm(0, 2, n, n, npw_, src, npw_, ss, src, npw_, ss, w_.G, n, nn));
       if (sync) GWB_CUDA_TRY(cudaMemsetAsync(w_.sync_flag, 0, sizeof(int), st_));
       GWB_TRY(gwb_chol_inv(nk_, n, w_.G, n, nn, w_.Linv, nn, w_.info, sync ? w_.sync_flag : w_.flags, st_));
       if (sync) {
@@ -482,12 +484,10 @@ class Solver {
           return GWB_OK;
         }
       }
-      GWB_TRY(zgemm(0, 0, n, npw_, n, w_.Linv, n, nn, Y, npw_, ys, Ytmp, npw_, (int64_t)nb_ * npw_));
-      GWB_TRY(copy_rows(Y, ys, Ytmp, (int64_t)nb_ * npw_, n));
-      if (Z) {
-        GWB_TRY(zgemm(0, 0, n, npw_, n, w_.Linv, n, nn, Z, npw_, ys, Ztmp, npw_, (int64_t)nb_ * npw_));
-        GWB_TRY(copy_rows(Z, ys, Ztmp, (int64_t)nb_ * npw_, n));
-      }
+      GWB_TRY(zgemm(0, 0, n, npw_, n, w_.Linv, n, nn, src, npw_, ss, pass ? out : Ytmp, npw_, pass ? os : ts));
+      if (Z)
+        GWB_TRY(zgemm(0, 0, n, npw_, n, w_.Linv, n, nn, pass ? Ztmp : Z, npw_, pass ? ts : ys, pass ? Z : Ztmp, npw_,
+                      pass ? ys : ts));
     }
     return GWB_OK;
   }
@@ -505,7 +505,7 @@ class Solver {
     GWB_TRY(gwb_row_repair(nk_, n, npw_, w_.D, nbp, mask_, repair_thresh_, w_.flags, st_));
     if (m) GWB_TRY(project_out(w_.D, nbp, n, m));
     int ok = 1;
-    return cholqr2(w_.D, nbp, n, w_.D2, nullptr, nullptr, false, &ok);
+    return cholqr2(w_.D, nbp, n, w_.D2, w_.V + (int64_t)m * npw_, (int64_t)md_ * npw_, nullptr, nullptr, false, &ok);
   }
 
   gwb_ham* h_;

@@ -101,7 +101,101 @@ __global__ void __launch_bounds__(ZN_TN * 4) k_zmma_nn(int nb, int N, int K, con
   }
 }
 
+// The same tiles for the solver's short products (triangular transforms,
+// projections, Ritz vectors: few rows, long rows of B).
+template <int TM, bool TA>
+__global__ void __launch_bounds__(ZN_TN * 4) k_zmma_ab(int M, int N, int K, cplx<double> alpha,
+                                                       const cplx<double>* __restrict__ A, int64_t lda, int64_t sA,
+                                                       const cplx<double>* __restrict__ B, int64_t ldb, int64_t sB,
+                                                       cplx<double> beta, cplx<double>* C, int64_t ldc, int64_t sC) {
+  constexpr int NT = ZN_TN * 4, MT = TM / 8, STAGE = TM * ZM_PK + ZM_K * ZN_PN;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  cplx<double>* sm = reinterpret_cast<cplx<double>*>(smem_raw);
+  const int n0 = blockIdx.x * ZN_TN, i0 = blockIdx.y * TM;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const cplx<double>* Ab = A + blockIdx.z * sA;
+  const cplx<double>* Bb = B + blockIdx.z * sB;
+  cplx<double>* Cb = C + blockIdx.z * sC;
+  const int nsteps = (K + ZM_K - 1) / ZM_K;
+
+  auto load = [&](int step) {
+    if (step < nsteps) {
+      const int q0 = step * ZM_K;
+      cplx<double>* st = sm + (size_t)(step % ZM_STAGES) * STAGE;
+#pragma unroll
+      for (int idx = tid; idx < TM * ZM_K; idx += NT) {
+        const int r = TA ? idx % TM : idx / ZM_K, qq = TA ? idx / TM : idx % ZM_K, i = i0 + r, q = q0 + qq;
+        const bool ok = i < M && q < K;
+        const cplx<double>* src = TA ? Ab + (int64_t)q * lda + i : Ab + (int64_t)i * lda + q;
+        cp_async16(st + r * ZM_PK + qq, ok ? src : Ab, ok);
+      }
+#pragma unroll
+      for (int idx = tid; idx < ZM_K * ZN_TN; idx += NT) {
+        const int qq = idx / ZN_TN, nn = idx % ZN_TN, q = q0 + qq, n = n0 + nn;
+        const bool ok = q < K && n < N;
+        cp_async16(st + TM * ZM_PK + qq * ZN_PN + nn, ok ? Bb + (int64_t)q * ldb + n : Bb, ok);
+      }
+    }
+    cp_async_commit();
+  };
+  chain_wait();
+#pragma unroll
+  for (int p = 0; p < ZM_STAGES - 1; ++p) load(p);
+  double re[MT][2], im[MT][2];
+#pragma unroll
+  for (int t = 0; t < MT; ++t) re[t][0] = re[t][1] = im[t][0] = im[t][1] = 0.0;
+  for (int step = 0; step < nsteps; ++step) {
+    cp_async_wait<ZM_STAGES - 2>();
+    __syncthreads();
+    load(step + ZM_STAGES - 1);
+    const cplx<double>* st = sm + (size_t)(step % ZM_STAGES) * STAGE;
+    const cplx<double>* sa = st + (lane >> 2) * ZM_PK + (lane & 3);
+    const cplx<double>* sb = st + TM * ZM_PK + (lane & 3) * ZN_PN + w * 8 + (lane >> 2);
+#pragma unroll
+    for (int kk = 0; kk < ZM_K; kk += 4) {
+      const cplx<double> bv = sb[kk * ZN_PN];
+#pragma unroll
+      for (int t = 0; t < MT; ++t) {
+        const cplx<double> av = sa[t * 8 * ZM_PK + kk];
+        dmma(re[t], av.x, bv.x);
+        dmma(im[t], av.y, bv.x);
+        dmma(re[t], -av.y, bv.y);
+        dmma(im[t], av.x, bv.y);
+      }
+    }
+  }
+  cp_async_wait<0>();
+  const int n = n0 + w * 8 + 2 * (lane & 3);
+  const bool add = beta.x != 0.0 || beta.y != 0.0;
+#pragma unroll
+  for (int t = 0; t < MT; ++t) {
+    const int i = i0 + t * 8 + (lane >> 2);
+    if (i >= M) continue;
+    cplx<double>* dst = Cb + (int64_t)i * ldc;
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+      if (n + e < N) {
+        const cplx<double> v = alpha * mk<double>(re[t][e], im[t][e]);
+        dst[n + e] = add ? v + beta * dst[n + e] : v;
+      }
+  }
+}
+
 }  // namespace
+
+cudaError_t zmma_ab(bool TA, int M, int N, int K, cplx<double> alpha, const cplx<double>* A, int64_t lda, int64_t sA,
+                    const cplx<double>* B, int64_t ldb, int64_t sB, cplx<double> beta, cplx<double>* C, int64_t ldc,
+                    int64_t sC, int batch, cudaStream_t st) {
+  const int TM = zmma_edge(M, 32);
+  const dim3 grid((unsigned)((N + ZN_TN - 1) / ZN_TN), (unsigned)((M + TM - 1) / TM), batch);
+#define GWB_ZA_CASE(tm)                                                                                          \
+  if (TM == tm)                                                                                                  \
+    return launch_chained(TA ? k_zmma_ab<tm, true> : k_zmma_ab<tm, false>, grid, ZN_TN * 4, zmma_nn_smem<tm>(), st, M, \
+                          N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC);
+  GWB_ZA_CASE(8) GWB_ZA_CASE(16) GWB_ZA_CASE(24) GWB_ZA_CASE(32)
+#undef GWB_ZA_CASE
+  return cudaErrorInvalidValue;
+}
 
 int zmma_nh_slices(int M, int N, int K, int batch, int64_t cap, int target_blocks, int* kslice) {
   const int TM = zmma_edge(M, 32), TN = zmma_edge(N, 64);

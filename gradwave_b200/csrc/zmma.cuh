@@ -163,4 +163,10 @@ cudaError_t zmma_nn(int nb, int N, int K, const cplx<double>* A, const cplx<doub
                     const cplx<double>* c, int64_t ck, cplx<double>* out_h, int64_t hk, cplx<double>* out_s, int64_t sk,
                     const int* npw_k, int batch, cudaStream_t st);
 
+// C = alpha op(A) B + beta C with few rows: op(A) (M x K; TA: A is K x M), B (K x N),
+// C (M x N), row-major, batched by strides. C is not read where beta = 0.
+cudaError_t zmma_ab(bool TA, int M, int N, int K, cplx<double> alpha, const cplx<double>* A, int64_t lda, int64_t sA,
+                    const cplx<double>* B, int64_t ldb, int64_t sB, cplx<double> beta, cplx<double>* C, int64_t ldc,
+                    int64_t sC, int batch, cudaStream_t st);
+
 }  // namespace gwb
