@@ -512,7 +512,7 @@ static int chunk_scratch(gwb_ham* h, int nb, size_t es, int* nbc) {
     return rc;
   };
   auto bands = [&](size_t budget) {
-    const size_t most = std::max<size_t>(1, budget / per_band);
+    const size_t most = std::min<size_t>(32768, std::max<size_t>(1, budget / per_band));  // bands are a grid axis
     const size_t nchunks = ((size_t)nb + most - 1) / most;
     return (int)(((size_t)nb + nchunks - 1) / nchunks);
   };

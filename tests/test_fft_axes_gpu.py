@@ -118,3 +118,15 @@ def test_slots_of_one_box_cell(cuda_device):
     assert float((out[0] - ref).abs().max()) < 1e-13
     torch.cuda.synchronize()
     _lib.load().gwb_ham_destroy(h)
+
+
+def test_scratch_of_a_destroyed_handle(cuda_device):
+    """A handle that takes over another's scratch (larger, then smaller than it needs) gives the same result."""
+    points = {n: np.random.default_rng(n).choice(n ** 3, n * n, replace=False) for n in (12, 20)}
+    keep = _handle([4, 4, 4], np.zeros((1, 1)), 1, 1, [1], torch.zeros(4, 4, 4, dtype=torch.float64, device=cuda_device),
+                   torch.zeros(1, 1, dtype=torch.float64, device=cuda_device))
+    for n in (20, 12, 20, 12):
+        _check([n] * 3, points[n], cuda_device, n)
+    from gradwave_b200 import _lib
+    torch.cuda.synchronize()
+    _lib.load().gwb_ham_destroy(keep)

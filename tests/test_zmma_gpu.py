@@ -58,3 +58,45 @@ def test_nonlocal_of_both_outputs(nproj, nb, cuda_device):
     for got, ref in ((h, ref_h), (s, ref_s)):
         assert float((got - ref).norm() / ref.norm()) < 1e-14
         assert not got[1, :, 60:].any()
+
+
+@pytest.mark.parametrize("op", [0, 1])
+@pytest.mark.parametrize("M,N,K,batch", [(1, 8, 1, 1), (7, 63, 9, 2), (8, 64, 8, 3), (24, 193, 72, 2), (33, 1001, 17, 1),
+                                         (64, 513, 64, 2), (65, 600, 5, 1)])
+def test_short_row_products(op, M, N, K, batch, cuda_device):
+    """C = alpha op(A) B + beta C of up to 64 rows (65: the library's) with strides wider than the matrices; C is
+    not read where beta = 0. Bound as above."""
+    from gradwave_b200 import _lib
+    A = _rand(batch, M, K + 2, seed=1) if op == 0 else _rand(batch, K, M + 2, seed=1)
+    a = A[:, :, :K] if op == 0 else A[:, :, :M].mT
+    B, C0 = _rand(batch, K + 1, N + 3, seed=2), _rand(batch, M, N + 1, seed=3)
+    for alpha, beta in ((1.0, 0.0), (-1.0, 1.0), (0.5 - 2j, 0.25j)):
+        C = C0.clone() if beta != 0.0 else torch.full_like(C0, float("nan"))
+        alpha, beta = complex(alpha), complex(beta)
+        _lib.call("gwb_zgemm", op, 0, M, N, K, alpha.real, alpha.imag, A.data_ptr(), A.shape[2], A.shape[1] * A.shape[2],
+                  B.data_ptr(), N + 3, (K + 1) * (N + 3), beta.real, beta.imag, C.data_ptr(), N + 1, M * (N + 1), batch,
+                  _lib.stream_ptr())
+        ref = alpha * (a @ B[:, :K, :N]) + (beta * C0[:, :, :N] if beta != 0.0 else 0.0)
+        bound = (K + 2) * 2.3e-16 * abs(alpha) * 2.2 * (a.abs() @ B[:, :K, :N].abs()) + 1e-15 * (1 + abs(beta) * C0[:, :, :N].abs())
+        assert bool(((C[:, :, :N] - ref).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("n", [1, 2, 15, 16, 17, 33, 63, 64])
+def test_cholesky_and_inverse(n, cuda_device):
+    """L L^H = G and L^-1 L = 1 for two matrices (n eps cond: the random Gram matrices have cond below 1e4), the
+    third one indefinite: its pivot is reported, the others unaffected."""
+    from gradwave_b200 import _lib
+    X = _rand(3, n, 4 * n + 4, seed=n)
+    G = X @ X.mH
+    G[2, n - 1, n - 1] = -1.0
+    F, Li = G.clone(), torch.full((3, n, n), 7.0, dtype=torch.complex128, device=cuda_device)
+    info, flag = torch.zeros(3, dtype=torch.int32, device=cuda_device), torch.zeros(1, dtype=torch.int32, device=cuda_device)
+    _lib.call("gwb_chol_inv", 3, n, F.data_ptr(), n, n * n, Li.data_ptr(), n * n, info.data_ptr(), flag.data_ptr(),
+              _lib.stream_ptr())
+    assert info.tolist() == [0, 0, n] and int(flag) == 2
+    L = torch.tril(F[:2])
+    eye = torch.eye(n, dtype=torch.complex128, device=cuda_device)
+    assert float((L @ L.mH - G[:2]).norm() / G[:2].norm()) < n * 2.3e-16 * 4
+    assert float((Li[:2] @ L - eye).abs().max()) < n * 2.3e-16 * 1e4
+    assert not torch.triu(Li[:2], 1).any()
+    assert bool((Li[2] == 7.0).all())
