@@ -394,6 +394,7 @@ __global__ void __launch_bounds__(256) k_precond_row_stats(int npw, int nb, int 
   const cplx<double>* rr = r + k * rk + (int64_t)b * npw;
   const double* tk = t_ + (int64_t)k * npw;
   double tb = 0.0, r2 = 0.0;
+#pragma unroll 8
   for (int gi = threadIdx.x; gi < npw; gi += blockDim.x) {
     tb += tk[gi] * norm2(xr[gi]);
     r2 += norm2(rr[gi]);
@@ -551,16 +552,39 @@ __global__ void __launch_bounds__(PL_THREADS) k_precond_learned_tc(
   }
 }
 
-// d row <- d row / |d row|, the norm summed from the chunk partials in order.
-__global__ void k_precond_normalize(int npw, int n_add, int chunks, const double* __restrict__ partial,
-                                    cplx<double>* __restrict__ d, int64_t dk) {
-  const int row = blockIdx.x, k = row / n_add, s = row % n_add;
+// Sum of n partials in order, by every thread of the block: loaded side by side
+// into shared memory, added one after another from there (each thread walking
+// them in global memory cost 20 us of L2 latency per block at 290 partials).
+__device__ __forceinline__ double ordered_sum(const double* __restrict__ partial, int n) {
+  __shared__ double buf[256];
   double a = 0.0;
-  for (int c = 0; c < chunks; ++c) a += partial[(int64_t)row * chunks + c];
+  for (int c0 = 0; c0 < n; c0 += 256) {
+    const int m = min(256, n - c0);
+    __syncthreads();
+    if ((int)threadIdx.x < m) buf[threadIdx.x] = partial[c0 + threadIdx.x];
+    __syncthreads();
+    for (int c = 0; c < m; ++c) a += buf[c];
+  }
+  return a;
+}
+
+// Blocks per row of the scaling kernels: about eight per SM over all rows (a
+// block per row streamed at half of the bandwidth).
+inline unsigned normalize_splits(int rows) { return (unsigned)std::max(1, std::min(16, 8 * 148 / std::max(1, rows))); }
+
+// d row <- d row / |d row|, the norm summed from the chunk partials in order;
+// block y of a row takes every gridDim.y-th stretch of it.
+__global__ void __launch_bounds__(256) k_precond_normalize(int npw, int n_add, int chunks,
+                                                           const double* __restrict__ partial,
+                                                           cplx<double>* __restrict__ d, int64_t dk) {
+  const int row = blockIdx.x, k = row / n_add, s = row % n_add;
+  const double a = ordered_sum(partial + (int64_t)row * chunks, chunks);
   if (!(a > 0.0)) return;
   const double inv = 1.0 / sqrt(a);
   cplx<double>* dr = d + k * dk + (int64_t)s * npw;
-  for (int gi = threadIdx.x; gi < npw; gi += blockDim.x) dr[gi] = scale(dr[gi], inv);
+#pragma unroll 4
+  for (int gi = blockIdx.y * blockDim.x + threadIdx.x; gi < npw; gi += gridDim.y * blockDim.x)
+    dr[gi] = scale(dr[gi], inv);
 }
 
 // ---------------------------------------------------------------------------
@@ -926,15 +950,17 @@ __global__ void __launch_bounds__(256) k_precond_row_stats_gamma(int nhalf, int 
 
 // Embedded rows: d <- d / |d| over the 2 nhalf - 1 coordinates, the norm
 // summed from the tile partials in order; pad columns set to zero.
-__global__ void k_precond_normalize_gamma(int nhalf, int npad, int tiles, const double* __restrict__ partial,
-                                          double* __restrict__ d, int64_t d_row) {
+__global__ void __launch_bounds__(256) k_precond_normalize_gamma(int nhalf, int npad, int tiles,
+                                                                 const double* __restrict__ partial,
+                                                                 double* __restrict__ d, int64_t d_row) {
   const int s = blockIdx.x;
-  double a = 0.0;
-  for (int c = 0; c < tiles; ++c) a += partial[(int64_t)s * tiles + c];
+  const double a = ordered_sum(partial + (int64_t)s * tiles, tiles);
   const double inv = a > 0.0 ? 1.0 / sqrt(a) : 1.0;
   double* dr = d + (int64_t)s * d_row;
   const int nphi = 2 * nhalf - 1;
-  for (int i = threadIdx.x; i < npad; i += blockDim.x) dr[i] = i < nphi ? dr[i] * inv : 0.0;
+#pragma unroll 4
+  for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < npad; i += gridDim.y * blockDim.x)
+    dr[i] = i < nphi ? dr[i] * inv : 0.0;
 }
 
 // Stall rule of the learned preconditioner: a band whose residual has not
@@ -1099,14 +1125,14 @@ int gwb_precond_learned(const float* params, int32_t nk, int32_t nb, int32_t n_a
     k_precond_learned_tc<<<dim3(chunks, rows), PL_THREADS, 0, st>>>(params, npw, nb, n_add, (const cplx<double>*)r,
                                                                     r_kstride, t, eig, sel, tpa_only, stats,
                                                                     (cplx<double>*)d, d_kstride, partial);
-    k_precond_normalize<<<rows, 256, 0, st>>>(npw, n_add, chunks, partial, (cplx<double>*)d, d_kstride);
+    k_precond_normalize<<<dim3(rows, normalize_splits(rows)), 256, 0, st>>>(npw, n_add, chunks, partial, (cplx<double>*)d, d_kstride);
   } else {
     const int64_t tiles = (npw + PU_TILE - 1) / PU_TILE;
     int* status = reinterpret_cast<int*>(partial + (int64_t)rows * tiles);
     int rc = precond_umma<false>(params, nb, n_add, npw, r, r_kstride, 0, t, eig, sel, tpa_only, stats, d, d_kstride,
                                  0, partial, rows, status, st);
     if (rc) return rc;
-    k_precond_normalize<<<rows, 256, 0, st>>>(npw, n_add, (int)tiles, partial, (cplx<double>*)d, d_kstride);
+    k_precond_normalize<<<dim3(rows, normalize_splits(rows)), 256, 0, st>>>(npw, n_add, (int)tiles, partial, (cplx<double>*)d, d_kstride);
   }
   GWB_LAUNCH_CHECK();
   count_launches(3);
@@ -1137,7 +1163,7 @@ int gwb_precond_learned_gamma(const float* params, int32_t nb, int32_t n_add, in
   int rc = precond_umma<true>(params, nb, n_add, nhalf, r, 0, r_row, t_half, eig, sel, tpa_only, stats, d, 0, d_row,
                               partial, n_add, status, st);
   if (rc) return rc;
-  k_precond_normalize_gamma<<<n_add, 256, 0, st>>>(nhalf, npad, tiles, partial, d, d_row);
+  k_precond_normalize_gamma<<<dim3(n_add, normalize_splits(n_add)), 256, 0, st>>>(nhalf, npad, tiles, partial, d, d_row);
   GWB_LAUNCH_CHECK();
   count_launches(3);
   return GWB_OK;
