@@ -108,9 +108,9 @@ static bool axis_ok(int n) {
   return n == 1;
 }
 
-// Scratch of one band chunk. Measured on the FFT launches of a float64 96^3
-// apply of 240 rows: 8.9 ms at 48 MB (L2 sized), 8.4 at 96, 7.9 at 400, 7.7 at
-// 1200 (launch ramps and last waves weigh more than L2 misses).
+// Scratch of one band chunk. A float64 96^3 Gamma apply of 240 rows takes 8.2 ms
+// at 48 MB (L2 sized), 8.0 at 96 to 192, 7.7 at 512, 7.5 at 1024: launch ramps and
+// last waves weigh more than L2 misses, and past 512 MB little is left.
 constexpr long kWBudgetMB = 512, kWBudgetLowMB = 48;
 
 static size_t w_budget_bytes() {

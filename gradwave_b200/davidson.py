@@ -18,7 +18,8 @@ buffer), the subspace matrix is updated incrementally (only the new columns
 are formed, ``gwb_subspace_insert``), and orthonormalisation is CholQR2
 (float64 Gram, Cholesky, triangular inverse; the reference's own optional
 path, ``solvers/davidson.py:195-222``) with the reference's jitter + QR
-fallback on breakdown.
+fallback on breakdown. A cold start of a large basis gets seeded noise on its
+first expansion rows (``_Solver.break_symmetry``).
 
 Modes:
   ``mode="fp64"``     every apply in float64 (plain TPA Davidson).
