@@ -19,7 +19,7 @@ template <int TM> constexpr size_t zmma_nn_smem() {
   return (size_t)ZM_STAGES * (TM * ZM_PK + ZM_K * ZN_PN) * 16;
 }
 
-template <int TM, bool HS>
+template <int TM, bool HS, int CHAIN>
 __global__ void __launch_bounds__(ZN_TN * 4) k_zmma_nn(int nb, int N, int K, const cplx<double>* __restrict__ A,
                                                        const cplx<double>* __restrict__ A2,
                                                        const cplx<double>* __restrict__ P,
@@ -63,9 +63,7 @@ __global__ void __launch_bounds__(ZN_TN * 4) k_zmma_nn(int nb, int N, int K, con
   for (int p = 0; p < ZM_STAGES - 1; ++p) load(p);
 
   const int n = n0 + w * 8 + 2 * (lane & 3);
-  double re[MT][2], im[MT][2];
-#pragma unroll
-  for (int t = 0; t < MT; ++t) re[t][0] = re[t][1] = im[t][0] = im[t][1] = 0.0;
+  ZmmaSums<MT, CHAIN> sum;
   for (int step = 0; step < nsteps; ++step) {
     cp_async_wait<ZM_STAGES - 2>();
     __syncthreads();
@@ -73,18 +71,8 @@ __global__ void __launch_bounds__(ZN_TN * 4) k_zmma_nn(int nb, int N, int K, con
     const cplx<double>* st = sm + (size_t)(step % ZM_STAGES) * STAGE;
     const cplx<double>* sa = st + (lane >> 2) * ZM_PK + (lane & 3);
     const cplx<double>* sp = st + TM * ZM_PK + (lane & 3) * ZN_PN + w * 8 + (lane >> 2);
-#pragma unroll
-    for (int kk = 0; kk < ZM_K; kk += 4) {
-      const cplx<double> pv = sp[kk * ZN_PN];
-#pragma unroll
-      for (int t = 0; t < MT; ++t) {
-        const cplx<double> av = sa[t * 8 * ZM_PK + kk];
-        dmma(re[t], av.x, pv.x);
-        dmma(im[t], av.y, pv.x);
-        dmma(re[t], -av.y, pv.y);
-        dmma(im[t], av.x, pv.y);
-      }
-    }
+    sum.template add<false>(step, nsteps, [&](int t, int kk) { return sa[t * 8 * ZM_PK + kk]; },
+                            [&](int kk) { return sp[kk * ZN_PN]; });
   }
   cp_async_wait<0>();
 #pragma unroll
@@ -97,7 +85,7 @@ __global__ void __launch_bounds__(ZN_TN * 4) k_zmma_nn(int nb, int N, int K, con
 #pragma unroll
     for (int e = 0; e < 2; ++e)
       if (n + e < N)
-        dst[n + e] = sr && n + e >= npw ? mk<double>(0.0, 0.0) : src[n + e] + mk<double>(re[t][e], im[t][e]);
+        dst[n + e] = sr && n + e >= npw ? mk<double>(0.0, 0.0) : src[n + e] + sum.at(t, e);
   }
 }
 
@@ -141,9 +129,7 @@ __global__ void __launch_bounds__(ZN_TN * 4) k_zmma_ab(int M, int N, int K, cplx
   chain_wait();
 #pragma unroll
   for (int p = 0; p < ZM_STAGES - 1; ++p) load(p);
-  double re[MT][2], im[MT][2];
-#pragma unroll
-  for (int t = 0; t < MT; ++t) re[t][0] = re[t][1] = im[t][0] = im[t][1] = 0.0;
+  ZmmaSums<MT, 1> sum;
   for (int step = 0; step < nsteps; ++step) {
     cp_async_wait<ZM_STAGES - 2>();
     __syncthreads();
@@ -151,18 +137,8 @@ __global__ void __launch_bounds__(ZN_TN * 4) k_zmma_ab(int M, int N, int K, cplx
     const cplx<double>* st = sm + (size_t)(step % ZM_STAGES) * STAGE;
     const cplx<double>* sa = st + (lane >> 2) * ZM_PK + (lane & 3);
     const cplx<double>* sb = st + TM * ZM_PK + (lane & 3) * ZN_PN + w * 8 + (lane >> 2);
-#pragma unroll
-    for (int kk = 0; kk < ZM_K; kk += 4) {
-      const cplx<double> bv = sb[kk * ZN_PN];
-#pragma unroll
-      for (int t = 0; t < MT; ++t) {
-        const cplx<double> av = sa[t * 8 * ZM_PK + kk];
-        dmma(re[t], av.x, bv.x);
-        dmma(im[t], av.y, bv.x);
-        dmma(re[t], -av.y, bv.y);
-        dmma(im[t], av.x, bv.y);
-      }
-    }
+    sum.template add<false>(step, nsteps, [&](int t, int kk) { return sa[t * 8 * ZM_PK + kk]; },
+                            [&](int kk) { return sb[kk * ZN_PN]; });
   }
   cp_async_wait<0>();
   const int n = n0 + w * 8 + 2 * (lane & 3);
@@ -175,7 +151,7 @@ __global__ void __launch_bounds__(ZN_TN * 4) k_zmma_ab(int M, int N, int K, cplx
 #pragma unroll
     for (int e = 0; e < 2; ++e)
       if (n + e < N) {
-        const cplx<double> v = alpha * mk<double>(re[t][e], im[t][e]);
+        const cplx<double> v = alpha * sum.at(t, e);
         dst[n + e] = add ? v + beta * dst[n + e] : v;
       }
   }
@@ -234,11 +210,15 @@ cudaError_t zmma_nn(int nb, int N, int K, const cplx<double>* A, const cplx<doub
                     const int* npw_k, int batch, cudaStream_t st) {
   const int rows = A2 ? 2 * nb : nb;
   const int TM = zmma_edge(rows, 32);
+  const bool uncut = K <= ZM_UNCUT;
   const dim3 grid((unsigned)((N + ZN_TN - 1) / ZN_TN), (unsigned)((rows + TM - 1) / TM), batch);
 #define GWB_ZN_CASE(tm)                                                                                            \
-  if (TM == tm)                                                                                                    \
-    return launch_chained(A2 ? k_zmma_nn<tm, true> : k_zmma_nn<tm, false>, grid, ZN_TN * 4, zmma_nn_smem<tm>(), st, \
-                          nb, N, K, A, A2, P, c, ck, out_h, hk, out_s, sk, npw_k);
+  if (TM == tm) {                                                                                                  \
+    auto* kern = A2 ? (uncut ? k_zmma_nn<tm, true, 0> : k_zmma_nn<tm, true, ZM_CHAIN>)                             \
+                    : (uncut ? k_zmma_nn<tm, false, 0> : k_zmma_nn<tm, false, ZM_CHAIN>);                          \
+    return launch_chained(kern, grid, ZN_TN * 4, zmma_nn_smem<tm>(), st, nb, N, K, A, A2, P, c, ck, out_h, hk,     \
+                          out_s, sk, npw_k);                                                                       \
+  }
   GWB_ZN_CASE(8) GWB_ZN_CASE(16) GWB_ZN_CASE(24) GWB_ZN_CASE(32)
 #undef GWB_ZN_CASE
   return cudaErrorInvalidValue;

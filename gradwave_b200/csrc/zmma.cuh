@@ -15,11 +15,19 @@
 // instructions, which held these products at 10-14 TFLOP/s of the 37 the chip
 // has in float64. A warp owns one 8-column tile and all TM rows of the block,
 // so each B fragment is loaded once and there are 2 TM / 8 independent
-// accumulation chains. The tensor instruction rounds after every FMA, twice per
-// complex term where a product rounded first costs one addition, so chains are
-// cut every 128 terms and the update is summed apart from the row it is added
-// to: the result is no further from exact than on the FMA pipe. Operands arrive by cp.async in 8-wide K steps, three
+// accumulation chains. Operands arrive by cp.async in 8-wide K steps, three
 // stages deep.
+//
+// The tensor instruction rounds after every FMA, twice per complex term where a
+// product rounded first costs one addition, so a chain of K terms from zero errs
+// by sqrt(K) roundings of its sum. Chains are cut (and the sum taken over them)
+// so that no product is further from exact than on the FMA pipe or in cuBLAS:
+// after one K step in k_zmma_ab (24 x 256 x 96: 4.7e-16 uncut, 1.8e-16, cuBLAS
+// 1.9e-16; 64 x 512 x 640: 12, 3.3, 6.0), after ZM_CHAIN in k_zmma_nh (24 x 24 x
+// 100: 4.8e-16 with chains of 128 terms, 2.8e-16, FMA pipe 3.5e-16). The update is
+// summed apart from the row it is added to, uncut up to ZM_UNCUT projectors (256:
+// 8.3e-16, FMA pipe 9.2e-16; 864: 14 uncut, 4.4, 12); beyond, the second set of
+// sums costs registers and a block per SM (5 % of a 64-atom apply at 256).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -43,7 +51,47 @@ __device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
 
 constexpr int ZM_K = 8;       // K step
 constexpr int ZM_STAGES = 3;  // steps in flight
-constexpr int ZM_FLUSH = 16;  // steps summed in one chain before they join the slice's sum
+constexpr int ZM_CHAIN = 4;   // steps in one chain of the long products
+constexpr int ZM_UNCUT = 256;  // longest update summed in one chain
+
+// Sums of a warp's 8 MT x 8 tile in chains of CHAIN steps (0: one chain): lane l
+// holds rows 8 t + l / 4, columns 2 (l % 4) + {0, 1}.
+template <int MT, int CHAIN> struct ZmmaSums {
+  static constexpr int MS = CHAIN ? MT : 1;
+  double re[MT][2] = {}, im[MT][2] = {}, sr[MS][2] = {}, si[MS][2] = {};
+  // K step `step` of nsteps; a(t, kk), b(kk): this lane's elements of fragment kk (CONJ: product with conj(b)).
+  template <bool CONJ, class FA, class FB>
+  __device__ __forceinline__ void add(int step, int nsteps, FA&& a, FB&& b) {
+#pragma unroll
+    for (int kk = 0; kk < ZM_K; kk += 4) {
+      const cplx<double> bv = b(kk);
+#pragma unroll
+      for (int t = 0; t < MT; ++t) {
+        const cplx<double> av = a(t, kk);
+        dmma(re[t], av.x, bv.x);
+        dmma(im[t], av.y, bv.x);
+        dmma(re[t], CONJ ? av.y : -av.y, bv.y);
+        dmma(im[t], CONJ ? -av.x : av.x, bv.y);
+      }
+    }
+    if constexpr (CHAIN > 0) {
+      if (step % CHAIN == CHAIN - 1 || step == nsteps - 1) {
+#pragma unroll
+        for (int t = 0; t < MT; ++t)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            sr[t][e] += re[t][e];
+            si[t][e] += im[t][e];
+            re[t][e] = im[t][e] = 0.0;
+          }
+      }
+    }
+  }
+  __device__ __forceinline__ cplx<double> at(int t, int e) const {
+    return CHAIN ? mk<double>(sr[t % MS][e], si[t % MS][e]) : mk<double>(re[t][e], im[t][e]);
+  }
+};
+
 // Row pitch of a K-contiguous tile: 12 elements of 16 bytes put the two rows of
 // a quarter-warp (8 lanes: 2 rows x 4 k) 64 bytes apart modulo 128.
 constexpr int ZM_PK = ZM_K + 4;
@@ -86,11 +134,7 @@ __global__ void __launch_bounds__(TN * 4) k_zmma_nh(int M, int N, int K, int ksl
     cp_async_commit();  // one group per step, empty past the end
   };
 
-  double re[MT][2], im[MT][2], sr[MT][2], si[MT][2];
-#pragma unroll
-  for (int t = 0; t < MT; ++t)
-#pragma unroll
-    for (int e = 0; e < 2; ++e) re[t][e] = im[t][e] = sr[t][e] = si[t][e] = 0.0;
+  ZmmaSums<MT, ZM_CHAIN> sum;
   chain_wait();
 #pragma unroll
   for (int p = 0; p < ZM_STAGES - 1; ++p) load(p);
@@ -101,28 +145,8 @@ __global__ void __launch_bounds__(TN * 4) k_zmma_nh(int M, int N, int K, int ksl
     const cplx<double>* st = sm + (size_t)(step % ZM_STAGES) * (TM + TN) * ZM_PK;
     const cplx<double>* sa = st + (lane >> 2) * ZM_PK + (lane & 3);
     const cplx<double>* sb = st + (TM + w * 8 + (lane >> 2)) * ZM_PK + (lane & 3);
-#pragma unroll
-    for (int kk = 0; kk < ZM_K; kk += 4) {
-      const cplx<double> bv = sb[kk];
-#pragma unroll
-      for (int t = 0; t < MT; ++t) {
-        const cplx<double> av = sa[t * 8 * ZM_PK + kk];
-        dmma(re[t], av.x, bv.x);
-        dmma(im[t], av.y, bv.x);
-        dmma(re[t], av.y, bv.y);
-        dmma(im[t], -av.x, bv.y);
-      }
-    }
-    if (step % ZM_FLUSH == ZM_FLUSH - 1 || step == nsteps - 1) {
-#pragma unroll
-      for (int t = 0; t < MT; ++t)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          sr[t][e] += re[t][e];
-          si[t][e] += im[t][e];
-          re[t][e] = im[t][e] = 0.0;
-        }
-    }
+    sum.template add<true>(step, nsteps, [&](int t, int kk) { return sa[t * 8 * ZM_PK + kk]; },
+                           [&](int kk) { return sb[kk]; });
   }
   cp_async_wait<0>();
   cplx<double>* P = part + ((int64_t)s * batch + b) * M * N;
@@ -131,8 +155,8 @@ __global__ void __launch_bounds__(TN * 4) k_zmma_nh(int M, int N, int K, int ksl
   for (int t = 0; t < MT; ++t) {
     const int i = i0 + t * 8 + (lane >> 2);
     if (i < M) {
-      if (j < N) P[(int64_t)i * N + j] = mk<double>(sr[t][0], si[t][0]);
-      if (j + 1 < N) P[(int64_t)i * N + j + 1] = mk<double>(sr[t][1], si[t][1]);
+      if (j < N) P[(int64_t)i * N + j] = sum.at(t, 0);
+      if (j + 1 < N) P[(int64_t)i * N + j + 1] = sum.at(t, 1);
     }
   }
 }

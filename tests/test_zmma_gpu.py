@@ -1,5 +1,6 @@
 """Float64 tensor-instruction products (split-K A B^H, nonlocal update) at tile edges, against torch."""
 
+import numpy as np
 import pytest
 import torch
 
@@ -100,3 +101,65 @@ def test_cholesky_and_inverse(n, cuda_device):
     assert float((Li[:2] @ L - eye).abs().max()) < n * 2.3e-16 * 1e4
     assert not torch.triu(Li[:2], 1).any()
     assert bool((Li[2] == 7.0).all())
+
+
+def _err_extended(got, a, b):
+    """Relative 2-norm error of got against a b in extended precision."""
+    g, ar, br = [(v.real.astype(np.longdouble), v.imag.astype(np.longdouble))
+                 for v in (np.asarray(x.resolve_conj().cpu()) for x in (got, a, b))]
+    re, im = ar[0] @ br[0] - ar[1] @ br[1], ar[0] @ br[1] + ar[1] @ br[0]
+    return float(np.sqrt(((g[0] - re) ** 2 + (g[1] - im) ** 2).sum() / (re ** 2 + im ** 2).sum()))
+
+
+# rounding of one operation on numbers of the result's size: uniform in half a unit
+_ROUND = 2.0 ** -53 / np.sqrt(3.0)
+
+
+@pytest.mark.parametrize("op,M,N,K", [(0, 24, 256, 96), (1, 24, 256, 96), (0, 64, 512, 200), (1, 64, 512, 640)])
+def test_short_row_products_rounding(op, M, N, K, cuda_device):
+    """Rounding of a random product. A sum that grows like sqrt(k) errs by sqrt(n / 2) roundings of its final size
+    after n of them: chains of 16 and one addition per 8 terms give sqrt(8 + K / 16), plus the last operations;
+    one chain of 2 K roundings would give sqrt(K)."""
+    from gradwave_b200 import _lib
+    A, B = _rand(*((M, K) if op == 0 else (K, M)), seed=1), _rand(K, N, seed=2)
+    C = torch.empty(M, N, dtype=torch.complex128, device=cuda_device)
+    _lib.call("gwb_zgemm", op, 0, M, N, K, 1.0, 0.0, A.data_ptr(), A.shape[1], 0, B.data_ptr(), N, 0, 0.0, 0.0,
+              C.data_ptr(), N, 0, 1, _lib.stream_ptr())
+    assert _err_extended(C, A if op == 0 else A.T, B) < _ROUND * np.sqrt(10 + K / 16)
+
+
+@pytest.mark.parametrize("M,N,K", [(24, 24, 100), (24, 24, 128), (33, 61, 250)])
+def test_a_bh_products_rounding(M, N, K, cuda_device):
+    """As above with chains of 32 terms (64 roundings) and slices of at least 64 terms: sqrt(32 + K / 64 + 2)."""
+    from gradwave_b200 import _lib
+    A, B = _rand(M, K, seed=1), _rand(N, K, seed=2)
+    C, work = torch.empty(M, N, dtype=torch.complex128, device=cuda_device), torch.empty(8 << 20, dtype=torch.uint8, device=cuda_device)
+    _lib.call("gwb_zgemm_nh", M, N, K, 1.0, 0.0, A.data_ptr(), K, 0, B.data_ptr(), K, 0, 0.0, 0.0, C.data_ptr(), N, 0, 1,
+              work.data_ptr(), work.numel(), _lib.stream_ptr())
+    assert _err_extended(C, A, B.mH) < _ROUND * np.sqrt(34 + K / 64)
+
+
+@pytest.mark.parametrize("nproj", [256, 257, 864])
+def test_nonlocal_rounding(nproj, cuda_device):
+    """S c where the projector sum outweighs c: the contraction (as above, 500 plane waves), and the update with one
+    chain up to 256 projectors (2 nproj roundings), chains of 32 beyond."""
+    from gradwave_b200.basis import BatchedK
+    from gradwave_b200.uspp import BatchedHS
+    npw, nb, n = 500, 8, 12
+    g = torch.Generator().manual_seed(1)
+    z = torch.zeros(1, npw, dtype=torch.float64)
+    d = torch.eye(nproj, dtype=torch.float64)
+    bk = BatchedK(torch.tensor([npw]), torch.ones(1, npw, dtype=torch.bool), torch.randperm(n ** 3, generator=g)[None, :npw],
+                  torch.zeros(1, npw, 3, dtype=torch.float64), z, torch.zeros(0, dtype=torch.complex128),
+                  torch.zeros(nproj, dtype=torch.int64), d).to(cuda_device)
+    p, c = _rand(1, nproj, npw, seed=5), _rand(1, nb, npw, seed=6)
+    v = torch.zeros(n, n, n, dtype=torch.float64, device=cuda_device)
+    s = BatchedHS(bk, (n, n, n), v, p, d, d).hs(c)[1]
+    pe, ce = np.asarray(p[0].cpu()), np.asarray(c[0].cpu())
+    pr, pi, cr, ci = (x.astype(np.longdouble) for x in (pe.real, pe.imag, ce.real, ce.imag))
+    br, bi = cr @ pr.T + ci @ pi.T, ci @ pr.T - cr @ pi.T
+    re, im = cr + br @ pr - bi @ pi, ci + br @ pi + bi @ pr
+    got = np.asarray(s[0].cpu())
+    err = float(np.sqrt(((got.real - re) ** 2 + (got.imag - im) ** 2).sum() / (re ** 2 + im ** 2).sum()))
+    update = nproj if nproj <= 256 else 32 + nproj / 64
+    assert err < _ROUND * np.sqrt(34 + npw / 64 + update + 4)
