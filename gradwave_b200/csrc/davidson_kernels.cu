@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(256) k_chol_inv_smem(cplx<double>* G, int n, i
       if (tid == 0) bad = j + 1;
       break;
     }
-    const double inv = rsqrt(dj);
+    const double ljj = sqrt(dj), inv = 1.0 / ljj;
     // row j of W and column j of L take their scale; the pivot itself stays
     // untouched until every thread has read it
     if (tid < n) {
@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(256) k_chol_inv_smem(cplx<double>* G, int n, i
         else if (c <= i) A[i * n + c] = A[i * n + c] - mul_conj(l, A[c * n + j]);
       }
     }
-    if (tid == 0) A[j * n + j] = mk<double>(dj * inv, 0.0);
+    if (tid == 0) A[j * n + j] = mk<double>(ljj, 0.0);
     __syncthreads();
   }
   __syncthreads();

@@ -163,3 +163,15 @@ def test_nonlocal_rounding(nproj, cuda_device):
     err = float(np.sqrt(((got.real - re) ** 2 + (got.imag - im) ** 2).sum() / (re ** 2 + im ** 2).sum()))
     update = nproj if nproj <= 256 else 32 + nproj / 64
     assert err < _ROUND * np.sqrt(34 + npw / 64 + update + 4)
+
+
+def test_cholesky_of_pivots(cuda_device):
+    """1 x 1 matrices: the factor is the rounded square root and its inverse the rounded quotient, to the last bit."""
+    from gradwave_b200 import _lib
+    g = torch.rand(4096, dtype=torch.float64, generator=torch.Generator().manual_seed(1)) * 100.0
+    F = g.to(torch.complex128).to(cuda_device)
+    Li, info = torch.empty_like(F), torch.zeros(4096, dtype=torch.int32, device=cuda_device)
+    _lib.call("gwb_chol_inv", 4096, 1, F.data_ptr(), 1, 1, Li.data_ptr(), 1, info.data_ptr(), None, _lib.stream_ptr())
+    root = np.sqrt(g.numpy())
+    assert np.array_equal(F.cpu().numpy(), root.astype(np.complex128))
+    assert np.array_equal(Li.cpu().numpy(), (1.0 / root).astype(np.complex128))
