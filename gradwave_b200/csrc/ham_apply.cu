@@ -853,15 +853,17 @@ int gwb_ham_create(const gwb_ham_geometry* geom, int device, gwb_ham** out) {
     }
   h->ndup = (int)(dup.size() / 3);
   std::vector<int> npw32(h->npw_host.begin(), h->npw_host.end());
-  // twiddles exp(-2 pi i a k / n) at k R2 + a (n = R1 R2), computed in double on the host
+  // twiddles exp(-2 pi i a k / n) at k R2 + a (n = R1 R2), the angle reduced exactly: cos and sin of the rounded
+  // 2 pi a k / n are off by up to 8e-16
   std::vector<cplx<double>> tw64[3];
   std::vector<cplx<float>> tw32[3];
   for (int a = 0; a < 3; ++a) {
     const int n = g.n[a], R2 = n / fft_r1(n);
     for (int t = 0; t < n; ++t) {
-      const double ang = -2.0 * M_PI * (double)((t / R2) * (t % R2)) / (double)n;
-      tw64[a].push_back(mk<double>(std::cos(ang), std::sin(ang)));
-      tw32[a].push_back(mk<float>((float)std::cos(ang), (float)std::sin(ang)));
+      const int m = (t / R2) * (t % R2);
+      const double c = rdft_detail::cis(m, n, 0), s = -rdft_detail::cis(m, n, 1);
+      tw64[a].push_back(mk<double>(c, s));
+      tw32[a].push_back(mk<float>((float)c, (float)s));
     }
   }
   auto fail = [&](cudaError_t e) {

@@ -10,9 +10,8 @@
 // that one thread holds.
 //
 // The twiddle constants cos/sin(2 pi k / N) come from a constexpr evaluator
-// (octant reduction on the integer ratio k/N, then Taylor series on
-// [0, pi/4)); they agree with the correctly rounded values to a few ulps of
-// double and are rounded to float once.
+// (quarter-turn reduction on the integer ratio k/N, then Taylor series on
+// [-pi/4, pi/4] in sums of two doubles) and are rounded once.
 #pragma once
 
 #include <type_traits>
@@ -22,44 +21,61 @@
 namespace gwb {
 namespace rdft_detail {
 
-constexpr double kPi = 3.14159265358979323846264338327950288;
-
-constexpr double sin_series(double x) {  // |x| <= pi/4
-  double term = x, sum = x;
-  for (int n = 1; n < 12; ++n) {
-    term *= -x * x / ((2.0 * n) * (2.0 * n + 1.0));
-    sum += term;
-  }
-  return sum;
+// Unevaluated sums h + l of two doubles, for the constants only (Dekker, Numer.
+// Math. 18 (1971) 224).
+struct dd {
+  double h, l;
+};
+constexpr dd two_sum(double a, double b) {
+  const double s = a + b, t = s - a;
+  return {s, (a - (s - t)) + (b - t)};
 }
-constexpr double cos_series(double x) {
-  double term = 1.0, sum = 1.0;
-  for (int n = 1; n < 12; ++n) {
-    term *= -x * x / ((2.0 * n - 1.0) * (2.0 * n));
-    sum += term;
-  }
-  return sum;
+constexpr dd two_prod(double a, double b) {
+  const double ca = 134217729.0 * a, cb = 134217729.0 * b;
+  const double ah = ca - (ca - a), al = a - ah, bh = cb - (cb - b), bl = b - bh;
+  const double p = a * b;
+  return {p, ((ah * bh - p) + ah * bl + al * bh) + al * bl};
 }
-// cos(2 pi k / n) (which = 0) or sin(2 pi k / n) (which = 1)
+constexpr dd add(dd a, dd b) {
+  const dd s = two_sum(a.h, b.h);
+  return two_sum(s.h, s.l + (a.l + b.l));
+}
+constexpr dd mul(dd a, dd b) {
+  const dd p = two_prod(a.h, b.h);
+  return two_sum(p.h, p.l + (a.h * b.l + a.l * b.h));
+}
+constexpr dd div(dd a, double d) {
+  const double q = a.h / d;
+  const dd p = two_prod(q, d);
+  return two_sum(q, ((a.h - p.h) - p.l + a.l) / d);
+}
+// x - x^3/3! + ... (odd) or 1 - x^2/2! + ..., |x| <= pi/4
+constexpr double sin_cos_series(dd x, bool odd) {
+  const dd x2 = mul(x, x);
+  dd term = odd ? x : dd{1.0, 0.0}, sum = term;
+  for (int n = 1; n < 12; ++n) {
+    term = div(mul(term, x2), -(odd ? 2.0 * n * (2.0 * n + 1.0) : (2.0 * n - 1.0) * (2.0 * n)));
+    sum = add(sum, term);
+  }
+  return sum.h;
+}
+// cos(2 pi k / n) (which = 0) or sin(2 pi k / n) (which = 1), rounded to nearest:
+// a constant off by a few units changes the length of what it rotates, and that
+// error adds up in phase over the passes (density of a 49 x 50 x 14 box against
+// extended precision: 5.7e-16 with constants good to a few units, 2.3e-16).
 constexpr double cis(long k, long n, int which) {
   k %= n;
   if (k < 0) k += n;
-  const long q8 = (8 * k) / n;  // octant
-  const double r = 2.0 * kPi * (double)(8 * k - q8 * n) / (8.0 * (double)n);
-  const double cs = cos_series(r), sn = sin_series(r);
-  const double h = 0.70710678118654752440;
-  double cc = 0.0, ss = 0.0;
-  switch (q8) {
-    case 0: cc = cs; ss = sn; break;
-    case 1: cc = h * (cs - sn); ss = h * (cs + sn); break;
-    case 2: cc = -sn; ss = cs; break;
-    case 3: cc = -h * (cs + sn); ss = h * (cs - sn); break;
-    case 4: cc = -cs; ss = -sn; break;
-    case 5: cc = -h * (cs - sn); ss = -h * (cs + sn); break;
-    case 6: cc = sn; ss = -cs; break;
-    default: cc = h * (cs + sn); ss = -h * (cs - sn); break;
+  const long q = (8 * k + n) / (2 * n);  // nearest quarter turn
+  const dd two_pi = {6.283185307179586, 2.4492935982947064e-16};
+  const dd x = div(mul(two_pi, dd{(double)(4 * k - q * n), 0.0}), 4.0 * (double)n);
+  const double c = sin_cos_series(x, false), s = sin_cos_series(x, true);
+  switch (q % 4) {
+    case 0: return which == 0 ? c : s;
+    case 1: return which == 0 ? -s : c;
+    case 2: return which == 0 ? -c : -s;
+    default: return which == 0 ? s : -c;
   }
-  return which == 0 ? cc : ss;
 }
 
 constexpr int first_radix(int n) {
@@ -119,6 +135,16 @@ __host__ __device__ __forceinline__ void small_dft(cplx<T> (&t)[R]) {
     t[2] = a0 - b0;
     t[1] = a1 + b1;
     t[3] = a1 - b1;
+  } else if constexpr (R == 6) {
+    // coprime factors, no twiddles (Good, J. R. Stat. Soc. B 20 (1958) 361):
+    // input 3 a + 2 b, output 3 k + 4 l (mod 6). As 3 x 2 with twiddles the
+    // rounding of sin(pi / 3) enters twice per pass, always with one sign.
+    cplx<T> u[3] = {t[0], t[2], t[4]}, v[3] = {t[3], t[5], t[1]};
+    small_dft<3, SIGN>(u);
+    small_dft<3, SIGN>(v);
+    t[0] = u[0] + v[0], t[3] = u[0] - v[0];
+    t[4] = u[1] + v[1], t[1] = u[1] - v[1];
+    t[2] = u[2] + v[2], t[5] = u[2] - v[2];
   } else if constexpr (R == 5 || R == 7) {
     // odd prime length: with s_j = t_j + t_(R-j), d_j = t_j - t_(R-j),
     // X_k = t_0 + sum_j cos(2 pi j k / R) s_j + SIGN i sum_j sin(2 pi j k / R) d_j
@@ -153,7 +179,7 @@ __host__ __device__ __forceinline__ void small_dft(cplx<T> (&t)[R]) {
 // leaves output X[k]: for N = R M, X[kk + M q] lands where sub-DFT q kept its
 // output kk, i.e. at q + R pos_M(kk) (digit reversal over the radix chain).
 constexpr int out_pos(int n, int k) {
-  if (n <= 5 || n == 7) return k;
+  if (n <= 7) return k;
   const int r = first_radix(n), m = n / r;
   return (k / m) + r * out_pos(m, k % m);
 }
@@ -164,7 +190,7 @@ template <int N, int SIGN, int OFF, int STRIDE, typename T, int NT>
 __host__ __device__ __forceinline__ void dit_ip(cplx<T> (&x)[NT]) {
   if constexpr (N == 1) {
     return;
-  } else if constexpr (N <= 5 || N == 7) {
+  } else if constexpr (N <= 7) {
     cplx<T> t[N];
     StaticFor<0, N>::run([&](auto ic) { t[decltype(ic)::value] = x[OFF + STRIDE * decltype(ic)::value]; });
     small_dft<N, SIGN>(t);
