@@ -338,6 +338,34 @@ __global__ void __launch_bounds__(256) k_row_repair(int npw, int n, cplx<double>
   }
 }
 
+// Noise on the first expansion rows of a cold start (largest residual of the k
+// above cold): row s of every k gets the same random vector of norm about
+// `norm` on its mask, a function of (s, g) alone, so that a k-point gets the
+// same noise whatever batch it is solved in. One CTA per (k, row).
+__global__ void __launch_bounds__(256) k_start_noise(int npw, int n, cplx<double>* __restrict__ D, int64_t dk,
+                                                     const unsigned char* __restrict__ mask,
+                                                     const double* __restrict__ rn, int nb, double cold, double norm) {
+  __shared__ double red[8];
+  chain_wait();
+  D = after_wait(D);
+  mask = after_wait(mask);
+  rn = after_wait(rn);
+  const int k = blockIdx.x / n, s = blockIdx.x % n;
+  double worst = 0.0;
+  for (int b = 0; b < nb; ++b) worst = fmax(worst, rn[(int64_t)k * nb + b]);
+  if (!(worst > cold)) return;
+  const unsigned char* mk_ = mask + (int64_t)k * npw;
+  double count = 0.0;
+  for (int g = threadIdx.x; g < npw; g += blockDim.x) count += mk_[g] ? 1.0 : 0.0;
+  count = block_sum<256>(count, red);
+  const double a = norm * sqrt(1.5 / count);  // a uniform pair in [-1, 1) has mean square 2/3
+  cplx<double>* row = D + k * dk + (int64_t)s * npw;
+  for (int g = threadIdx.x; g < npw; g += blockDim.x) {
+    const unsigned long long key = (((unsigned long long)s << 32) + (unsigned long long)g) * 2ull;
+    if (mk_[g]) row[g] = row[g] + mk<double>(a * hash_unit(key), a * hash_unit(key + 1));
+  }
+}
+
 }  // namespace gwb
 
 using namespace gwb;
@@ -414,6 +442,16 @@ int gwb_row_repair(int32_t nk, int32_t n, int32_t npw, void* D, int64_t d_kstrid
   GWB_REQUIRE(nk > 0 && n > 0 && npw > 0, "bad sizes");
   GWB_REQUIRE(D && mask && flag, "null pointer");
   GWB_CUDA_TRY(launch_chained(k_row_repair, dim3(nk * n), 256, 0, (cudaStream_t)stream, npw, n, (cplx<double>*)D, d_kstride, mask, thresh, flag));
+  count_launches(1);
+  return GWB_OK;
+}
+
+int gwb_start_noise(int32_t nk, int32_t n, int32_t npw, void* D, int64_t d_kstride, const uint8_t* mask, const double* rn,
+                    int32_t nb, double cold, double norm, void* stream) {
+  GWB_REQUIRE(nk > 0 && n > 0 && npw > 0 && nb > 0, "bad sizes");
+  GWB_REQUIRE(D && mask && rn, "null pointer");
+  GWB_CUDA_TRY(launch_chained(k_start_noise, dim3(nk * n), 256, 0, (cudaStream_t)stream, npw, n, (cplx<double>*)D,
+                              d_kstride, mask, rn, nb, cold, norm));
   count_launches(1);
   return GWB_OK;
 }

@@ -90,6 +90,7 @@ int gwb_precond_teter(int32_t, int32_t, int32_t, int32_t, const void*, int64_t, 
 int gwb_subspace_insert(int32_t, int32_t, int32_t, const void*, void*, int32_t, int64_t, void*);
 int gwb_chol_inv(int32_t, int32_t, void*, int32_t, int64_t, void*, int64_t, int32_t*, int32_t*, void*);
 int gwb_row_repair(int32_t, int32_t, int32_t, void*, int64_t, const uint8_t*, double, int32_t*, void*);
+int gwb_start_noise(int32_t, int32_t, int32_t, void*, int64_t, const uint8_t*, const double*, int32_t, double, double, void*);
 int gwb_heev_lowest(int32_t, int32_t, int32_t, const void*, int32_t, int64_t, double*, void*, double*, int32_t*,
                     void*);
 int gwb_heev_max_dim(void);
@@ -103,6 +104,11 @@ int gwb_stall_update(const double*, double*, uint8_t*, uint8_t*, int32_t, double
 }
 
 namespace gwb {
+
+// Noise on the first expansion rows of a cold start (gwb_start_noise): norm, and
+// the largest residual [eV] above which a start counts as cold. The host driver
+// has the same (davidson.py, break_symmetry, with the reasons).
+constexpr double kStartNoise = 0.25, kColdStartEv = 1.0;
 
 struct Buf {
   size_t off = 0;
@@ -273,6 +279,7 @@ class Solver {
       if (rnmax < p_.tol) return finish(it, eig, eig_out, vec_out, rn_out, out, rnmax);
       GWB_TRY(gwb_select_worst(nk_, nb_, w_.rn, n_add, w_.sel, st_));
       GWB_TRY(precondition(n_add, eig));
+      if (it == 1) GWB_TRY(gwb_start_noise(nk_, n_add, npw_, w_.D, nbp, mask_, w_.rn, nb_, kColdStartEv, kStartNoise, st_));
       if (m + n_add > md_) {
         ++n_restart_;
         GWB_TRY(cholqr2(w_.X, nbp, nb_, w_.D2, w_.X, nbp, w_.HX, w_.R, /*sync=*/true, &ok));

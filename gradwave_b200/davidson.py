@@ -18,8 +18,8 @@ buffer), the subspace matrix is updated incrementally (only the new columns
 are formed, ``gwb_subspace_insert``), and orthonormalisation is CholQR2
 (float64 Gram, Cholesky, triangular inverse; the reference's own optional
 path, ``solvers/davidson.py:195-222``) with the reference's jitter + QR
-fallback on breakdown. A cold start of a large basis gets seeded noise on its
-first expansion rows (``_Solver.break_symmetry``).
+fallback on breakdown. A cold start gets noise on its first expansion rows
+(``_Solver.break_symmetry``; the native driver has the same).
 
 Modes:
   ``mode="fp64"``     every apply in float64 (plain TPA Davidson).
@@ -65,7 +65,7 @@ logger = logging.getLogger(__name__)
 _FP32_CERT_FLOOR_EPS = 32 * torch.finfo(torch.float32).eps
 _FP32_CERT_STALL = 0.7
 # norm of the noise on the unit rows of the first expansion of a cold start
-# (largest residual above _COLD_START_EV)
+# (largest residual of a k-point above _COLD_START_EV)
 _START_NOISE = 0.25
 _COLD_START_EV = 1.0
 _N, _T, _H = 0, 1, 2
@@ -578,7 +578,7 @@ class _Solver:
             with self.prof("precond"):
                 _lib.call("gwb_select_worst", nk, nb, _ptr(ws.rn), n_add, _ptr(ws.sel), self.stream)
                 self.precondition(n_add, eig)
-                if it == 1 and self.max_dim > self.heev_max and rnmax > _COLD_START_EV:
+                if it == 1:
                     self.break_symmetry(n_add)
             if m + n_add > md:
                 # restart: re-orthonormalise the Ritz block, images by the same
@@ -611,19 +611,24 @@ class _Solver:
         return self.result(eig, self.max_iter)
 
     def break_symmetry(self, n_add: int):
-        """Seeded noise on the first expansion rows of a cold start. A start
-        block of plane waves on a symmetric cell has no component in some
+        """Noise on the first expansion rows of the k-points that start cold. A
+        start block of plane waves on a symmetric cell has no component in some
         irreducible representations, and no step of the solver brings one in
-        but round-off: a solve may then converge to eigenpairs that skip a
-        level (64-atom cell, float64, identity start with 1e-15 of noise: 6 of
-        8 solves skip one at the block's upper edge; with the noise none of 45).
-        Rounds to 1e-10 eV by its norm (float64 / mixed / mixed with the
-        network): 3e-6 49-53 / 87-208 / 37-38, 3e-4 45-165 / 61-230 / 41-125,
-        0.03 78-100 / 79-137 / 38-44, 0.27 52-55 / 51-78 / 40."""
-        gen = torch.Generator(device=self.dev).manual_seed(20260 + n_add)
-        noise = torch.randn(self.nk, n_add, self.npw, 2, dtype=torch.float64, device=self.dev, generator=gen)
-        self.ws.D[:, :n_add].add_(torch.view_as_complex(noise) * self.mask[:, None, :], 
-                                      alpha=_START_NOISE / math.sqrt(2.0 * self.npw))
+        but round-off: such a level shows up only after round-off has grown to
+        the size of a Ritz vector, and a solve that converges before skips it.
+        Noise of the order of the rows themselves lets it converge with the
+        others. Perfect 2- and 8-atom cells, 6 to 40 bands, identity starts
+        1e-15 apart, float64 and mixed, both preconditioners: 21 of 864 solves
+        skip a level without it (0.2 to 5 eV), none with norms 0.05, 0.25 and
+        0.7; mean rounds 47, 47, 49 and 48. The perfect 64-atom cell: 6 of 8
+        without (float64), none of 24 with it (rounds, float64 / mixed / mixed
+        with the network: 51-57, 50-77, 39-40).
+
+        The noise is a function of row and plane wave alone, so that a k-point
+        is solved alike in whatever group or shard it is."""
+        ws, npw = self.ws, self.npw
+        _lib.call("gwb_start_noise", self.nk, n_add, npw, _ptr(ws.D), ws.D.shape[1] * npw, _ptr(self.mask_u8),
+                  _ptr(ws.rn), self.nb, _COLD_START_EV, _START_NOISE, self.stream)
 
     def precondition(self, n_add: int, eig: torch.Tensor):
         """D[:, :n_add] = preconditioned, unit-normalised worst residuals."""

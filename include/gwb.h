@@ -415,6 +415,13 @@ int gwb_chol_inv(int32_t nk, int32_t n, void* G, int32_t ldg, int64_t g_kstride,
 int gwb_row_repair(int32_t nk, int32_t n, int32_t npw, void* D, int64_t d_kstride, const uint8_t* mask,
                    double thresh, int32_t* flag, void* stream);
 
+/* Noise on the first expansion rows D of a cold start (nk blocks of n unit
+ * rows, d_kstride apart): k-points whose largest residual norm rn (nk, nb)
+ * exceeds cold get masked deterministic noise of norm about `norm` added to
+ * each row, the same for every k. No counterpart in the reference. */
+int gwb_start_noise(int32_t nk, int32_t n, int32_t npw, void* D, int64_t d_kstride, const uint8_t* mask, const double* rn,
+                    int32_t nb, double cold, double norm, void* stream);
+
 /* Lowest nb eigenpairs of nk Hermitian m x m matrices S (leading dim lds,
  * both triangles filled), float64: eig (nk, nb) ascending, U (nk, m, nb)
  * row-major eigenvector columns; zscratch (nk, gwb_heev_scratch_doubles(m))

@@ -220,3 +220,66 @@ def test_large_cells_match_reference(cuda_device, name, mode):
     assert abs(_band_energy(eig, ci.kweights, nocc) - _band_energy(g["eigenvalues"], ci.kweights, nocc)) < BAND_E_TOL
     if mode == "mixed":
         assert res.info.get("tc_projection")
+
+
+def _dense_lowest(apply, mask, nb):
+    """Lowest nb eigenvalues of the operator's dense matrix at each k."""
+    nk, npw = mask.shape
+    out = []
+    for k in range(nk):
+        n = int(mask[k].sum())
+        h = torch.empty(n, n, dtype=torch.complex128, device=mask.device)
+        for s in range(0, n, 256):
+            e = min(n, s + 256)
+            c = torch.zeros(nk, e - s, npw, dtype=torch.complex128, device=mask.device)
+            c[k, torch.arange(e - s), torch.arange(s, e)] = 1.0
+            h[s:e] = apply(c)[k, :, :n]
+        out.append(torch.linalg.eigvalsh((0.5 * (h + h.mH)).mT.contiguous())[:nb])
+    return torch.stack(out)
+
+
+@pytest.mark.parametrize("precond", ["teter", "learned"])
+def test_symmetric_cell_keeps_every_level(cuda_device, precond):
+    """Identity starts (with and without 1e-15 of noise) on the perfect 8-atom cell, bases on both sides of the
+    batched eigensolver's limit (native and host driver): the lowest eigenvalues of the dense matrices."""
+    from gradwave_b200 import learned
+    from gradwave_b200.davidson import davidson_batched
+    if precond == "learned":
+        if not learned.available():
+            pytest.skip("no trained network")
+        precond = learned.LearnedPreconditioner.load(device=cuda_device)
+    ci, bk, full = _cell_ham("si8_cubic")
+    h = full.k_slice(0, 2)
+    mask, t = bk.mask[:2], bk.t[:2]
+    exact = _dense_lowest(h.apply, mask, 32)
+    gen = torch.Generator(device=cuda_device).manual_seed(1)
+    for nb in (16, 20, 26, 32):
+        x0 = torch.zeros(2, nb, mask.shape[1], dtype=torch.complex128, device=cuda_device)
+        x0[:, torch.arange(nb), torch.arange(nb)] = 1.0
+        for eps in (0.0, 1e-15, 1e-15):
+            x = x0 + eps * torch.randn(x0.shape, dtype=x0.dtype, device=cuda_device, generator=gen) * mask[:, None]
+            res = davidson_batched(h.apply, x, t, mask, tol=1e-8, max_iter=300, precond=precond)
+            # an eigenvalue's error is below its residual (1e-8) once the right level is found
+            assert float((res.eigenvalues - exact[:, :nb]).abs().max()) < 1e-7, (nb, eps)
+
+
+def test_start_noise_of_a_k_point(cuda_device):
+    """The noise of a cold start: the same for a k-point alone and in a batch of wider rows, nothing off its sphere
+    or at a k-point that starts near its solution, norm 0.25 (5 sigma of a sum of 3000 uniform squares: 5 %)."""
+    from gradwave_b200 import _lib
+    npw, nb = [3000, 700, 1500], 6
+    mask = torch.zeros(3, 3100, dtype=torch.uint8, device=cuda_device)
+    for k in range(3):
+        mask[k, :npw[k]] = 1
+    rn = torch.tensor([[0.1, 2.0, 0, 0, 0, 0], [0.5, 0.9, 0, 0, 0, 0], [0, 0, 0, 0, 0, 1.5]], dtype=torch.float64,
+                      device=cuda_device)
+    d = torch.zeros(3, nb, 3100, dtype=torch.complex128, device=cuda_device)
+    _lib.call("gwb_start_noise", 3, nb, 3100, d.data_ptr(), nb * 3100, mask.data_ptr(), rn.data_ptr(), nb, 1.0, 0.25,
+              _lib.stream_ptr())
+    assert not d[1].any() and not d[0, :, 3000:].any() and not d[2, :, 1500:].any()
+    norm = torch.linalg.vector_norm(d, dim=-1)
+    assert float((norm[[0, 2]] / 0.25 - 1.0).abs().max()) < 0.05
+    alone = torch.zeros(1, nb, 1500, dtype=torch.complex128, device=cuda_device)
+    _lib.call("gwb_start_noise", 1, nb, 1500, alone.data_ptr(), nb * 1500, mask[2, :1500].contiguous().data_ptr(),
+              rn[2].contiguous().data_ptr(), nb, 1.0, 0.25, _lib.stream_ptr())
+    assert torch.equal(alone[0], d[2, :, :1500])
