@@ -25,6 +25,7 @@ the reference's ``davidson_gamma`` runs the single-k ``davidson``
 from __future__ import annotations
 
 import ctypes
+import math
 import os
 from dataclasses import dataclass
 
@@ -759,7 +760,7 @@ def davidson_gamma(ham: GammaHamiltonian, x0: torch.Tensor, tol: float = 1e-9, m
     if n_buffer < 0:
         raise ValueError(f"n_buffer must be >= 0, got {n_buffer}")
     import os
-    from .davidson import _PhaseTimer
+    from .davidson import _COLD_START_EV, _START_NOISE, _PhaseTimer
     prof = _PhaseTimer(os.environ.get("GWB_PROFILE", "0") == "1")
     lock = (mode == "mixed") if lock is None else bool(lock)
     gb, dev = ham.gb, ham.device
@@ -812,6 +813,7 @@ def davidson_gamma(ham: GammaHamiltonian, x0: torch.Tensor, tol: float = 1e-9, m
     own_eigh = _OwnEigh(dev) if dev.type == "cuda" and os.environ.get("GWB_OWN_EIGH", "1") != "0" else None
     info = {"rounds_tc": 0, "rounds_f32": 0, "rounds_f64": 0, "handoff_rn_ev": None, "m": []}
     v0 = _orthonormalize(phi0.clone())
+    no_random_row = v0.shape[0] == nb
     if v0.shape[0] < nb:  # degenerate start: pad with seeded noise (``:345-350``)
         gen = torch.Generator(device="cpu").manual_seed(1234)
         pad = torch.randn(nb - v0.shape[0], nphi, generator=gen, dtype=torch.float64).to(dev)
@@ -961,6 +963,19 @@ def davidson_gamma(ham: GammaHamiltonian, x0: torch.Tensor, tol: float = 1e-9, m
             else:
                 t_band = (x * x * t_phi[None, :]).sum(dim=1)
                 pr = _teter(r[unconv], t_phi, t_band[unconv])
+            if it == 1 and no_random_row and rmax > _COLD_START_EV:
+                # a start of plane waves on a symmetric cell lacks whole
+                # irreducible representations (davidson.py, break_symmetry):
+                # 36 of 96 solves of the perfect 8-atom cell skipped a level by
+                # 2 to 5 eV. A level must have grown from this noise to a Ritz
+                # vector when the others reach tol: none of 440 solves to 1e-6
+                # eV or below skips with 0.3 sqrt(tol), 9 with 0.1 sqrt(tol);
+                # larger noise costs the tight solves of small cells rounds
+                # (2 atoms to 1e-6 eV: 19 without, 20-22, 20-26 at sqrt(tol))
+                pr = pr / torch.linalg.vector_norm(pr, dim=1, keepdim=True).clamp_min(1e-300)
+                gen = torch.Generator(device=dev).manual_seed(20260)
+                noise = torch.randn(pr.shape, generator=gen, dtype=pr.dtype, device=dev)
+                pr += min(_START_NOISE, 0.3 * math.sqrt(tol)) / math.sqrt(nphi) * noise
             pr[:, nphi:] = 0.0  # the pad column is not a coordinate of the operator
         with phase("orthonormalize"):
             t = _expand(pr, v, tcp, locked.rows(), mm, low=low and tc_active)

@@ -102,3 +102,20 @@ def test_gamma_apply_accepts_transposed_blocks(cuda_device):
     phi = torch.randn(2 * gb.nhalf - 1, 6, generator=g, dtype=torch.float64).to(cuda_device).T
     assert not phi.is_contiguous()
     assert torch.equal(gh.apply_phi(phi), gh.apply_phi(phi.contiguous()))
+
+
+@pytest.mark.parametrize("nb", [16, 18, 20, 24])
+def test_symmetric_cell_keeps_every_level(cuda_device, nb):
+    """Identity start on the perfect 8-atom cell at Gamma, float64 (no random row in the start block): the
+    reference's own eigenvalues of that k-point, both preconditioners."""
+    from gradwave_b200 import learned
+    from gradwave_b200.cells import make_cell
+    from gradwave_b200.gamma import GammaHamiltonian, build_gamma_basis, davidson_gamma, gamma_start
+    ci = make_cell("si8_cubic")
+    gb = build_gamma_basis(ci.spheres[0], ci.shape)
+    gh = GammaHamiltonian(gb, ci.v_eff_r, ci.p[0][:, :gb.npw], ci.bk.dij_full, device=cuda_device)
+    exact = load_golden("si8_cubic")["eigenvalues"][0, :nb]
+    pcs = ["teter"] + ([learned.LearnedPreconditioner.load(device=cuda_device)] if learned.available() else [])
+    for pc in pcs:
+        res = davidson_gamma(gh, gamma_start(gb, nb, cuda_device), tol=1e-8, max_iter=300, precond=pc)
+        assert np.abs(res.eigenvalues.cpu().numpy() - exact).max() < 1e-7
