@@ -174,10 +174,13 @@ inline cudaError_t allow_smem(F* func) {
 
 }  // namespace gwb
 
+// A failed call is reported once: its code leaves the thread's last-error slot,
+// where the next launch check would take it for its own.
 #define GWB_CUDA_TRY(expr)                                                        \
   do {                                                                            \
     cudaError_t _e = (expr);                                                      \
     if (_e != cudaSuccess) {                                                      \
+      cudaGetLastError();                                                         \
       gwb::set_error(std::string(#expr) + ": " + cudaGetErrorString(_e));         \
       return GWB_ERR_CUDA;                                                        \
     }                                                                             \

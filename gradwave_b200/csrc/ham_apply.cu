@@ -867,6 +867,7 @@ int gwb_ham_create(const gwb_ham_geometry* geom, int device, gwb_ham** out) {
     }
   }
   auto fail = [&](cudaError_t e) {
+    cudaGetLastError();
     set_error(std::string("gwb_ham_create: ") + cudaGetErrorString(e));
     gwb_ham_destroy(h);
     return GWB_ERR_CUDA;
@@ -918,6 +919,8 @@ int gwb_ham_destroy(gwb_ham* h) {
     if (idle) {
       scratch_give(h->device, h->d_W, h->W_bytes);
       h->d_W = nullptr;
+    } else {
+      cudaGetLastError();
     }
     cudaSetDevice(cur);
   }

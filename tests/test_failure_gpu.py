@@ -118,3 +118,25 @@ def test_tensor_core_wait_runs_out(cuda_device):
     ref = A @ B.conj().transpose(-1, -2)
     bound = A.abs() @ B.abs().transpose(-1, -2)
     assert float(((C - ref).abs() / bound).max()) < 4e-5
+
+
+def test_refused_launch_is_reported_once(cuda_device):
+    """A launch that the runtime refuses (the sum over slices of 1537 projectors asks for more shared memory than a
+    block has by default) is an error of its own call and of no later one."""
+    from gradwave_b200 import _lib
+    from gradwave_b200.basis import BatchedK
+    from gradwave_b200.hamiltonian import BatchedHamiltonian
+    nproj, npw, n = 1537, 40, 6
+    g = torch.Generator().manual_seed(1)
+    bk = BatchedK(torch.tensor([npw]), torch.ones(1, npw, dtype=torch.bool), torch.randperm(n ** 3, generator=g)[None, :npw],
+                  torch.zeros(1, npw, 3, dtype=torch.float64), torch.zeros(1, npw, dtype=torch.float64),
+                  torch.zeros(0, dtype=torch.complex128), torch.zeros(nproj, dtype=torch.int64),
+                  torch.eye(nproj, dtype=torch.float64)).to(cuda_device)
+    v = torch.ones(n, n, n, dtype=torch.float64, device=cuda_device)
+    h = BatchedHamiltonian(bk, (n, n, n), v, torch.zeros(1, nproj, npw, dtype=torch.complex128, device=cuda_device))
+    c = torch.ones(1, 2, npw, dtype=torch.complex128, device=cuda_device)
+    with pytest.raises(_lib.GwbError):
+        h.apply(c)
+    torch.cuda.synchronize()
+    _lib.call("gwb_ham_set_potential", h._h, v.data_ptr(), _lib.stream_ptr())
+    assert float((h.apply_fp32(c) - c).abs().max()) < 1e-5   # v = 1: H c = c
