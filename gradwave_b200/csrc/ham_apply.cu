@@ -19,12 +19,11 @@
 #include <cstdlib>
 #include <cstring>
 #include <atomic>
-#include <map>
-#include <mutex>
 #include <string>
 #include <vector>
 
 #include "common.cuh"
+#include "device_pool.cuh"
 #include "fft_axis.cuh"
 #include "zmma.cuh"
 
@@ -401,81 +400,25 @@ __global__ void k_column_lists(const double* __restrict__ D, int n, int* __restr
   cnt[q] = c;
 }
 
-static cudaError_t alloc_columns(ColumnLists* c, int n) {
-  const cudaError_t e = cudaMalloc((void**)&c->cnt, (size_t)n * sizeof(int));
-  return e != cudaSuccess ? e : cudaMalloc((void**)&c->idx, (size_t)n * n * sizeof(int));
-}
-
 __global__ void k_c128_to_c64(const cplx<double>* src, cplx<float>* dst, size_t n) {
   size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (i < n) dst[i] = mk<float>((float)src[i].x, (float)src[i].y);
 }
 
-// The band-chunk scratch of a destroyed handle waits here for the next handle
-// on the device (mapping half a GB takes milliseconds, as long as many an
-// apply): at most one buffer per device, kept only while a handle lives there
-// and given back when an allocation fails.
-struct ScratchSlot {
-  int handles = 0;
-  void* p = nullptr;
-  size_t bytes = 0;
-};
-static std::mutex g_scratch_mu;
-static std::map<int, ScratchSlot> g_scratch;
-
-static void scratch_handle(int dev, int n) {
-  void* drop = nullptr;
-  {
-    std::lock_guard<std::mutex> lk(g_scratch_mu);
-    ScratchSlot& s = g_scratch[dev];
-    s.handles += n;
-    if (s.handles == 0) {
-      drop = s.p;
-      s.p = nullptr;
-      s.bytes = 0;
-    }
-  }
-  if (drop) cudaFree(drop);
-}
-
-// A kept buffer of at least need bytes (need = 0: any), or null.
-static void* scratch_take(int dev, size_t need, size_t* bytes) {
-  std::lock_guard<std::mutex> lk(g_scratch_mu);
-  ScratchSlot& s = g_scratch[dev];
-  if (!s.p || s.bytes < need) return nullptr;
-  void* p = s.p;
-  *bytes = s.bytes;
-  s.p = nullptr;
-  s.bytes = 0;
-  return p;
-}
-
-// p is idle (its device has been synchronised). The larger of it and the kept
-// buffer stays.
-static void scratch_give(int dev, void* p, size_t bytes) {
-  {
-    std::lock_guard<std::mutex> lk(g_scratch_mu);
-    ScratchSlot& s = g_scratch[dev];
-    if (s.handles > 0 && bytes > s.bytes) {
-      std::swap(p, s.p);
-      s.bytes = bytes;
-    }
-  }
-  if (p) cudaFree(p);
-}
-
-static int ensure_buf(void** p, size_t* have, size_t need) {
-  if (*have >= need) return GWB_OK;
-  if (*p) cudaFree(*p);
-  *p = nullptr;
-  *have = 0;
-  if (cudaMalloc(p, need) != cudaSuccess) {
+struct CudaMemory {
+  static bool alloc(void** p, size_t bytes) {
+    if (cudaMalloc(p, bytes) == cudaSuccess) return true;
     cudaGetLastError();
-    set_error("device allocation of " + std::to_string(need) + " bytes failed");
-    return GWB_ERR_ALLOC;
+    return false;
   }
-  *have = need;
-  return GWB_OK;
+  static void free(void* p) { cudaFree(p); }
+};
+static DevicePool<CudaMemory> g_pool;
+
+static int ensure_buf(const gwb_ham* h, void** p, size_t* have, size_t need) {
+  if (g_pool.ensure(h->device, p, have, need)) return GWB_OK;
+  set_error("device allocation of " + std::to_string(need) + " bytes failed");
+  return GWB_ERR_ALLOC;
 }
 
 // G slices of the becp reduction: enough CTAs to fill the GPU (4 per SM)
@@ -496,20 +439,13 @@ static int chunk_scratch(gwb_ham* h, int nb, size_t es, int* nbc) {
   const size_t per_band = (size_t)h->nk * ((size_t)g.L[0] * g.n[1] + g.nrow) * g.n[2] * es;
   auto ensure = [&](size_t need) {
     if (h->W_bytes >= need) return GWB_OK;
-    if (void* p = scratch_take(h->device, need, &need)) {
+    if (void* p = g_pool.take(h->device, need, &need)) {
       if (h->d_W) cudaFree(h->d_W);
       h->d_W = p;
       h->W_bytes = need;
       return GWB_OK;
     }
-    int rc = ensure_buf(&h->d_W, &h->W_bytes, need);
-    size_t n = 0;
-    void* kept = rc == GWB_ERR_ALLOC ? scratch_take(h->device, 0, &n) : nullptr;
-    if (kept) {
-      cudaFree(kept);
-      rc = ensure_buf(&h->d_W, &h->W_bytes, need);
-    }
-    return rc;
+    return ensure_buf(h, &h->d_W, &h->W_bytes, need);
   };
   auto bands = [&](size_t budget) {
     const size_t most = std::min<size_t>(32768, std::max<size_t>(1, budget / per_band));  // bands are a grid axis
@@ -574,21 +510,22 @@ static int nonlocal_tc(gwb_ham* h, const cplx<double>* c, int64_t ck, cplx<doubl
   const int64_t ldp = ((int64_t)npw + 7) / 8 * 8, ldq = ((int64_t)np + 7) / 8 * 8;
   int rc;
   if (!h->d_tcstatus) {
-    GWB_CUDA_TRY(cudaMalloc((void**)&h->d_tcstatus, sizeof(int)));
+    size_t n = 0;
+    if ((rc = ensure_buf(h, (void**)&h->d_tcstatus, &n, sizeof(int)))) return rc;
     GWB_CUDA_TRY(cudaMemsetAsync(h->d_tcstatus, 0, sizeof(int), st));
   }
   if (!h->pplanes_ok) {
-    if ((rc = ensure_buf(&h->d_pplanes, &h->pplanes_bytes, (size_t)nk * 4 * np * ldp * 2))) return rc;
+    if ((rc = ensure_buf(h, &h->d_pplanes, &h->pplanes_bytes, (size_t)nk * 4 * np * ldp * 2))) return rc;
     if ((rc = gwb_tc_planes(nk, np, npw, h->d_p64, npw, (int64_t)np * npw, GWB_C128, 0, h->d_pplanes, ldp, np, 0,
                             st)))
       return rc;
     h->pplanes_ok = true;
   }
-  if ((rc = ensure_buf(&h->d_cplanes, &h->cplanes_bytes, (size_t)nk * 4 * nb * ldp * 2))) return rc;
-  if ((rc = ensure_buf(&h->d_becp, &h->becp_bytes, (size_t)nk * nb * np * 16))) return rc;
-  if ((rc = ensure_buf(&h->d_bdplanes, &h->bdplanes_bytes, (size_t)nk * 4 * nb * ldq * 2))) return rc;
+  if ((rc = ensure_buf(h, &h->d_cplanes, &h->cplanes_bytes, (size_t)nk * 4 * nb * ldp * 2))) return rc;
+  if ((rc = ensure_buf(h, &h->d_becp, &h->becp_bytes, (size_t)nk * nb * np * 16))) return rc;
+  if ((rc = ensure_buf(h, &h->d_bdplanes, &h->bdplanes_bytes, (size_t)nk * 4 * nb * ldq * 2))) return rc;
   const int64_t wb = gwb_zgemm_tc_work_bytes(2, nb, np, npw, nk);
-  if (wb > 0 && (rc = ensure_buf(&h->d_tcwork, &h->tcwork_bytes, (size_t)wb))) return rc;
+  if (wb > 0 && (rc = ensure_buf(h, &h->d_tcwork, &h->tcwork_bytes, (size_t)wb))) return rc;
   if ((rc = gwb_tc_planes(nk, nb, npw, c, npw, ck, GWB_C128, 0, h->d_cplanes, ldp, nb, 0, st))) return rc;
   if ((rc = gwb_zgemm_tc(2, nb, np, npw, 1.0, 0.0, h->d_cplanes, ldp, nb, h->d_pplanes, ldp, np, 0.0, 0.0, h->d_becp,
                          np, (int64_t)nb * np, nk, h->d_tcwork, h->tcwork_bytes, h->d_tcstatus, st)))
@@ -647,9 +584,9 @@ static int becp_slices(gwb_ham* h, const SIO* c, int64_t ck, int nb, int* nsl, c
     gslice = ((npw + ns - 1) / ns + NL_TG - 1) / NL_TG * NL_TG;
     *nsl = (npw + gslice - 1) / gslice;
   }
-  int rc = ensure_buf(&h->d_part, &h->part_bytes, (size_t)*nsl * h->nk * nb * np * es);
+  int rc = ensure_buf(h, &h->d_part, &h->part_bytes, (size_t)*nsl * h->nk * nb * np * es);
   if (rc) return rc;
-  if ((rc = ensure_buf(&h->d_bd, &h->bd_bytes, (size_t)h->nk * nb * np * es))) return rc;
+  if ((rc = ensure_buf(h, &h->d_bd, &h->bd_bytes, (size_t)h->nk * nb * np * es))) return rc;
   if constexpr (nl_zmma<T, SIO>) {
     GWB_CUDA_TRY(zmma_nh(nb, np, npw, gslice, *nsl, c, npw, ck, h->d_p64, npw, (int64_t)np * npw,
                          (cplx<double>*)h->d_part, h->nk, st));
@@ -705,7 +642,7 @@ static int apply_hs_impl(gwb_ham* h, const SIO* c, int64_t ck, SIO* out_h, int64
   if (h->nproj > 0) {
     int nsl = 0;
     if ((rc = becp_slices<T, SIO>(h, c, ck, nb, &nsl, st))) return rc;
-    if ((rc = ensure_buf(&h->d_bq, &h->bq_bytes, (size_t)h->nk * nb * h->nproj * es))) return rc;
+    if ((rc = ensure_buf(h, &h->d_bq, &h->bq_bytes, (size_t)h->nk * nb * h->nproj * es))) return rc;
     const T* D = dbl ? (const T*)h->d_d64 : (const T*)h->d_d32;
     const T* Q = dbl ? (const T*)h->d_q64 : (const T*)h->d_q32;
     const int ngrp = std::max(1, 128 / h->nproj);
@@ -743,7 +680,7 @@ static int density_impl(gwb_ham* h, const SIO* c, int64_t ck, int nb, const doub
   // the same for every chunking, so that chunks do not change the sums
   const int64_t blocks = (int64_t)h->nk * ((g.n[1] * g.n[2] + 15) / 16);
   const int ngrp = (int)std::max<int64_t>(1, std::min<int64_t>((8 * 148 + blocks - 1) / blocks, nb / 2));
-  rc = ensure_buf((void**)&h->d_rhok, &h->rhok_bytes, (size_t)h->nk * ngrp * N * sizeof(double));
+  rc = ensure_buf(h, (void**)&h->d_rhok, &h->rhok_bytes, (size_t)h->nk * ngrp * N * sizeof(double));
   if (rc) return rc;
   FftRun<double> f = fft_run<double>(h, nbc);
   f.c = c, f.ck = ck, f.io64 = sizeof(SIO) == 16;
@@ -872,12 +809,12 @@ int gwb_ham_create(const gwb_ham_geometry* geom, int device, gwb_ham** out) {
     gwb_ham_destroy(h);
     return GWB_ERR_CUDA;
   };
+  auto no_room = [&] { return fail(cudaErrorMemoryAllocation); };
   cudaError_t e = cudaSetDevice(device);
   if (e != cudaSuccess) return fail(e);
 #define GWB_ALLOC_COPY(dst, vec)                                                            \
   do {                                                                                      \
-    e = cudaMalloc((void**)&(dst), (vec).size() * sizeof((vec)[0]));                        \
-    if (e != cudaSuccess) return fail(e);                                                   \
+    if (!g_pool.alloc(device, (void**)&(dst), (vec).size() * sizeof((vec)[0]))) return no_room(); \
     e = cudaMemcpy((dst), (vec).data(), (vec).size() * sizeof((vec)[0]), cudaMemcpyHostToDevice); \
     if (e != cudaSuccess) return fail(e);                                                   \
   } while (0)
@@ -891,19 +828,20 @@ int gwb_ham_create(const gwb_ham_geometry* geom, int device, gwb_ham** out) {
   }
 #undef GWB_ALLOC_COPY
   const size_t nkp = (size_t)h->nk * h->npw_max;
-  if ((e = cudaMalloc((void**)&h->d_t64, nkp * 8)) != cudaSuccess) return fail(e);
-  if ((e = cudaMalloc((void**)&h->d_t32, nkp * 4)) != cudaSuccess) return fail(e);
-  if ((e = cudaMalloc((void**)&h->d_v64, nbox * 8)) != cudaSuccess) return fail(e);
-  if ((e = cudaMalloc((void**)&h->d_v32, nbox * 4)) != cudaSuccess) return fail(e);
+  if (!g_pool.alloc(device, (void**)&h->d_t64, nkp * 8)) return no_room();
+  if (!g_pool.alloc(device, (void**)&h->d_t32, nkp * 4)) return no_room();
+  if (!g_pool.alloc(device, (void**)&h->d_v64, nbox * 8)) return no_room();
+  if (!g_pool.alloc(device, (void**)&h->d_v32, nbox * 4)) return no_room();
   if (h->nproj > 0) {
     const size_t np = (size_t)h->nk * h->nproj * h->npw_max;
-    if ((e = cudaMalloc((void**)&h->d_p64, np * 16)) != cudaSuccess) return fail(e);
-    if ((e = cudaMalloc((void**)&h->d_p32, np * 8)) != cudaSuccess) return fail(e);
-    if ((e = cudaMalloc((void**)&h->d_d64, (size_t)h->nproj * h->nproj * 8)) != cudaSuccess) return fail(e);
-    if ((e = cudaMalloc((void**)&h->d_d32, (size_t)h->nproj * h->nproj * 4)) != cudaSuccess) return fail(e);
-    if ((e = alloc_columns(&h->d_cols, h->nproj)) != cudaSuccess) return fail(e);
+    if (!g_pool.alloc(device, (void**)&h->d_p64, np * 16)) return no_room();
+    if (!g_pool.alloc(device, (void**)&h->d_p32, np * 8)) return no_room();
+    if (!g_pool.alloc(device, (void**)&h->d_d64, (size_t)h->nproj * h->nproj * 8)) return no_room();
+    if (!g_pool.alloc(device, (void**)&h->d_d32, (size_t)h->nproj * h->nproj * 4)) return no_room();
+    if (!g_pool.alloc(device, (void**)&h->d_cols.cnt, (size_t)h->nproj * sizeof(int))) return no_room();
+    if (!g_pool.alloc(device, (void**)&h->d_cols.idx, (size_t)h->nproj * h->nproj * sizeof(int))) return no_room();
   }
-  scratch_handle(device, 1);
+  g_pool.handles(device, 1);
   h->counted = true;
   *out = h;
   return GWB_OK;
@@ -917,14 +855,14 @@ int gwb_ham_destroy(gwb_ham* h) {
     const bool idle = cudaGetDevice(&cur) == cudaSuccess && cudaSetDevice(h->device) == cudaSuccess &&
                       cudaDeviceSynchronize() == cudaSuccess;
     if (idle) {
-      scratch_give(h->device, h->d_W, h->W_bytes);
+      g_pool.give(h->device, h->d_W, h->W_bytes);
       h->d_W = nullptr;
     } else {
       cudaGetLastError();
     }
     cudaSetDevice(cur);
   }
-  if (h->counted) scratch_handle(h->device, -1);
+  if (h->counted) g_pool.handles(h->device, -1);
   void* ptrs[] = {h->d_npw, h->d_map, h->d_rowof, h->d_dup, h->d_t64, h->d_t32, h->d_v64,
                   h->d_v32, h->d_p64, h->d_p32, h->d_d64, h->d_d32, h->d_q64, h->d_q32, h->d_cols.cnt, h->d_cols.idx,
                   h->q_cols.cnt, h->q_cols.idx, h->d_W, h->d_part, h->d_bd, h->d_bq,
@@ -1045,9 +983,11 @@ int gwb_ham_set_overlap(gwb_ham* h, const double* q, void* stream) {
   cudaStream_t st = (cudaStream_t)stream;
   const size_t nd = (size_t)h->nproj * h->nproj;
   if (!h->d_q64) {
-    GWB_CUDA_TRY(cudaMalloc((void**)&h->d_q64, nd * 8));
-    GWB_CUDA_TRY(cudaMalloc((void**)&h->d_q32, nd * 4));
-    GWB_CUDA_TRY(alloc_columns(&h->q_cols, h->nproj));
+    auto alloc = [&](void** p, size_t bytes) { return g_pool.alloc(h->device, p, bytes) ? cudaSuccess : cudaErrorMemoryAllocation; };
+    GWB_CUDA_TRY(alloc((void**)&h->d_q64, nd * 8));
+    GWB_CUDA_TRY(alloc((void**)&h->d_q32, nd * 4));
+    GWB_CUDA_TRY(alloc((void**)&h->q_cols.cnt, (size_t)h->nproj * sizeof(int)));
+    GWB_CUDA_TRY(alloc((void**)&h->q_cols.idx, nd * sizeof(int)));
   }
   GWB_CUDA_TRY(cudaMemcpyAsync(h->d_q64, q, nd * 8, cudaMemcpyDeviceToDevice, st));
   k_scale_copy<float><<<blocks_for(nd, 256), 256, 0, st>>>(q, h->d_q32, nd, 1.0);

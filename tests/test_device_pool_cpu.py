@@ -1,0 +1,89 @@
+"""The bookkeeping of device memory (csrc/device_pool.cuh) against a fake allocator of 100 bytes."""
+
+import shutil
+import subprocess
+from pathlib import Path
+
+import pytest
+
+CSRC = Path(__file__).resolve().parents[1] / "gradwave_b200" / "csrc"
+
+FAKE = """
+#include <cassert>
+#include <cstdio>
+#include <cstdlib>
+#include <map>
+#include "device_pool.cuh"
+
+struct Fake {
+  static inline std::map<void*, size_t> live;
+  static inline size_t room = 100;
+  static inline int calls = 0;
+  static bool alloc(void** p, size_t n) {
+    ++calls;
+    if (n > room) return false;
+    *p = std::malloc(1);
+    live[*p] = n;
+    room -= n;
+    return true;
+  }
+  static void free(void* p) {
+    assert(live.count(p));
+    room += live[p];
+    live.erase(p);
+    std::free(p);
+  }
+};
+using Pool = gwb::DevicePool<Fake>;
+#define CHECK(x) if (!(x)) { std::printf("line %d: %s\\n", __LINE__, #x); return 1; }
+"""
+
+KEPT = """
+int main() {
+  Pool pool;
+  void *w = nullptr, *p = nullptr, *q = nullptr;
+  size_t n = 0, have = 0;
+  pool.handles(0, 2);
+  CHECK(pool.ensure(0, &w, &have, 60) && Fake::room == 40);
+  pool.give(0, w, have);                       // a destroyed handle's scratch stays ...
+  CHECK(Fake::room == 40);
+  CHECK(!pool.take(0, 61, &n) && !pool.take(1, 1, &n));
+  CHECK(pool.alloc(0, &p, 30) && Fake::room == 10);
+  CHECK(pool.alloc(0, &q, 50) && Fake::room == 20);   // ... until any allocation needs its room
+  CHECK(!pool.take(0, 0, &n));
+  void* r = &n;
+  CHECK(!pool.alloc(0, &r, 21) && r == nullptr && Fake::room == 20);
+  have = 30;
+  CHECK(!pool.ensure(0, &p, &have, 60) && p == nullptr && have == 0);
+  CHECK(pool.ensure(0, &p, &have, 40) && have == 40);
+  pool.give(0, p, 40);
+  pool.give(0, q, 50);                         // the larger of two stays
+  CHECK(Fake::room == 50 && pool.take(0, 50, &n) == q && n == 50);
+  pool.give(0, q, 50);
+  pool.handles(0, -1);
+  CHECK(Fake::room == 50);
+  pool.handles(0, -1);                         // the last handle takes it along
+  CHECK(Fake::room == 100 && Fake::live.empty());
+  return 0;
+}
+"""
+
+
+def _run(tmp_path, main):
+    cxx = shutil.which("g++")
+    if cxx is None:
+        pytest.skip("no g++")
+    (tmp_path / "t.cpp").write_text(FAKE + main)
+    subprocess.run([cxx, "-std=c++17", "-I", str(CSRC), "-o", str(tmp_path / "t"), str(tmp_path / "t.cpp"), "-pthread"], check=True)
+    run = subprocess.run([str(tmp_path / "t")], capture_output=True, text=True)
+    assert run.returncode == 0, run.stdout + run.stderr
+
+
+def test_kept_scratch_is_given_back(tmp_path):
+    _run(tmp_path, KEPT)
+
+
+def test_every_allocation_of_a_handle_uses_the_pool():
+    """No handle allocates past the pool: cudaMalloc is called in its Api alone."""
+    for src in sorted(CSRC.glob("*.cu*")):
+        assert src.read_text().count("cudaMalloc(") == (src.name == "ham_apply.cu"), src.name
