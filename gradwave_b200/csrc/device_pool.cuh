@@ -65,6 +65,20 @@ template <class Api> class DevicePool {
     return false;
   }
 
+  // All of the (pointer, bytes) buffers, or none: those made before a failure are freed, all pointers null.
+  bool alloc_all(int dev, std::initializer_list<std::pair<void**, size_t>> bufs) {
+    for (const auto& b : bufs) *b.first = nullptr;
+    for (const auto& b : bufs)
+      if (!alloc(dev, b.first, b.second)) {
+        for (const auto& c : bufs) {
+          if (*c.first) Api::free(*c.first);
+          *c.first = nullptr;
+        }
+        return false;
+      }
+    return true;
+  }
+
   // *p of at least need bytes; what it held is lost when it has to grow.
   bool ensure(int dev, void** p, size_t* have, size_t need) {
     if (*have >= need) return true;

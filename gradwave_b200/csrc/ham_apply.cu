@@ -983,11 +983,14 @@ int gwb_ham_set_overlap(gwb_ham* h, const double* q, void* stream) {
   cudaStream_t st = (cudaStream_t)stream;
   const size_t nd = (size_t)h->nproj * h->nproj;
   if (!h->d_q64) {
-    auto alloc = [&](void** p, size_t bytes) { return g_pool.alloc(h->device, p, bytes) ? cudaSuccess : cudaErrorMemoryAllocation; };
-    GWB_CUDA_TRY(alloc((void**)&h->d_q64, nd * 8));
-    GWB_CUDA_TRY(alloc((void**)&h->d_q32, nd * 4));
-    GWB_CUDA_TRY(alloc((void**)&h->q_cols.cnt, (size_t)h->nproj * sizeof(int)));
-    GWB_CUDA_TRY(alloc((void**)&h->q_cols.idx, nd * sizeof(int)));
+    // all of the tables or none: a later call must not find some of them
+    if (!g_pool.alloc_all(h->device, {{(void**)&h->d_q64, nd * 8},
+                                      {(void**)&h->d_q32, nd * 4},
+                                      {(void**)&h->q_cols.cnt, (size_t)h->nproj * sizeof(int)},
+                                      {(void**)&h->q_cols.idx, nd * sizeof(int)}})) {
+      set_error("device allocation of the overlap tables failed");
+      return GWB_ERR_CUDA;
+    }
   }
   GWB_CUDA_TRY(cudaMemcpyAsync(h->d_q64, q, nd * 8, cudaMemcpyDeviceToDevice, st));
   k_scale_copy<float><<<blocks_for(nd, 256), 256, 0, st>>>(q, h->d_q32, nd, 1.0);

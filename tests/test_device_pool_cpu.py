@@ -68,6 +68,17 @@ int main() {
 }
 """
 
+ALL_OR_NONE = """
+int main() {
+  Pool pool;
+  void *a = nullptr, *b = nullptr, *c = nullptr;
+  CHECK(!pool.alloc_all(0, {{&a, 40}, {&b, 40}, {&c, 40}}));
+  CHECK(!a && !b && !c && Fake::room == 100 && Fake::live.empty());
+  CHECK(pool.alloc_all(0, {{&a, 40}, {&b, 40}, {&c, 20}}) && a && b && c && Fake::room == 0);
+  return 0;
+}
+"""
+
 
 def _run(tmp_path, main):
     cxx = shutil.which("g++")
@@ -81,6 +92,12 @@ def _run(tmp_path, main):
 
 def test_kept_scratch_is_given_back(tmp_path):
     _run(tmp_path, KEPT)
+
+
+def test_tables_of_a_set_come_all_or_none(tmp_path):
+    """gwb_ham_set_overlap tells by its first table whether it has them: a set that a failure left incomplete would
+    send the next call to a null one."""
+    _run(tmp_path, ALL_OR_NONE)
 
 
 def test_every_allocation_of_a_handle_uses_the_pool():
