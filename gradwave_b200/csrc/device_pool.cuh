@@ -2,13 +2,22 @@
 // bool alloc(void**, size_t) and void free(void*).
 #pragma once
 
+#include <algorithm>
 #include <cstddef>
+#include <cstdint>
 #include <initializer_list>
 #include <map>
 #include <mutex>
 #include <utility>
 
 namespace gwb {
+
+// Scratch of a chunk of bands.
+struct ChunkScratch {
+  void* p = nullptr;
+  size_t bytes = 0;
+  size_t denied = SIZE_MAX;  // the least size that could not be had
+};
 
 // Every allocation of a handle goes through a pool. The band-chunk scratch of a
 // destroyed handle waits there for the next handle on the device (mapping half a
@@ -87,6 +96,39 @@ template <class Api> class DevicePool {
     if (!alloc(dev, p, need)) return false;
     *have = need;
     return true;
+  }
+
+  // Bands per chunk, with scratch for one in w: as few chunks as the budget
+  // allows, all of (nearly) equal size; where the device has no room for that,
+  // chunks of the low budget or of what w held. 0: no room at all. A size that
+  // was refused is not asked for again: every call would give up its scratch and
+  // map it anew (and could not be captured).
+  int chunk(int dev, ChunkScratch& w, int nb, size_t per_band, size_t budget, size_t low) {
+    const size_t had = w.bytes;
+    auto bands = [&](size_t bytes) {
+      const size_t most = std::min<size_t>(32768, std::max<size_t>(1, bytes / per_band));  // bands are a grid axis
+      const size_t nchunks = ((size_t)nb + most - 1) / most;
+      return (int)(((size_t)nb + nchunks - 1) / nchunks);
+    };
+    auto fits = [&](size_t need) {
+      if (w.bytes >= need) return true;
+      size_t n = 0;
+      if (void* p = take(dev, need, &n)) {
+        if (w.p) Api::free(w.p);
+        w.p = p;
+        w.bytes = n;
+        return true;
+      }
+      return ensure(dev, &w.p, &w.bytes, need);
+    };
+    int n = bands(budget);
+    if (per_band * n <= w.bytes) return n;
+    if (per_band * n < w.denied) {
+      if (fits(per_band * n)) return n;
+      w.denied = per_band * n;
+    }
+    n = std::min(n, bands(std::max(low, had)));
+    return fits(per_band * n) ? n : 0;
   }
 
  private:

@@ -68,8 +68,7 @@ struct gwb_ham {
   gwb::cplx<double>* d_tw64[3] = {nullptr, nullptr, nullptr};
   gwb::cplx<float>* d_tw32[3] = {nullptr, nullptr, nullptr};
   // scratch
-  void* d_W = nullptr;  // planes of a band chunk, then its rows
-  size_t W_bytes = 0;
+  gwb::ChunkScratch W;   // planes of a band chunk, then its rows
   bool counted = false;  // among its device's live handles (gwb_ham_create completed)
   void* d_part = nullptr;  // becp partials
   size_t part_bytes = 0;
@@ -431,35 +430,15 @@ static int nl_slices(const gwb_ham* h, int nb) {
   return std::max(1, std::min(want, cap));
 }
 
-// Bands per chunk and the chunk's scratch (W: L0 planes, W2: the disc's rows):
-// as few chunks as the budget allows, all of (nearly) equal size. When the
-// device has no room for that scratch, chunks of kWBudgetLowMB.
+// Bands per chunk and the chunk's scratch (W: L0 planes, W2: the disc's rows).
 static int chunk_scratch(gwb_ham* h, int nb, size_t es, int* nbc) {
   const FftGeom& g = h->g;
   const size_t per_band = (size_t)h->nk * ((size_t)g.L[0] * g.n[1] + g.nrow) * g.n[2] * es;
-  auto ensure = [&](size_t need) {
-    if (h->W_bytes >= need) return GWB_OK;
-    if (void* p = g_pool.take(h->device, need, &need)) {
-      if (h->d_W) cudaFree(h->d_W);
-      h->d_W = p;
-      h->W_bytes = need;
-      return GWB_OK;
-    }
-    return ensure_buf(h, &h->d_W, &h->W_bytes, need);
-  };
-  auto bands = [&](size_t budget) {
-    const size_t most = std::min<size_t>(32768, std::max<size_t>(1, budget / per_band));  // bands are a grid axis
-    const size_t nchunks = ((size_t)nb + most - 1) / most;
-    return (int)(((size_t)nb + nchunks - 1) / nchunks);
-  };
-  *nbc = bands(h->w_budget ? h->w_budget : w_budget_bytes());
-  int rc = ensure(per_band * *nbc);
-  const int low = bands((size_t)kWBudgetLowMB << 20);
-  if (rc == GWB_ERR_ALLOC && low < *nbc) {
-    *nbc = low;
-    rc = ensure(per_band * *nbc);
-  }
-  return rc;
+  *nbc = g_pool.chunk(h->device, h->W, nb, per_band, h->w_budget ? h->w_budget : w_budget_bytes(),
+                      (size_t)kWBudgetLowMB << 20);
+  if (*nbc) return GWB_OK;
+  set_error("no device memory for the scratch of one band (" + std::to_string(per_band) + " bytes)");
+  return GWB_ERR_ALLOC;
 }
 
 template <typename T> static FftRun<T> fft_run(const gwb_ham* h, int nbc) {
@@ -475,7 +454,7 @@ template <typename T> static FftRun<T> fft_run(const gwb_ham* h, int nbc) {
   f.tw2 = dbl ? (const cplx<T>*)h->d_tw64[2] : (const cplx<T>*)h->d_tw32[2];
   f.v = dbl ? (const T*)h->d_v64 : (const T*)h->d_v32;
   f.t = dbl ? (const T*)h->d_t64 : (const T*)h->d_t32;
-  f.W = (cplx<T>*)h->d_W;
+  f.W = (cplx<T>*)h->W.p;
   return f;
 }
 
@@ -849,14 +828,14 @@ int gwb_ham_create(const gwb_ham_geometry* geom, int device, gwb_ham** out) {
 
 int gwb_ham_destroy(gwb_ham* h) {
   if (!h) return GWB_OK;
-  if (h->d_W) {
+  if (h->W.p) {
     // the scratch may serve the next handle once nothing in flight uses it
     int cur = 0;
     const bool idle = cudaGetDevice(&cur) == cudaSuccess && cudaSetDevice(h->device) == cudaSuccess &&
                       cudaDeviceSynchronize() == cudaSuccess;
     if (idle) {
-      g_pool.give(h->device, h->d_W, h->W_bytes);
-      h->d_W = nullptr;
+      g_pool.give(h->device, h->W.p, h->W.bytes);
+      h->W = {};
     } else {
       cudaGetLastError();
     }
@@ -865,7 +844,7 @@ int gwb_ham_destroy(gwb_ham* h) {
   if (h->counted) g_pool.handles(h->device, -1);
   void* ptrs[] = {h->d_npw, h->d_map, h->d_rowof, h->d_dup, h->d_t64, h->d_t32, h->d_v64,
                   h->d_v32, h->d_p64, h->d_p32, h->d_d64, h->d_d32, h->d_q64, h->d_q32, h->d_cols.cnt, h->d_cols.idx,
-                  h->q_cols.cnt, h->q_cols.idx, h->d_W, h->d_part, h->d_bd, h->d_bq,
+                  h->q_cols.cnt, h->q_cols.idx, h->W.p, h->d_part, h->d_bd, h->d_bq,
                   h->d_pplanes, h->d_cplanes, h->d_becp, h->d_bdplanes, h->d_tcwork, h->d_tcstatus, h->d_rhok,
                   h->d_tw64[0], h->d_tw64[1], h->d_tw64[2], h->d_tw32[0], h->d_tw32[1], h->d_tw32[2]};
   for (void* p : ptrs)
@@ -960,6 +939,7 @@ int gwb_ham_set_tuning(gwb_ham* h, int64_t w_budget_bytes, int32_t nl_target_cta
   GWB_REQUIRE(h, "null handle");
   GWB_REQUIRE(w_budget_bytes >= 0 && nl_target_ctas >= 0, "tuning values must be >= 0");
   h->w_budget = (size_t)w_budget_bytes;
+  h->W.denied = SIZE_MAX;
   h->nl_target = nl_target_ctas;
   return GWB_OK;
 }
@@ -1043,7 +1023,7 @@ int gwb_ham_density(gwb_ham* h, const void* c, int64_t c_kstride, int32_t nb, in
 }
 
 size_t gwb_ham_scratch_bytes(const gwb_ham* h) {
-  return h ? h->W_bytes + h->part_bytes + h->bd_bytes + h->bq_bytes + h->pplanes_bytes + h->cplanes_bytes + h->becp_bytes +
+  return h ? h->W.bytes + h->part_bytes + h->bd_bytes + h->bq_bytes + h->pplanes_bytes + h->cplanes_bytes + h->becp_bytes +
                  h->bdplanes_bytes + h->tcwork_bytes + h->rhok_bytes
            : 0;
 }

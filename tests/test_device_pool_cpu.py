@@ -79,6 +79,32 @@ int main() {
 }
 """
 
+CHUNKS = """
+int main() {
+  Pool pool;
+  gwb::ChunkScratch w;
+  size_t n = 0;
+  CHECK(pool.chunk(0, w, 7, 10, 40, 20) == 4 && w.bytes == 40);      // two chunks of 4 and 3
+  CHECK(pool.chunk(0, w, 100, 10, 5, 2) == 1 && w.bytes == 40);      // one band at least
+  CHECK(pool.chunk(0, w, 30, 10, 300, 20) == 4 && w.bytes == 40);    // no room for 300: what it held
+  const int calls = Fake::calls;
+  for (int i = 0; i < 3; ++i) CHECK(pool.chunk(0, w, 30, 10, 300, 20) == 4);
+  CHECK(Fake::calls == calls);                                       // and no further attempt
+  CHECK(pool.chunk(0, w, 6, 10, 300, 20) == 6 && w.bytes == 60);     // a smaller one may be had
+  CHECK(pool.chunk(0, w, 30, 10, 300, 20) == 6 && w.bytes == 60);
+  gwb::ChunkScratch v;
+  CHECK(pool.chunk(0, v, 30, 10, 300, 20) == 2 && v.bytes == 20);    // the low budget
+  gwb::ChunkScratch u;
+  CHECK(pool.chunk(0, u, 30, 21, 300, 20) == 0 && !u.p && u.bytes == 0);
+  Fake::free(v.p);
+  CHECK(pool.chunk(0, u, 30, 21, 300, 20) == 1 && u.bytes == 21);    // asked for again
+  pool.handles(0, 1);
+  pool.give(0, w.p, w.bytes);
+  CHECK(pool.chunk(0, u, 3, 20, 300, 20) == 3 && u.bytes == 60 && Fake::room == 40);   // a kept buffer taken over
+  return 0;
+}
+"""
+
 
 def _run(tmp_path, main):
     cxx = shutil.which("g++")
@@ -98,6 +124,10 @@ def test_tables_of_a_set_come_all_or_none(tmp_path):
     """gwb_ham_set_overlap tells by its first table whether it has them: a set that a failure left incomplete would
     send the next call to a null one."""
     _run(tmp_path, ALL_OR_NONE)
+
+
+def test_chunks_when_memory_is_short(tmp_path):
+    _run(tmp_path, CHUNKS)
 
 
 def test_every_allocation_of_a_handle_uses_the_pool():

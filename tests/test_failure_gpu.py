@@ -140,3 +140,37 @@ def test_refused_launch_is_reported_once(cuda_device):
     torch.cuda.synchronize()
     _lib.call("gwb_ham_set_potential", h._h, v.data_ptr(), _lib.stream_ptr())
     assert float((h.apply_fp32(c) - c).abs().max()) < 1e-5   # v = 1: H c = c
+
+
+def test_capture_when_the_scratch_budget_cannot_be_had(cuda_device):
+    """A budget beyond the device's memory (214 GB for 400 bands of 16 k in a 128^3 box): smaller chunks, and after
+    a first apply none that allocates, so that the next one can be captured."""
+    from gradwave_b200 import _lib
+    from gradwave_b200.basis import BatchedK
+    from gradwave_b200.hamiltonian import BatchedHamiltonian
+    nk, nb, n = 16, 400, 128
+    bk = BatchedK(torch.full((nk,), 2), torch.ones(nk, 2, dtype=torch.bool), torch.tensor([[0, 64 * n * n]] * nk),
+                  torch.zeros(nk, 2, 3, dtype=torch.float64), torch.ones(nk, 2, dtype=torch.float64),
+                  torch.zeros(0, dtype=torch.complex128), torch.zeros(0, dtype=torch.int64),
+                  torch.zeros(0, 0, dtype=torch.float64)).to(cuda_device)
+    h = BatchedHamiltonian(bk, (n, n, n), torch.full((n, n, n), 3.0, dtype=torch.float64, device=cuda_device),
+                           torch.zeros(nk, 0, 2, dtype=torch.complex128, device=cuda_device))
+    _lib.call("gwb_ham_set_tuning", h._h, 1 << 40, 0)
+    g = torch.Generator().manual_seed(1)
+    c = torch.randn(nk, nb, 2, dtype=torch.complex128, generator=g).to(cuda_device)
+    out = torch.zeros_like(c)
+
+    def apply():
+        _lib.call("gwb_ham_apply", h._h, c.data_ptr(), out.data_ptr(), nb, _lib.GWB_C128, _lib.GWB_FP64, _lib.stream_ptr())
+
+    apply()
+    torch.cuda.synchronize()
+    assert float((out - 4.0 * c).abs().max()) < 1e-13
+    assert h.scratch_bytes() < 1 << 30
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        apply()
+    c.mul_(-1.0)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert float((out - 4.0 * c).abs().max()) < 1e-13
