@@ -101,6 +101,7 @@ __global__ void k_zgemm_nh_reduce(int M, int N, int nslice, int batch, const cpl
   const int64_t total = (int64_t)batch * M * N;
   chain_wait();
   part = after_wait(part);
+  C = after_wait(C);
   for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
        idx += (int64_t)gridDim.x * blockDim.x) {
     const int b = (int)(idx / ((int64_t)M * N));

@@ -131,8 +131,10 @@ inline cudaError_t launch_chained(void (*kern)(P...), dim3 grid, unsigned thread
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
-// A pointer whose loads the compiler cannot move above this point (reads
-// through __restrict__ pointers may otherwise cross the wait).
+// A pointer whose loads the compiler cannot move above this point: reads through
+// __restrict__ pointers may otherwise cross the wait. Every such pointer that a
+// kernel before may have written goes through it; the tables and projectors of
+// an operator handle do not (the local term's kernels lie between).
 template <typename T> __device__ __forceinline__ T* after_wait(T* p) {
   asm volatile("" : "+l"(p)::"memory");
   return p;

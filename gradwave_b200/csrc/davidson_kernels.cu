@@ -133,6 +133,7 @@ __global__ void __launch_bounds__(256) k_precond_teter(int npw, int nb, int n_ad
   chain_wait();
   x = after_wait(x);
   r = after_wait(r);
+  t = after_wait(t);
   sel = after_wait(sel);
   const int k = blockIdx.x / n_add, s = blockIdx.x % n_add;
   const int b = sel[(int64_t)k * n_add + s];
@@ -322,6 +323,7 @@ __global__ void __launch_bounds__(256) k_row_repair(int npw, int n, cplx<double>
   __shared__ double red[8];
   chain_wait();
   D = after_wait(D);
+  mask = after_wait(mask);
   const int k = blockIdx.x / n, s = blockIdx.x % n;
   cplx<double>* row = D + k * dk + (int64_t)s * npw;
   double nn = 0.0;

@@ -38,6 +38,8 @@ __global__ void k_gamma_pack(int nb, int nphi, int npw, const double* __restrict
   const int64_t total = (int64_t)npair * npw;
   chain_wait();
   phi = after_wait(phi);
+  src_half = after_wait(src_half);
+  conj_full = after_wait(conj_full);
   for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
        idx += (int64_t)gridDim.x * blockDim.x) {
     const int p = (int)(idx / npw), g = (int)(idx % npw);
@@ -62,6 +64,8 @@ __global__ void k_gamma_unpack(int nb, int nhalf, int npw, const cplx<double>* _
   const int64_t total = (int64_t)npair * nhalf;
   chain_wait();
   hz = after_wait(hz);
+  rep_full = after_wait(rep_full);
+  partner_rep = after_wait(partner_rep);
   for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
        idx += (int64_t)gridDim.x * blockDim.x) {
     const int p = (int)(idx / nhalf), j = (int)(idx % nhalf);

@@ -266,6 +266,7 @@ __global__ void __launch_bounds__(256) k_nl_add(const cplx<T>* __restrict__ bd,
   const int gi_o = gt * TGO + lg;
   chain_wait();
   bd = after_wait(bd);
+  out = after_wait(out);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {  // the output rows first: their loads overlap the tile staging below
     const int b = bt * NL_TB + lb0 * 4 + i;
@@ -340,6 +341,8 @@ __global__ void __launch_bounds__(256) k_nl_add_hs(const cplx<T>* __restrict__ b
   chain_wait();
   bd = after_wait(bd);
   bq = after_wait(bq);
+  c = after_wait(c);
+  out_h = after_wait(out_h);  // without projectors the kernel just before this one wrote it
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int b = bt * NL_TB + lb0 * 4 + i;

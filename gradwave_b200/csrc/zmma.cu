@@ -59,6 +59,8 @@ __global__ void __launch_bounds__(ZN_TN * 4) k_zmma_nn(int nb, int N, int K, con
     cp_async_commit();
   };
   chain_wait();
+  c = after_wait(c);
+  out_h = after_wait(out_h);  // without projectors the kernel just before this one wrote it
 #pragma unroll
   for (int p = 0; p < ZM_STAGES - 1; ++p) load(p);
 

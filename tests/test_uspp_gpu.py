@@ -78,3 +78,31 @@ def test_fused_hs_apply(cuda_device, name):
     h32, s32 = hs.hs(c.to(torch.complex64))
     assert float((h32.to(torch.complex128) - h_ref).abs().max()) <= 3e-6 * scale
     assert np.abs(s32.cpu().numpy() - s_ref).max() <= 3e-6 * np.abs(s_ref).max()
+
+
+@pytest.mark.parametrize("dtype", [torch.complex128, torch.complex64])
+def test_fused_hs_apply_without_projectors(cuda_device, dtype):
+    """No projectors: H c is the plain apply, S c the masked block; many small applies in a row, so that the kernel
+    that copies c runs close behind the local term's last one."""
+    from gradwave_b200.basis import BatchedK
+    from gradwave_b200.hamiltonian import BatchedHamiltonian
+    from gradwave_b200.uspp import BatchedHS
+    npw, nb, n = [300, 211], 70, 12
+    g = torch.Generator().manual_seed(3)
+    mask = torch.zeros(2, 300, dtype=torch.bool)
+    flat = torch.zeros(2, 300, dtype=torch.int64)
+    for k in range(2):
+        mask[k, :npw[k]] = True
+        flat[k, :npw[k]] = torch.randperm(n ** 3, generator=g)[:npw[k]]
+    bk = BatchedK(torch.tensor(npw), mask, flat, torch.zeros(2, 300, 3, dtype=torch.float64),
+                  torch.rand(2, 300, dtype=torch.float64, generator=g) * mask, torch.zeros(0, dtype=torch.complex128),
+                  torch.zeros(0, dtype=torch.int64), torch.zeros(0, 0, dtype=torch.float64)).to(cuda_device)
+    v = torch.randn(n, n, n, dtype=torch.float64, generator=g).to(cuda_device)
+    p = torch.zeros(2, 0, 300, dtype=torch.complex128, device=cuda_device)
+    hs = BatchedHS(bk, (n, n, n), v, p, bk.dij_full, bk.dij_full)
+    c = torch.randn(2, nb, 300, dtype=torch.complex128, generator=g).to(cuda_device).to(dtype)
+    ref = BatchedHamiltonian(bk, (n, n, n), v, p).apply(c)
+    for _ in range(20):
+        h, s = hs.hs(c)
+        assert torch.equal(h, ref)
+        assert torch.equal(s, c * bk.mask[:, None, :])
