@@ -107,8 +107,9 @@ namespace gwb {
 
 // Noise on the first expansion rows of a cold start (gwb_start_noise): norm, and
 // the largest residual [eV] above which a start counts as cold. The host driver
-// has the same (davidson.py, break_symmetry, with the reasons).
-constexpr double kStartNoise = 0.25, kColdStartEv = 1.0;
+// has the same for bases of this size (davidson.py, break_symmetry, with the
+// reasons).
+constexpr double kStartNoise = 0.02, kColdStartEv = 1.0;
 
 struct Buf {
   size_t off = 0;

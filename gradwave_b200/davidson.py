@@ -65,8 +65,9 @@ logger = logging.getLogger(__name__)
 _FP32_CERT_FLOOR_EPS = 32 * torch.finfo(torch.float32).eps
 _FP32_CERT_STALL = 0.7
 # norm of the noise on the unit rows of the first expansion of a cold start
-# (largest residual of a k-point above _COLD_START_EV)
-_START_NOISE = 0.25
+# (largest residual of a k-point above _COLD_START_EV): bases within the batched
+# eigensolver's limit, and beyond (break_symmetry)
+_START_NOISE, _START_NOISE_LARGE = 0.02, 0.25
 _COLD_START_EV = 1.0
 _N, _T, _H = 0, 1, 2
 
@@ -617,18 +618,24 @@ class _Solver:
         but round-off: such a level shows up only after round-off has grown to
         the size of a Ritz vector, and a solve that converges before skips it.
         Noise of the order of the rows themselves lets it converge with the
-        others. Perfect 2- and 8-atom cells, 6 to 40 bands, identity starts
-        1e-15 apart, float64 and mixed, both preconditioners: 21 of 864 solves
-        skip a level without it (0.2 to 5 eV), none with norms 0.05, 0.25 and
-        0.7; mean rounds 47, 47, 49 and 48. The perfect 64-atom cell: 6 of 8
-        without (float64), none of 24 with it (rounds, float64 / mixed / mixed
-        with the network: 51-57, 50-77, 39-40).
+        others: it must come up before they reach the tolerance, so 3e-6 is
+        enough at 1e-10 eV, and 0.02 down to 4e-3 eV.
+
+        Perfect 2- and 8-atom cells, 6 to 40 bands, identity starts 1e-15
+        apart, float64 and mixed, both preconditioners: 21 of 864 solves skip
+        a level without noise (0.2 to 5 eV), none of 4896 with norms from 3e-6
+        to 0.7; mean rounds 47 without, 46 to 49 with it. What the norm costs
+        in rounds is another matter. Displaced 8-atom cells, 24 bands (TPA /
+        network): 54 / 35 without, 51 / 35 at 0.02, 57 / 44 at 0.25. Perfect
+        64-atom cell, 160 bands, six starts (TPA / mixed / mixed with the
+        network): 75-204 / 83-300 / 38 at 0.02, 51-57 / 50-77 / 39-40 at 0.25.
 
         The noise is a function of row and plane wave alone, so that a k-point
         is solved alike in whatever group or shard it is."""
         ws, npw = self.ws, self.npw
         _lib.call("gwb_start_noise", self.nk, n_add, npw, _ptr(ws.D), ws.D.shape[1] * npw, _ptr(self.mask_u8),
-                  _ptr(ws.rn), self.nb, _COLD_START_EV, _START_NOISE, self.stream)
+                  _ptr(ws.rn), self.nb, _COLD_START_EV,
+                  _START_NOISE if self.max_dim <= self.heev_max else _START_NOISE_LARGE, self.stream)
 
     def precondition(self, n_add: int, eig: torch.Tensor):
         """D[:, :n_add] = preconditioned, unit-normalised worst residuals."""
