@@ -216,8 +216,8 @@ cudaError_t zmma_nn(int nb, int N, int K, const cplx<double>* A, const cplx<doub
   const dim3 grid((unsigned)((N + ZN_TN - 1) / ZN_TN), (unsigned)((rows + TM - 1) / TM), batch);
 #define GWB_ZN_CASE(tm)                                                                                            \
   if (TM == tm) {                                                                                                  \
-    auto* kern = A2 ? (uncut ? k_zmma_nn<tm, true, 0> : k_zmma_nn<tm, true, ZM_CHAIN>)                             \
-                    : (uncut ? k_zmma_nn<tm, false, 0> : k_zmma_nn<tm, false, ZM_CHAIN>);                          \
+    auto* kern = A2 ? (uncut ? k_zmma_nn<tm, true, 0> : k_zmma_nn<tm, true, 1>)                             \
+                    : (uncut ? k_zmma_nn<tm, false, 0> : k_zmma_nn<tm, false, 1>);                          \
     return launch_chained(kern, grid, ZN_TN * 4, zmma_nn_smem<tm>(), st, nb, N, K, A, A2, P, c, ck, out_h, hk,     \
                           out_s, sk, npw_k);                                                                       \
   }

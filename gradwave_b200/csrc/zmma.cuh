@@ -26,8 +26,9 @@
 // 1.9e-16; 64 x 512 x 640: 12, 3.3, 6.0), after ZM_CHAIN in k_zmma_nh (24 x 24 x
 // 100: 4.8e-16 with chains of 128 terms, 2.8e-16, FMA pipe 3.5e-16). The update is
 // summed apart from the row it is added to, uncut up to ZM_UNCUT projectors (256:
-// 8.3e-16, FMA pipe 9.2e-16; 864: 14 uncut, 4.4, 12); beyond, the second set of
-// sums costs registers and a block per SM (5 % of a 64-atom apply at 256).
+// 8.3e-16, FMA pipe 9.2e-16; 512: 11 uncut, 3.7, 10; 864: 14, 4.3, 12); beyond, a
+// cut per K step costs 5 % of an apply (400 projectors, 98 bands: 1051 -> 1112 us;
+// per two steps 1137, whose live chains take a block per SM).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -51,8 +52,8 @@ __device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
 
 constexpr int ZM_K = 8;       // K step
 constexpr int ZM_STAGES = 3;  // steps in flight
-constexpr int ZM_CHAIN = 4;   // steps in one chain of the long products
-constexpr int ZM_UNCUT = 256;  // longest update summed in one chain
+constexpr int ZM_CHAIN = 4;   // steps in one chain of k_zmma_nh
+constexpr int ZM_UNCUT = 320;  // longest update summed in one chain
 
 // Sums of a warp's 8 MT x 8 tile in chains of CHAIN steps (0: one chain): lane l
 // holds rows 8 t + l / 4, columns 2 (l % 4) + {0, 1}.
