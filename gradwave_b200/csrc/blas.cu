@@ -59,6 +59,7 @@ extern "C" int gwb_zgemm(int opA, int opB, int64_t M, int64_t N, int64_t K, doub
   // and Ritz vectors of small blocks): own tiles, launched in chain; cuBLAS for
   // the rest, whose larger tiles load less
   if (opB == 0 && opA <= 1 && M <= kShortRows && N >= 8 * M && K > 0 && batch <= 65535) {
+    GWB_REQUIRE(lda >= (opA ? M : K) && ldb >= N && ldc >= N, "leading dimension smaller than a row");  // as cuBLAS
     GWB_CUDA_TRY(zmma_ab(opA == 1, (int)M, (int)N, (int)K, mk<double>(alpha_re, alpha_im), (const cplx<double>*)A, lda,
                          strideA, (const cplx<double>*)B, ldb, strideB, mk<double>(beta_re, beta_im), (cplx<double>*)C,
                          ldc, strideC, (int)batch, (cudaStream_t)stream));

@@ -171,3 +171,14 @@ def test_new_switches_and_gamma_preconditioner_refuse_bad_arguments():
         _lib.call("gwb_precond_learned_gamma", p, 8, 4, nhalf, 2 * nhalf, p, 2 * nhalf, p, 2 * nhalf, p, p, p,
                   None, p, 2 * nhalf, p, need - 8, None)
     assert ex.value.status == _lib.GWB_ERR_ARG
+
+
+@pytest.mark.parametrize("op,lda,ldb,ldc", [(0, 9, 200, 200), (1, 7, 200, 200), (0, 10, 199, 200), (0, 10, 200, 199)])
+def test_short_products_refuse_short_rows(op, lda, ldb, ldc):
+    """op(A) 8 x 10 times B 10 x 200: rows that overlap are refused before anything is launched, as cuBLAS refuses
+    them for the other products."""
+    from gradwave_b200 import _lib
+    p = 1 << 20   # never read
+    with pytest.raises(_lib.GwbError) as e:
+        _lib.call("gwb_zgemm", op, 0, 8, 200, 10, 1.0, 0.0, p, lda, 0, p, ldb, 0, 0.0, 0.0, p, ldc, 0, 1, 0)
+    assert e.value.status == _lib.GWB_ERR_ARG
