@@ -79,6 +79,15 @@ def density_from_handle(handle, nk: int, npw_max: int, shape, coeffs: torch.Tens
     return rho
 
 
+def _reference(bk, key):
+    """bk by a call, as long as it lives: the handle (and its scratch) goes with it. A bk that takes no weak
+    reference (named tuple, slots) is kept instead, and its handle with it."""
+    try:
+        return weakref.ref(bk, lambda _: _HANDLES.pop(key, None))
+    except TypeError:
+        return lambda: bk
+
+
 def density_b(coeffs: torch.Tensor, occ: torch.Tensor, kweights: torch.Tensor, bk, shape, volume: float
               ) -> torch.Tensor:
     """rho(r) on the dense grid [e/A^3], the reference's ``density_b``
@@ -88,8 +97,7 @@ def density_b(coeffs: torch.Tensor, occ: torch.Tensor, kweights: torch.Tensor, b
     key = (id(bk), tuple(int(s) for s in shape), dev.index)
     h = _HANDLES.get(key)
     if h is None or h[1]() is not bk:
-        # the handle (and its scratch) goes when bk does
-        h = (_GeometryHandle(bk, shape, dev), weakref.ref(bk, lambda _, key=key: _HANDLES.pop(key, None)))
+        h = (_GeometryHandle(bk, shape, dev), _reference(bk, key))
         _HANDLES[key] = h
     g = h[0]
     return density_from_handle(g._h, g.nk, g.npw_max, g.shape, coeffs, occ, kweights, volume)

@@ -182,3 +182,31 @@ def test_short_products_refuse_short_rows(op, lda, ldb, ldc):
     with pytest.raises(_lib.GwbError) as e:
         _lib.call("gwb_zgemm", op, 0, 8, 200, 10, 1.0, 0.0, p, lda, 0, p, ldb, 0, 0.0, 0.0, p, ldc, 0, 1, 0)
     assert e.value.status == _lib.GWB_ERR_ARG
+
+
+def test_density_handles_of_any_batch(monkeypatch):
+    """``density_b`` keeps one handle per batch object: one that takes no weak reference (a named tuple) is accepted
+    too, and the handle of one that does goes with it."""
+    from collections import namedtuple
+    from types import SimpleNamespace
+    from gradwave_b200 import density
+    made = []
+
+    class Batch:
+        pass
+
+    class Handle:
+        def __init__(self, bk, shape, device):
+            self._h, self.nk, self.npw_max, self.shape = object(), 1, 4, shape
+            made.append(self)
+
+    monkeypatch.setattr(density, "_GeometryHandle", Handle)
+    monkeypatch.setattr(density, "density_from_handle", lambda h, *a: h)
+    monkeypatch.setattr(density, "_HANDLES", {})
+    c = torch.zeros(1, 1, 4, dtype=torch.complex128)
+    for bk in (namedtuple("Bk", "mask npw flat_idx")(1, 2, 3), SimpleNamespace(mask=1), Batch()):
+        first = density.density_b(c, None, None, bk, (2, 2, 2), 1.0)
+        assert density.density_b(c, None, None, bk, (2, 2, 2), 1.0) is first
+    assert len(made) == len(density._HANDLES) == 3
+    del bk
+    assert len(density._HANDLES) == 2
