@@ -80,10 +80,15 @@ def density_from_handle(handle, nk: int, npw_max: int, shape, coeffs: torch.Tens
 
 
 def _reference(bk, key):
-    """bk by a call, as long as it lives: the handle (and its scratch) goes with it. A bk that takes no weak
-    reference (named tuple, slots) is kept instead, and its handle with it."""
+    """bk by a call, as long as it lives: the handle (and its scratch) goes with it, at the next call where a stream
+    capture is under way (which freeing device memory would end). A bk that takes no weak reference (named tuple,
+    slots) is kept instead, and its handle with it."""
+    def gone(_):
+        if not (torch.cuda.is_initialized() and torch.cuda.is_current_stream_capturing()):
+            _HANDLES.pop(key, None)
+
     try:
-        return weakref.ref(bk, lambda _: _HANDLES.pop(key, None))
+        return weakref.ref(bk, gone)
     except TypeError:
         return lambda: bk
 
@@ -97,6 +102,8 @@ def density_b(coeffs: torch.Tensor, occ: torch.Tensor, kweights: torch.Tensor, b
     key = (id(bk), tuple(int(s) for s in shape), dev.index)
     h = _HANDLES.get(key)
     if h is None or h[1]() is not bk:
+        for k in [k for k, v in list(_HANDLES.items()) if v[1]() is None]:
+            _HANDLES.pop(k, None)
         h = (_GeometryHandle(bk, shape, dev), _reference(bk, key))
         _HANDLES[key] = h
     g = h[0]

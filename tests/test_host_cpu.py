@@ -210,3 +210,30 @@ def test_density_handles_of_any_batch(monkeypatch):
     assert len(made) == len(density._HANDLES) == 3
     del bk
     assert len(density._HANDLES) == 2
+
+
+def test_density_handle_of_a_batch_that_dies_under_capture(monkeypatch):
+    """Its handle is left alone until the next new batch: freeing device memory would end the capture."""
+    from gradwave_b200 import density
+
+    class Batch:
+        pass
+
+    class Handle:
+        def __init__(self, bk, shape, device):
+            self._h, self.nk, self.npw_max, self.shape = object(), 1, 4, shape
+
+    monkeypatch.setattr(density, "_GeometryHandle", Handle)
+    monkeypatch.setattr(density, "density_from_handle", lambda h, *a: h)
+    monkeypatch.setattr(density, "_HANDLES", {})
+    monkeypatch.setattr(torch.cuda, "is_initialized", lambda: True)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: True)
+    c = torch.zeros(1, 1, 4, dtype=torch.complex128)
+    bk = Batch()
+    density.density_b(c, None, None, bk, (2, 2, 2), 1.0)
+    del bk
+    assert len(density._HANDLES) == 1
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    bk = Batch()
+    density.density_b(c, None, None, bk, (4, 2, 2), 1.0)
+    assert [k[1] for k in density._HANDLES] == [(4, 2, 2)]
