@@ -19,6 +19,8 @@
 #include <cstdlib>
 #include <cstring>
 #include <atomic>
+#include <memory>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -693,12 +695,13 @@ const char* gwb_last_error(void) { return g_last_error.c_str(); }
 const char* gwb_version(void) { return "gwb 0.1 sm_100a"; }
 unsigned long long gwb_launch_count(void) { return g_launches.load(std::memory_order_relaxed); }
 
-int gwb_ham_create(const gwb_ham_geometry* geom, int device, gwb_ham** out) {
+static int create_handle(const gwb_ham_geometry* geom, int device, gwb_ham** out) {
   GWB_REQUIRE(geom && out, "null argument");
   GWB_REQUIRE(geom->nk > 0 && geom->npw_max > 0 && geom->nproj >= 0, "bad nk/npw_max/nproj");
   GWB_REQUIRE(geom->npw && geom->flat_idx, "null npw/flat_idx");
   *out = nullptr;
-  auto* h = new gwb_ham();
+  std::unique_ptr<gwb_ham, int (*)(gwb_ham*)> owner(new gwb_ham(), gwb_ham_destroy);  // also where host memory runs out
+  gwb_ham* h = owner.get();
   h->device = device;
   h->nk = geom->nk;
   h->npw_max = geom->npw_max;
@@ -707,7 +710,6 @@ int gwb_ham_create(const gwb_ham_geometry* geom, int device, gwb_ham** out) {
   for (int a = 0; a < 3; ++a) {
     g.n[a] = geom->n[a];
     if (!axis_ok(g.n[a])) {
-      delete h;
       set_error("FFT axis length " + std::to_string(geom->n[a]) + " unsupported (need <=128, factors 2,3,5,7)");
       return GWB_ERR_ARG;
     }
@@ -719,25 +721,27 @@ int gwb_ham_create(const gwb_ham_geometry* geom, int device, gwb_ham** out) {
   struct Cell {
     uint8_t i0, i1, i2;
   };
-  std::vector<Cell> cell((size_t)h->nk * h->npw_max);
-  int M[3] = {0, 0, 0};
+  std::vector<size_t> first(h->nk + 1, 0);  // k's points in cell (the padding takes no host memory)
   for (int k = 0; k < h->nk; ++k) {
     const int64_t np_k = h->npw_host[k];
     if (np_k < 0 || np_k > h->npw_max) {
-      delete h;
       set_error("npw[k] out of range");
       return GWB_ERR_ARG;
     }
-    for (int64_t gi = 0; gi < np_k; ++gi) {
+    first[k + 1] = first[k] + np_k;
+  }
+  std::vector<Cell> cell(first[h->nk]);
+  int M[3] = {0, 0, 0};
+  for (int k = 0; k < h->nk; ++k) {
+    for (int64_t gi = 0; gi < h->npw_host[k]; ++gi) {
       const int64_t f = geom->flat_idx[(size_t)k * h->npw_max + gi];
       if (f < 0 || f >= nbox) {
-        delete h;
         set_error("flat_idx out of the box");
         return GWB_ERR_ARG;
       }
       const unsigned u = (unsigned)f, q = u / (unsigned)n2, i0 = q / (unsigned)n1;
       const int idx[3] = {(int)i0, (int)(q - i0 * n1), (int)(u - q * n2)};
-      cell[(size_t)k * h->npw_max + gi] = {(uint8_t)idx[0], (uint8_t)idx[1], (uint8_t)idx[2]};
+      cell[first[k] + gi] = {(uint8_t)idx[0], (uint8_t)idx[1], (uint8_t)idx[2]};
       for (int a = 0; a < 3; ++a) {
         const int m = idx[a] <= g.n[a] / 2 ? idx[a] : idx[a] - g.n[a];
         M[a] = std::max(M[a], std::abs(m));
@@ -755,7 +759,7 @@ int gwb_ham_create(const gwb_ham_geometry* geom, int device, gwb_ham** out) {
   std::vector<int> nrow_k(h->nk, 0);
   for (int k = 0; k < h->nk; ++k) {
     int* ro = rowof.data() + (size_t)k * L0 * n1;
-    const Cell* ck = cell.data() + (size_t)k * h->npw_max;
+    const Cell* ck = cell.data() + first[k];
     for (int64_t gi = 0; gi < h->npw_host[k]; ++gi) ro[compact0(ck[gi].i0) * n1 + ck[gi].i1] = 0;
     for (int i = 0; i < L0 * n1; ++i)
       if (ro[i] == 0) ro[i] = nrow_k[k]++;
@@ -764,7 +768,7 @@ int gwb_ham_create(const gwb_ham_geometry* geom, int device, gwb_ham** out) {
   std::vector<int> map((size_t)h->nk * g.nrow * n2, -1), dup;
   for (int k = 0; k < h->nk; ++k)
     for (int64_t gi = h->npw_host[k] - 1; gi >= 0; --gi) {
-      const Cell p = cell[(size_t)k * h->npw_max + gi];
+      const Cell p = cell[first[k] + gi];
       const int row = rowof[((size_t)k * L0 + compact0(p.i0)) * n1 + p.i1];
       int& slot = map[((size_t)k * g.nrow + row) * n2 + p.i2];
       if (slot < 0) slot = (int)gi;
@@ -788,7 +792,6 @@ int gwb_ham_create(const gwb_ham_geometry* geom, int device, gwb_ham** out) {
   auto fail = [&](cudaError_t e) {
     cudaGetLastError();
     set_error(std::string("gwb_ham_create: ") + cudaGetErrorString(e));
-    gwb_ham_destroy(h);
     return GWB_ERR_CUDA;
   };
   auto no_room = [&] { return fail(cudaErrorMemoryAllocation); };
@@ -825,8 +828,17 @@ int gwb_ham_create(const gwb_ham_geometry* geom, int device, gwb_ham** out) {
   }
   g_pool.handles(device, 1);
   h->counted = true;
-  *out = h;
+  *out = owner.release();
   return GWB_OK;
+}
+
+int gwb_ham_create(const gwb_ham_geometry* geom, int device, gwb_ham** out) {
+  try {
+    return create_handle(geom, device, out);
+  } catch (const std::bad_alloc&) {
+    set_error("gwb_ham_create: out of host memory");
+    return GWB_ERR_ALLOC;
+  }
 }
 
 int gwb_ham_destroy(gwb_ham* h) {

@@ -237,3 +237,27 @@ def test_density_handle_of_a_batch_that_dies_under_capture(monkeypatch):
     bk = Batch()
     density.density_b(c, None, None, bk, (4, 2, 2), 1.0)
     assert [k[1] for k in density._HANDLES] == [(4, 2, 2)]
+
+
+def test_handle_creation_takes_host_memory_for_points_only():
+    """A geometry of one point in rows of 2^31 - 1, with 2 GB of address space left: no table is as long as the padded
+    row, and running out of host memory is an error code, not an exception through the C interface."""
+    import subprocess
+    import sys
+    code = """
+import ctypes, resource
+import numpy as np
+from gradwave_b200 import _lib
+_lib.load()
+size = int(open("/proc/self/statm").read().split()[0]) * resource.getpagesize()
+resource.setrlimit(resource.RLIMIT_AS, (size + (2 << 30), -1))
+def create(nk, npw_max, npw):
+    npw, flat = np.full(nk, npw, dtype=np.int64), np.zeros(max(1, npw), dtype=np.int64)
+    g = _lib.Geometry(nk, npw_max, (ctypes.c_int32 * 3)(4, 4, 4), 0, npw.ctypes.data_as(ctypes.POINTER(ctypes.c_int64)),
+                      flat.ctypes.data_as(ctypes.POINTER(ctypes.c_int64)))
+    h = ctypes.c_void_p()
+    return _lib.load().gwb_ham_create(ctypes.byref(g), 10 ** 6, ctypes.byref(h))
+print(create(1, 2 ** 31 - 1, 1), create(60000000, 1, 0))
+"""
+    run = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True)
+    assert run.stdout.split() == ["2", "6"], run.stdout + run.stderr   # no such device; no host memory
