@@ -31,7 +31,8 @@ def _handle(shape, flat, nk, npw_max, npw, v, t):
 
 
 def _check(shape, sel, dev, seed, nb=3):
-    """Two k: the points ``sel`` of the box (box indices), the second k short of a third of them."""
+    """Two k: the points ``sel`` of the box (box indices), the second k short of a third of them. Returns the applies
+    (complex128 and complex64 rows in both precisions) and the density."""
     from gradwave_b200 import _lib
     rng = np.random.default_rng(seed)
     n = int(np.prod(shape))
@@ -56,6 +57,7 @@ def _check(shape, sel, dev, seed, nb=3):
         rho += (w[k, :, None, None, None] * psi.abs() ** 2).sum(0)
         loc = torch.fft.fftn(psi * v, dim=(1, 2, 3)).reshape(nb, n)[:, idx] / n
         ref[k, :, :npw[k]] = t[k, :npw[k]] * c[k, :, :npw[k]] + loc
+    got = []
     try:
         # a transform's error is a few eps sqrt(log N) of its norm: 1e-14 and 1e-6 leave a factor of ten
         for dt, prec, tol in ((torch.complex128, 1, 1e-14), (torch.complex128, 0, 1e-6), (torch.complex64, 0, 1e-6),
@@ -68,10 +70,12 @@ def _check(shape, sel, dev, seed, nb=3):
             assert err < tol, (shape, dt, prec, err)
             for k in range(2):
                 assert not out[k, :, npw[k]:].any()
+            got.append(out)
         r = torch.empty(shape, dtype=torch.float64, device=dev)
         _lib.call("gwb_ham_density", h, c.data_ptr(), nb * npw_max, nb, 1, w.data_ptr(), nb, 1.0, r.data_ptr(),
                   _lib.stream_ptr())
         assert float((r - rho).norm() / rho.norm()) < 1e-14
+        return got + [r]
     finally:
         torch.cuda.synchronize()
         _lib.load().gwb_ham_destroy(h)
@@ -91,12 +95,23 @@ def test_every_axis_length(n, cuda_device):
         _check(shape, few, cuda_device, n + 1, nb=5)
 
 
+@pytest.mark.parametrize("n", LENGTHS)
+def test_bands_of_one_block(n, cuda_device):
+    """Length n on axis 0 with so many pencils that a block of the axis-0 kernel takes several bands (10 bands in
+    groups of 3 or 4, the last one short), the next band's points arriving while one is transformed."""
+    shape = [n, 96, 100]
+    sel = np.random.default_rng(n).choice(n * 9600, 1500, replace=False)
+    _check(shape, sel, cuda_device, n, nb=10)
+
+
 def test_unequal_axes_and_chunks(cuda_device, monkeypatch):
     """A large box with unequal axes, in one chunk and band by band: bit for bit the same."""
+    sel = np.random.default_rng(0).choice(30 * 108 * 49, 9000, replace=False)
     monkeypatch.setenv("GWB_W_BUDGET_MB", "1")
-    _check([30, 108, 49], np.random.default_rng(0).choice(30 * 108 * 49, 9000, replace=False), cuda_device, 1, nb=7)
+    bands = _check([30, 108, 49], sel, cuda_device, 1, nb=7)
     monkeypatch.delenv("GWB_W_BUDGET_MB")
-    _check([30, 108, 49], np.random.default_rng(0).choice(30 * 108 * 49, 9000, replace=False), cuda_device, 1, nb=7)
+    chunk = _check([30, 108, 49], sel, cuda_device, 1, nb=7)
+    assert all(torch.equal(x, y) for x, y in zip(bands, chunk))
 
 
 def test_slots_of_one_box_cell(cuda_device):
