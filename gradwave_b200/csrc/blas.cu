@@ -37,7 +37,19 @@ int blas_handle(cublasHandle_t* out) {
   return GWB_OK;
 }
 
-constexpr int64_t kShortRows = 64;
+// Products of few rows against long ones that the own tiles (zmma_ab, launched in
+// chain) take from cuBLAS. Measured, us own / cuBLAS, op(A) = A, batch 10 x N =
+// 4625, 4 x 37000 and 1 x 750: 8 x 112: 18 / 31, 52 / 85, 6 / 8; 16 x 64: 21 / 21,
+// 58 / 62, 6 / 7; 16 x 112: 34 / 33, 93 / 93, 8 / 8; 24 x 24: 14 / 20, 37 / 54, 6 /
+// 19; 24 x 96: 37 / 41, 107 / 121, 10 / 19; 24 x 448: 151 / 159, 464 / 502, 40 / 17;
+// 32 x 32: 20 / 21, 57 / 55, 6 / 14; 32 x 128: 65 / 58, 189 / 154, 17 / 9; 40 x 40:
+// 34 / 37, 94 / 111, 6 / 16; 48 x 48: 40 / 39, 112 / 119; 64 x 64: 65 / 54, 182 /
+// 156. The longer K, the more a cut per 8 terms costs, and one block per tile has
+// the whole of K in sequence. 128 is past the native solver's bases (112); where
+// the two are level its launches stay in chain.
+static bool short_rows(int64_t M, int64_t N, int64_t K) {
+  return N >= 8 * M && K <= (M <= 24 ? 128 : (M <= 40 ? M : 0));
+}
 
 static cublasOperation_t to_op(int op) {
   return op == 0 ? CUBLAS_OP_N : (op == 1 ? CUBLAS_OP_T : CUBLAS_OP_C);
@@ -55,10 +67,8 @@ extern "C" int gwb_zgemm(int opA, int opB, int64_t M, int64_t N, int64_t K, doub
   GWB_REQUIRE(M >= 0 && N >= 0 && K >= 0 && batch >= 0, "negative size");
   if (M == 0 || N == 0 || batch == 0) return GWB_OK;
   GWB_REQUIRE(A && B && C, "null matrix");
-  // few rows against long ones (the solver's triangular transforms, projections
-  // and Ritz vectors of small blocks): own tiles, launched in chain; cuBLAS for
-  // the rest, whose larger tiles load less
-  if (opB == 0 && opA <= 1 && M <= kShortRows && N >= 8 * M && K > 0 && batch <= 65535) {
+  // the solver's triangular transforms, projections and Ritz vectors of small blocks
+  if (opB == 0 && opA <= 1 && K > 0 && batch <= 65535 && short_rows(M, N, K)) {
     GWB_REQUIRE(lda >= (opA ? M : K) && ldb >= N && ldc >= N, "leading dimension smaller than a row");  // as cuBLAS
     GWB_CUDA_TRY(zmma_ab(opA == 1, (int)M, (int)N, (int)K, mk<double>(alpha_re, alpha_im), (const cplx<double>*)A, lda,
                          strideA, (const cplx<double>*)B, ldb, strideB, mk<double>(beta_re, beta_im), (cplx<double>*)C,

@@ -82,6 +82,22 @@ def test_short_row_products(op, M, N, K, batch, cuda_device):
         assert bool(((C[:, :, :N] - ref).abs() <= bound).all())
 
 
+@pytest.mark.parametrize("M,N,K", [(8, 64, 128), (8, 63, 128), (24, 192, 128), (24, 192, 129), (25, 200, 25), (25, 200, 26),
+                                   (40, 320, 40), (41, 328, 41)])
+def test_short_row_rule(M, N, K, cuda_device):
+    """Both sides of every line between the own tiles and cuBLAS, and which side it is (the own tiles count their
+    launches)."""
+    from gradwave_b200 import _lib
+    A, B, C = _rand(2, M, K, seed=1), _rand(2, K, N, seed=2), torch.empty(2, M, N, dtype=torch.complex128, device=cuda_device)
+    before = _lib.launch_count()
+    _lib.call("gwb_zgemm", 0, 0, M, N, K, 1.0, 0.0, A.data_ptr(), K, M * K, B.data_ptr(), N, K * N, 0.0, 0.0, C.data_ptr(), N,
+              M * N, 2, _lib.stream_ptr())
+    own = N >= 8 * M and K <= (128 if M <= 24 else M if M <= 40 else 0)
+    assert _lib.launch_count() - before == int(own)
+    bound = (K + 2) * 2.3e-16 * 2.2 * (A.abs() @ B.abs())   # as above
+    assert bool(((C - A @ B).abs() <= bound).all())
+
+
 @pytest.mark.parametrize("n", [1, 2, 15, 16, 17, 33, 63, 64])
 def test_cholesky_and_inverse(n, cuda_device):
     """L L^H = G and L^-1 L = 1 for two matrices (n eps cond: the random Gram matrices have cond below 1e4), the
@@ -115,7 +131,7 @@ def _err_extended(got, a, b):
 _ROUND = 2.0 ** -53 / np.sqrt(3.0)
 
 
-@pytest.mark.parametrize("op,M,N,K", [(0, 24, 256, 96), (1, 24, 256, 96), (0, 64, 512, 200), (1, 64, 512, 640)])
+@pytest.mark.parametrize("op,M,N,K", [(0, 24, 256, 96), (1, 24, 256, 96), (0, 8, 512, 128), (1, 8, 512, 128), (0, 40, 512, 40)])
 def test_short_row_products_rounding(op, M, N, K, cuda_device):
     """Rounding of a random product. A sum that grows like sqrt(k) errs by sqrt(n / 2) roundings of its final size
     after n of them: chains of 16 and one addition per 8 terms give sqrt(8 + K / 16), plus the last operations;
