@@ -105,11 +105,12 @@ int gwb_stall_update(const double*, double*, uint8_t*, uint8_t*, int32_t, double
 
 namespace gwb {
 
-// Noise on the first expansion rows of a cold start (gwb_start_noise): norm, and
-// the largest residual [eV] above which a start counts as cold. The host driver
-// has the same for bases of this size (davidson.py, break_symmetry, with the
-// reasons).
-constexpr double kStartNoise = 0.02, kColdStartEv = 1.0;
+// Noise on the first expansion rows of a cold start (gwb_start_noise): its norm,
+// and the largest residual [eV] above which a start counts as cold. The host
+// driver has the same for bases of this size (davidson.py, break_symmetry, with
+// the reasons).
+inline double start_noise(double tol) { return std::min(0.25, 3.0 * std::sqrt(tol)); }
+constexpr double kColdStartEv = 1.0;
 
 struct Buf {
   size_t off = 0;
@@ -280,7 +281,8 @@ class Solver {
       if (rnmax < p_.tol) return finish(it, eig, eig_out, vec_out, rn_out, out, rnmax);
       GWB_TRY(gwb_select_worst(nk_, nb_, w_.rn, n_add, w_.sel, st_));
       GWB_TRY(precondition(n_add, eig));
-      if (it == 1) GWB_TRY(gwb_start_noise(nk_, n_add, npw_, w_.D, nbp, mask_, w_.rn, nb_, kColdStartEv, kStartNoise, st_));
+      if (it == 1)
+        GWB_TRY(gwb_start_noise(nk_, n_add, npw_, w_.D, nbp, mask_, w_.rn, nb_, kColdStartEv, start_noise(p_.tol), st_));
       if (m + n_add > md_) {
         ++n_restart_;
         GWB_TRY(cholqr2(w_.X, nbp, nb_, w_.D2, w_.X, nbp, w_.HX, w_.R, /*sync=*/true, &ok));

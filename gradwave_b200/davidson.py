@@ -64,12 +64,17 @@ logger = logging.getLogger(__name__)
 
 _FP32_CERT_FLOOR_EPS = 32 * torch.finfo(torch.float32).eps
 _FP32_CERT_STALL = 0.7
-# norm of the noise on the unit rows of the first expansion of a cold start
-# (largest residual of a k-point above _COLD_START_EV): bases within the batched
-# eigensolver's limit, and beyond (break_symmetry)
-_START_NOISE, _START_NOISE_LARGE = 0.02, 0.25
+# noise on the first expansion rows of a cold start (largest residual of a k-point
+# above _COLD_START_EV, eV): norm for bases beyond the batched eigensolver's limit
+_START_NOISE_LARGE = 0.25
 _COLD_START_EV = 1.0
 _N, _T, _H = 0, 1, 2
+
+
+def start_noise(tol: float, factor: float = 3.0) -> float:
+    """Norm of the noise on the unit rows of a cold start's first expansion
+    (``_Solver.break_symmetry``)."""
+    return min(0.25, factor * math.sqrt(tol))
 
 
 @dataclass
@@ -618,24 +623,25 @@ class _Solver:
         but round-off: such a level shows up only after round-off has grown to
         the size of a Ritz vector, and a solve that converges before skips it.
         Noise of the order of the rows themselves lets it converge with the
-        others: it must come up before they reach the tolerance, so 3e-6 is
-        enough at 1e-10 eV, and 0.02 down to 4e-3 eV.
-
-        Perfect 2- and 8-atom cells, 6 to 40 bands, identity starts 1e-15
-        apart, float64 and mixed, both preconditioners: 21 of 864 solves skip
-        a level without noise (0.2 to 5 eV), none of 4896 with norms from 3e-6
-        to 0.7; mean rounds 47 without, 46 to 49 with it. What the norm costs
-        in rounds is another matter. Displaced 8-atom cells, 24 bands (TPA /
-        network): 54 / 35 without, 51 / 35 at 0.02, 57 / 44 at 0.25. Perfect
-        64-atom cell, 160 bands, six starts (TPA / mixed / mixed with the
-        network): 75-204 / 83-300 / 38 at 0.02, 51-57 / 50-77 / 39-40 at 0.25.
+        others. It has to grow to a Ritz vector before they reach the
+        tolerance, whose square root sets the norm: perfect 8-atom cell, 16 to
+        24 bands, both preconditioners, tolerances 1e-4 to 1e-8, 300 solves: 12
+        skip a level with 0.3 sqrt(tol), one with 3 sqrt(tol). At 1e-10 eV
+        (perfect 2- and 8-atom cells, 6 to 40 bands, identity starts 1e-15
+        apart, float64 and mixed) 21 of 864 skip one without noise, by 0.2 to
+        5 eV, none of 1152 with 3 sqrt(tol). More of it costs the small solves
+        rounds (displaced 8-atom cells, 24 bands, TPA / network: 54 / 35
+        without, 53 / 35 with it, 57 / 44 at 0.25), but the perfect 64-atom
+        cell needs 0.25 (160 bands, six starts, TPA / mixed / mixed with the
+        network: 51-57 / 50-77 / 39-40 rounds; 75-204 / 83-300 / 38 at 0.02):
+        bases beyond the batched eigensolver's limit take that.
 
         The noise is a function of row and plane wave alone, so that a k-point
         is solved alike in whatever group or shard it is."""
         ws, npw = self.ws, self.npw
         _lib.call("gwb_start_noise", self.nk, n_add, npw, _ptr(ws.D), ws.D.shape[1] * npw, _ptr(self.mask_u8),
                   _ptr(ws.rn), self.nb, _COLD_START_EV,
-                  _START_NOISE if self.max_dim <= self.heev_max else _START_NOISE_LARGE, self.stream)
+                  start_noise(self.tol) if self.max_dim <= self.heev_max else _START_NOISE_LARGE, self.stream)
 
     def precondition(self, n_add: int, eig: torch.Tensor):
         """D[:, :n_add] = preconditioned, unit-normalised worst residuals."""

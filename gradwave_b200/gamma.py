@@ -760,7 +760,7 @@ def davidson_gamma(ham: GammaHamiltonian, x0: torch.Tensor, tol: float = 1e-9, m
     if n_buffer < 0:
         raise ValueError(f"n_buffer must be >= 0, got {n_buffer}")
     import os
-    from .davidson import _COLD_START_EV, _PhaseTimer
+    from .davidson import _COLD_START_EV, _PhaseTimer, start_noise
     prof = _PhaseTimer(os.environ.get("GWB_PROFILE", "0") == "1")
     lock = (mode == "mixed") if lock is None else bool(lock)
     gb, dev = ham.gb, ham.device
@@ -975,7 +975,7 @@ def davidson_gamma(ham: GammaHamiltonian, x0: torch.Tensor, tol: float = 1e-9, m
                 pr = pr / torch.linalg.vector_norm(pr, dim=1, keepdim=True).clamp_min(1e-300)
                 gen = torch.Generator(device=dev).manual_seed(20260)
                 noise = torch.randn(pr.shape, generator=gen, dtype=pr.dtype, device=dev)
-                pr += min(0.25, 0.3 * math.sqrt(tol)) / math.sqrt(nphi) * noise
+                pr += start_noise(tol, 0.3) / math.sqrt(nphi) * noise
             pr[:, nphi:] = 0.0  # the pad column is not a coordinate of the operator
         with phase("orthonormalize"):
             t = _expand(pr, v, tcp, locked.rows(), mm, low=low and tc_active)
