@@ -108,6 +108,16 @@ static bool axis_ok(int n) {
   return n == 1;
 }
 
+// exp(2 pi i m / n), the angle reduced to an eighth of a turn exactly and taken in
+// extended precision: cos and sin of a rounded 2 pi m / n are off by up to 8e-16.
+static cplx<double> unit_root(int m, int n) {
+  const int q = (8 * m + n) / (2 * n);  // nearest quarter turn
+  const long double x = 3.14159265358979323846264338327950288L * (4 * m - q * n) / (2 * n);
+  const double c = (double)std::cos(x), s = (double)std::sin(x);
+  const cplx<double> r[4] = {mk<double>(c, s), mk<double>(-s, c), mk<double>(-c, -s), mk<double>(s, -c)};
+  return r[q % 4];
+}
+
 // Scratch of one band chunk. A float64 96^3 Gamma apply of 240 rows takes 8.2 ms
 // at 48 MB (L2 sized), 8.0 at 96 to 192, 7.7 at 512, 7.5 at 1024: launch ramps and
 // last waves weigh more than L2 misses, and past 512 MB little is left.
@@ -776,17 +786,15 @@ static int create_handle(const gwb_ham_geometry* geom, int device, gwb_ham** out
     }
   h->ndup = (int)(dup.size() / 3);
   std::vector<int> npw32(h->npw_host.begin(), h->npw_host.end());
-  // twiddles exp(-2 pi i a k / n) at k R2 + a (n = R1 R2), the angle reduced exactly: cos and sin of the rounded
-  // 2 pi a k / n are off by up to 8e-16
+  // twiddles exp(-2 pi i a k / n) at k R2 + a (n = R1 R2)
   std::vector<cplx<double>> tw64[3];
   std::vector<cplx<float>> tw32[3];
   for (int a = 0; a < 3; ++a) {
     const int n = g.n[a], R2 = n / fft_r1(n);
     for (int t = 0; t < n; ++t) {
-      const int m = (t / R2) * (t % R2);
-      const double c = rdft_detail::cis(m, n, 0), s = -rdft_detail::cis(m, n, 1);
-      tw64[a].push_back(mk<double>(c, s));
-      tw32[a].push_back(mk<float>((float)c, (float)s));
+      const cplx<double> w = conj(unit_root((t / R2) * (t % R2), n));
+      tw64[a].push_back(w);
+      tw32[a].push_back(mk<float>((float)w.x, (float)w.y));
     }
   }
   auto fail = [&](cudaError_t e) {
