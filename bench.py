@@ -599,8 +599,8 @@ def _gamma_line(args, ci, gold, dev, flush, ws, rank) -> dict:
     ms_plain = _max_over_ranks(ms_plain, ws, dev)
     npw = float(gb.npw)
     roof = _apply_roofline(tm, 0.5, npw, float(np.prod(ci.shape)), int(ci.p.shape[1]), 1, ms_fast,
-                           "gwb_gamma_apply (pack + plane_inverse + pencil_vloc + plane_forward + nonlocal + "
-                           "unpack; two real bands per complex row)", f"gwb_gamma_apply_{args.config}")
+                           "gwb_gamma_apply (pack + rows_inverse + cols_inverse + pencil_vloc + cols_forward + "
+                           "rows_forward + nonlocal + unpack; two real bands per complex row)", f"gwb_gamma_apply_{args.config}")
     line = {"metric": METRIC, "value": round(ms_fast / ws, 3), "unit": "ms", "n_gpus": ws,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": round(ms_fast, 3),
             "higher_is_better": False, "scaling": "weak",
@@ -687,7 +687,8 @@ def _kpoint_line(args, ci, gold, dev, flush, ws, rank) -> dict:
           "bands": int(res.n_apply_low + res.n_apply_full)}
     npw = float(bk.npw.float().mean())
     roof = _apply_roofline(tm, 1.0, npw, float(np.prod(ci.shape)), int(ci.p.shape[1]), k1 - k0, ms_fast,
-                           "gwb_ham_apply (plane_inverse + pencil_vloc + plane_forward + becp + nl_add)",
+                           "gwb_ham_apply (rows_inverse + cols_inverse + pencil_vloc + cols_forward + rows_forward + "
+                           "becp + nonlocal update)",
                            f"gwb_ham_apply_{args.config}")
     return {"metric": METRIC, "value": round(ms_fast, 3), "unit": "ms", "n_gpus": ws,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": round(ms_fast, 3),

@@ -111,7 +111,8 @@ void count_launches(int n);
 // writes anything that an earlier kernel of the stream touches; the wait ends
 // when all of the kernel before it has completed and its writes are visible.
 // The hand-on to the next kernel comes after the wait, so that whatever is two
-// kernels back is complete too. (25^3 apply of 8 kernels: ZZ us with, ZZ without.)
+// kernels back is complete too. (Applies without and with: 2 atoms 43.0 -> 39.4 us,
+// 42^3 complex64 192 -> 182, H c and S c of 8 atoms 240 -> 232.)
 __device__ __forceinline__ void chain_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(256) k_row_repair(int npw, int n, cplx<double>
   nn = block_sum<256>(nn, red);
   if (sqrt(nn) < thresh) {
     const unsigned long long base = ((unsigned long long)k * 4099ull + (unsigned long long)s) * 1000003ull;
-      for (int g = threadIdx.x; g < npw; g += blockDim.x) {
+    for (int g = threadIdx.x; g < npw; g += blockDim.x) {
       const unsigned long long key = (base + (unsigned long long)g) * 2ull;
       row[g] = mask[(int64_t)k * npw + g] ? mk<double>(hash_unit(key), hash_unit(key + 1)) : mk<double>(0.0, 0.0);
     }
@@ -380,7 +380,9 @@ int gwb_residual(int32_t nk, int32_t nb, int32_t npw, const void* x, int64_t x_k
   GWB_REQUIRE(nk >= 0 && nb >= 0 && npw > 0, "bad sizes");
   if (nk == 0 || nb == 0) return GWB_OK;
   GWB_REQUIRE(x && hx && eig && r && rn, "null pointer");
-  GWB_CUDA_TRY(launch_chained(k_residual, dim3(nk * nb), 256, 0, (cudaStream_t)stream, npw, (const cplx<double>*)x, x_kstride, (const cplx<double>*)hx, hx_kstride, eig, eig_kstride, (cplx<double>*)r, r_kstride, rn, nb));
+  GWB_CUDA_TRY(launch_chained(k_residual, dim3(nk * nb), 256, 0, (cudaStream_t)stream, npw, (const cplx<double>*)x,
+                              x_kstride, (const cplx<double>*)hx, hx_kstride, eig, eig_kstride, (cplx<double>*)r,
+                              r_kstride, rn, nb));
   count_launches(1);
   return GWB_OK;
 }
@@ -404,7 +406,9 @@ int gwb_precond_teter(int32_t nk, int32_t nb, int32_t n_add, int32_t npw, const 
                       int64_t d_kstride, void* stream) {
   GWB_REQUIRE(nk > 0 && nb > 0 && n_add > 0 && n_add <= nb && npw > 0, "bad sizes");
   GWB_REQUIRE(x && r && t && sel && d, "null pointer");
-  GWB_CUDA_TRY(launch_chained(k_precond_teter, dim3(nk * n_add), 256, 0, (cudaStream_t)stream, npw, nb, n_add, (const cplx<double>*)x, x_kstride, (const cplx<double>*)r, r_kstride, t, sel, (cplx<double>*)d, d_kstride));
+  GWB_CUDA_TRY(launch_chained(k_precond_teter, dim3(nk * n_add), 256, 0, (cudaStream_t)stream, npw, nb, n_add,
+                              (const cplx<double>*)x, x_kstride, (const cplx<double>*)r, r_kstride, t, sel,
+                              (cplx<double>*)d, d_kstride));
   count_launches(1);
   return GWB_OK;
 }
@@ -416,7 +420,8 @@ int gwb_subspace_insert(int32_t nk, int32_t m, int32_t m0, const void* C, void* 
   const int64_t total = (int64_t)m * (m - m0);
   const int blocks = (int)std::min<int64_t>((total + 255) / 256, 1024);
   dim3 grid(blocks, nk);
-  GWB_CUDA_TRY(launch_chained(k_subspace_insert, grid, 256, 0, (cudaStream_t)stream, (const cplx<double>*)C, m, m0, (cplx<double>*)S, lds, s_kstride));
+  GWB_CUDA_TRY(launch_chained(k_subspace_insert, grid, 256, 0, (cudaStream_t)stream, (const cplx<double>*)C, m, m0,
+                              (cplx<double>*)S, lds, s_kstride));
   count_launches(1);
   return GWB_OK;
 }
@@ -443,13 +448,14 @@ int gwb_row_repair(int32_t nk, int32_t n, int32_t npw, void* D, int64_t d_kstrid
                    double thresh, int32_t* flag, void* stream) {
   GWB_REQUIRE(nk > 0 && n > 0 && npw > 0, "bad sizes");
   GWB_REQUIRE(D && mask && flag, "null pointer");
-  GWB_CUDA_TRY(launch_chained(k_row_repair, dim3(nk * n), 256, 0, (cudaStream_t)stream, npw, n, (cplx<double>*)D, d_kstride, mask, thresh, flag));
+  GWB_CUDA_TRY(launch_chained(k_row_repair, dim3(nk * n), 256, 0, (cudaStream_t)stream, npw, n, (cplx<double>*)D,
+                              d_kstride, mask, thresh, flag));
   count_launches(1);
   return GWB_OK;
 }
 
-int gwb_start_noise(int32_t nk, int32_t n, int32_t npw, void* D, int64_t d_kstride, const uint8_t* mask, const double* rn,
-                    int32_t nb, double cold, double norm, void* stream) {
+int gwb_start_noise(int32_t nk, int32_t n, int32_t npw, void* D, int64_t d_kstride, const uint8_t* mask,
+                    const double* rn, int32_t nb, double cold, double norm, void* stream) {
   GWB_REQUIRE(nk > 0 && n > 0 && npw > 0 && nb > 0, "bad sizes");
   GWB_REQUIRE(D && mask && rn, "null pointer");
   GWB_CUDA_TRY(launch_chained(k_start_noise, dim3(nk * n), 256, 0, (cudaStream_t)stream, npw, n, (cplx<double>*)D,

@@ -90,7 +90,8 @@ int gwb_precond_teter(int32_t, int32_t, int32_t, int32_t, const void*, int64_t, 
 int gwb_subspace_insert(int32_t, int32_t, int32_t, const void*, void*, int32_t, int64_t, void*);
 int gwb_chol_inv(int32_t, int32_t, void*, int32_t, int64_t, void*, int64_t, int32_t*, int32_t*, void*);
 int gwb_row_repair(int32_t, int32_t, int32_t, void*, int64_t, const uint8_t*, double, int32_t*, void*);
-int gwb_start_noise(int32_t, int32_t, int32_t, void*, int64_t, const uint8_t*, const double*, int32_t, double, double, void*);
+int gwb_start_noise(int32_t, int32_t, int32_t, void*, int64_t, const uint8_t*, const double*, int32_t, double, double,
+                    void*);
 int gwb_heev_lowest(int32_t, int32_t, int32_t, const void*, int32_t, int64_t, double*, void*, double*, int32_t*,
                     void*);
 int gwb_heev_max_dim(void);
@@ -282,7 +283,8 @@ class Solver {
       GWB_TRY(gwb_select_worst(nk_, nb_, w_.rn, n_add, w_.sel, st_));
       GWB_TRY(precondition(n_add, eig));
       if (it == 1)
-        GWB_TRY(gwb_start_noise(nk_, n_add, npw_, w_.D, nbp, mask_, w_.rn, nb_, kColdStartEv, start_noise(p_.tol), st_));
+        GWB_TRY(gwb_start_noise(nk_, n_add, npw_, w_.D, nbp, mask_, w_.rn, nb_, kColdStartEv, start_noise(p_.tol),
+                                st_));
       if (m + n_add > md_) {
         ++n_restart_;
         GWB_TRY(cholqr2(w_.X, nbp, nb_, w_.D2, w_.X, nbp, w_.HX, w_.R, /*sync=*/true, &ok));

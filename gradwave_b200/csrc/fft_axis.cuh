@@ -27,10 +27,10 @@
 // of the sphere's disc, 0.4 of W) written and read once more each way. Measured
 // against the passes in shared memory (whole applies, us; in brackets with the
 // predicates, twiddle layout and prefetch below, chained launches and the
-// products of zmma.cuh): 42^3 float32 240 rows 1086 -> 212 (183), 36x36x108
-// float64 244 rows 2760 -> 763 (583), 84^3 float64 258 rows 13836 -> 5513 (3648),
-// 108^3 float32 166 rows 14936 -> 3096 (2702), 96^3 float64 240 rows 12031 -> 7830
-// (7437). Bound by issue and the float64 pipe in the pencils, by latency in the
+// products of zmma.cuh): 42^3 float32 240 rows 1086 -> 212 (181), 36x36x108
+// float64 244 rows 2760 -> 763 (585), 84^3 float64 258 rows 13836 -> 5513 (3733),
+// 108^3 float32 166 rows 14936 -> 3096 (2678), 96^3 float64 240 rows 12031 -> 7830
+// (7505). Bound by issue and the float64 pipe in the pencils, by latency in the
 // others (up to 4 TB/s of scratch traffic), not by HBM.
 #pragma once
 

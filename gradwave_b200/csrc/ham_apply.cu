@@ -14,6 +14,8 @@
 //   K4 becp_partial   becp partial sums conj(p) . c over a slice of G
 //   K5 becp_reduce_d  sum of slices, times D  -> bd (nk, nb, nproj)
 //   K6 nl_add         out += bd . p
+// (float64 arithmetic on complex128 rows: K4 and K6 on the float64 tensor
+// instruction, zmma.cuh)
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -524,12 +526,14 @@ static int nonlocal_tc(gwb_ham* h, const cplx<double>* c, int64_t ck, cplx<doubl
   if ((rc = gwb_zgemm_tc(2, nb, np, npw, 1.0, 0.0, h->d_cplanes, ldp, nb, h->d_pplanes, ldp, np, 0.0, 0.0, h->d_becp,
                          np, (int64_t)nb * np, nk, h->d_tcwork, h->tcwork_bytes, h->d_tcstatus, st)))
     return rc;
-  if ((rc = tc_becp_d_planes(nk, nb, np, (const cplx<double>*)h->d_becp, h->d_d64, h->d_cols, h->d_bdplanes, ldq, st))) return rc;
+  if ((rc = tc_becp_d_planes(nk, nb, np, (const cplx<double>*)h->d_becp, h->d_d64, h->d_cols, h->d_bdplanes, ldq,
+                             st)))
+    return rc;
   return gwb_zgemm_tc(0, nb, npw, np, 1.0, 0.0, h->d_bdplanes, ldq, nb, h->d_pplanes, ldp, np, 1.0, 0.0, out, npw, ok,
                       nk, nullptr, 0, h->d_tcstatus, st);
 }
 
-// out = T c + local(c): the kinetic and FFT local terms, band chunks sized to L2.
+// out = T c + local(c): the kinetic and FFT local terms, in chunks of bands.
 template <typename T, typename SIO>
 static int local_term(gwb_ham* h, const SIO* c, int64_t ck, SIO* out, int64_t ok, int nb, cudaStream_t st) {
   int nbc = 0;
@@ -560,8 +564,8 @@ static int local_term(gwb_ham* h, const SIO* c, int64_t ck, SIO* out, int64_t ok
 
 // float64 arithmetic on complex128 rows: the float64 tensor instruction
 // (zmma.cuh); anything else the CUDA-core kernels above. Measured with 256
-// projectors, 2 k x 129 bands x 37,000 plane waves: becp 1908 -> 880 us, update
-// 1369 -> 720 us.
+// projectors, 2 k x 129 bands x 37,000 plane waves: becp 1908 -> 920 us, update
+// 1369 -> 750 us.
 template <typename T, typename SIO>
 constexpr bool nl_zmma = std::is_same<T, double>::value && std::is_same<SIO, cplx<double>>::value;
 
@@ -625,7 +629,7 @@ static int apply_impl(gwb_ham* h, const SIO* c, int64_t ck, SIO* out, int64_t ok
 }
 
 // Generalized apply: out_h = H c and out_s = S c = (c + sum_pq |p> q_pq <q|c>)
-// masked, from one becp contraction (CUDA cores, every precision).
+// masked, from one becp contraction.
 template <typename T, typename SIO>
 static int apply_hs_impl(gwb_ham* h, const SIO* c, int64_t ck, SIO* out_h, int64_t ohk, SIO* out_s, int64_t osk,
                          int nb, cudaStream_t st) {

@@ -693,7 +693,7 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
 // operations per plane wave at 80 % of its rate. Bit for bit the conversion's
 // value up to |h| = 5e33, where g overflows; beyond, the factor ends at a clamp
 // of the network's output (e^-3 or e^3) either way. Split at 2^-16 h it would
-// not overflow, at 1305 -> 1365 us of the 404 rows below.
+// not overflow (whole call on 404 rows of 37,000 plane waves: 1305 -> 1365 us).
 __device__ __forceinline__ f32x2 silu_bf16_2(uint32_t z0, uint32_t z1) {
   const f32x2 h = mul2(pk2(__uint_as_float(z0), __uint_as_float(z1)), pk2(0.5f, 0.5f));
   float h0, h1;
@@ -1128,14 +1128,16 @@ int gwb_precond_learned(const float* params, int32_t nk, int32_t nb, int32_t n_a
     k_precond_learned_tc<<<dim3(chunks, rows), PL_THREADS, 0, st>>>(params, npw, nb, n_add, (const cplx<double>*)r,
                                                                     r_kstride, t, eig, sel, tpa_only, stats,
                                                                     (cplx<double>*)d, d_kstride, partial);
-    k_precond_normalize<<<dim3(rows, normalize_splits(rows)), 256, 0, st>>>(npw, n_add, chunks, partial, (cplx<double>*)d, d_kstride);
+    k_precond_normalize<<<dim3(rows, normalize_splits(rows)), 256, 0, st>>>(npw, n_add, chunks, partial,
+                                                                            (cplx<double>*)d, d_kstride);
   } else {
     const int64_t tiles = (npw + PU_TILE - 1) / PU_TILE;
     int* status = reinterpret_cast<int*>(partial + (int64_t)rows * tiles);
     int rc = precond_umma<false>(params, nb, n_add, npw, r, r_kstride, 0, t, eig, sel, tpa_only, stats, d, d_kstride,
                                  0, partial, rows, status, st);
     if (rc) return rc;
-    k_precond_normalize<<<dim3(rows, normalize_splits(rows)), 256, 0, st>>>(npw, n_add, (int)tiles, partial, (cplx<double>*)d, d_kstride);
+    k_precond_normalize<<<dim3(rows, normalize_splits(rows)), 256, 0, st>>>(npw, n_add, (int)tiles, partial,
+                                                                            (cplx<double>*)d, d_kstride);
   }
   GWB_LAUNCH_CHECK();
   count_launches(3);
@@ -1166,7 +1168,8 @@ int gwb_precond_learned_gamma(const float* params, int32_t nb, int32_t n_add, in
   int rc = precond_umma<true>(params, nb, n_add, nhalf, r, 0, r_row, t_half, eig, sel, tpa_only, stats, d, 0, d_row,
                               partial, n_add, status, st);
   if (rc) return rc;
-  k_precond_normalize_gamma<<<dim3(n_add, normalize_splits(n_add)), 256, 0, st>>>(nhalf, npad, tiles, partial, d, d_row);
+  k_precond_normalize_gamma<<<dim3(n_add, normalize_splits(n_add)), 256, 0, st>>>(nhalf, npad, tiles, partial, d,
+                                                                                  d_row);
   GWB_LAUNCH_CHECK();
   count_launches(3);
   return GWB_OK;

@@ -113,8 +113,8 @@ def zgemm(opA, opB, M, N, K, A, lda, sA, B, ldb, sB, C, ldc, sC, batch, alpha=1.
           a_off=0, b_off=0, c_off=0, stream=None, work=None):
     """Row-major batched complex128 GEMM (offsets in elements): A B^H products
     with a small output go to the split-K kernel gwb_zgemm_nh (partial sums in
-    ``work``, default a per-device buffer), the rest to cuBLAS through
-    gwb_zgemm."""
+    ``work``, default a per-device buffer), the rest through gwb_zgemm to its
+    own tiles (few rows) or cuBLAS."""
     s = _lib.stream_ptr(C.device) if stream is None else stream
     a = complex(alpha)
     b = complex(beta)
@@ -622,8 +622,7 @@ class _Solver:
         irreducible representations, and no step of the solver brings one in
         but round-off: such a level shows up only after round-off has grown to
         the size of a Ritz vector, and a solve that converges before skips it.
-        Noise of the order of the rows themselves lets it converge with the
-        others. It has to grow to a Ritz vector before they reach the
+        Noise lets it converge with the others. It has to grow to a Ritz vector before they reach the
         tolerance, whose square root sets the norm: perfect 8-atom cell, 16 to
         24 bands, both preconditioners, tolerances 1e-4 to 1e-8, 300 solves: 12
         skip a level with 0.3 sqrt(tol), one with 3 sqrt(tol). At 1e-10 eV
