@@ -65,7 +65,7 @@ def test_nonlocal_of_both_outputs(nproj, nb, cuda_device):
 @pytest.mark.parametrize("M,N,K,batch", [(1, 8, 1, 1), (7, 63, 9, 2), (8, 64, 8, 3), (24, 193, 72, 2), (33, 1001, 17, 1),
                                          (64, 513, 64, 2), (65, 600, 5, 1)])
 def test_short_row_products(op, M, N, K, batch, cuda_device):
-    """C = alpha op(A) B + beta C of up to 64 rows (65: the library's) with strides wider than the matrices; C is
+    """C = alpha op(A) B + beta C of few rows (own tiles; 64 and 65: cuBLAS) with strides wider than the matrices; C is
     not read where beta = 0. Bound as above."""
     from gradwave_b200 import _lib
     A = _rand(batch, M, K + 2, seed=1) if op == 0 else _rand(batch, K, M + 2, seed=1)
