@@ -122,13 +122,12 @@ template <class Api> class DevicePool {
       return ensure(dev, &w.p, &w.bytes, need);
     };
     int n = bands(budget);
-    if (per_band * n <= w.bytes) return n;
-    if (per_band * n < w.denied) {
-      if (fits(per_band * n)) return n;
-      w.denied = per_band * n;
-    }
+    const size_t want = per_band * n;
+    if (want <= w.bytes || (want < w.denied && fits(want))) return n;
     n = std::min(n, bands(std::max(low, had)));
-    return fits(per_band * n) ? n : 0;
+    if (!fits(per_band * n)) return 0;     // nothing can be had (under a capture, say): asked for again
+    if (want > w.bytes) w.denied = std::min(w.denied, want);
+    return n;
   }
 
  private:

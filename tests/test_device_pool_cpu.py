@@ -97,6 +97,15 @@ int main() {
   gwb::ChunkScratch u;
   CHECK(pool.chunk(0, u, 30, 21, 300, 20) == 0 && !u.p && u.bytes == 0);
   Fake::free(v.p);
+  Fake::free(w.p);
+  w = {};
+  Fake::room = 0;                                                    // no allocation at all (a stream capture) ...
+  CHECK(pool.chunk(0, w, 9, 10, 90, 20) == 0 && w.bytes == 0);
+  Fake::room = 100;
+  CHECK(pool.chunk(0, w, 9, 10, 90, 20) == 9 && w.bytes == 90);      // ... says nothing about the room
+  Fake::free(w.p);
+  w = {};
+  CHECK(pool.chunk(0, w, 6, 10, 300, 20) == 6);
   CHECK(pool.chunk(0, u, 30, 21, 300, 20) == 1 && u.bytes == 21);    // asked for again
   pool.handles(0, 1);
   pool.give(0, w.p, w.bytes);
